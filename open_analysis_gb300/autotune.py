@@ -3,7 +3,7 @@
 Each block of a sweep marches ``tile_z`` planes; longer marches amortise the pipeline prologue
 and the carried-plane reload, shorter ones expose more blocks. Four sweep variants exist: the
 fused H + E sweep of the interior (3), planes staged through shared memory by TMA tensor copies
-(2) or by cp.async (1), or marched in registers (0). The best point depends on the grid and the
+(2) or by cp.async (1), or the direct sweeps (0). The best point depends on the grid and the
 batch. :func:`tune` times each candidate on the
 engine itself with CUDA events (a few 64-step chunks after one warm-up chunk, which also captures
 the graph of that shape) and leaves the fastest shape set on the engine. Timing steps advance
@@ -17,7 +17,7 @@ from typing import Any
 
 TILES = (4, 8, 16, 24, 32, 64)
 FUSED_TILES = (8, 16, 32, 64, 128)  # the fused sweep recomputes one plane per march: longer ones
-VARIANTS = (3, 2, 1, 0)  # fused, staged by TMA, staged by cp.async, register marching
+VARIANTS = (3, 2, 1, 0)  # fused, staged by TMA, staged by cp.async, direct
 
 
 @dataclass(frozen=True)
@@ -29,7 +29,7 @@ class TuneResult:
 
 
 def _candidates(tiles: tuple[int, ...], variants: tuple[int, ...]) -> list[tuple[int, int]]:
-    # variant 0 runs the slab kernel alone, whose march does not depend on the tile; the fused
+    # variant 0 runs the direct sweeps alone, whose march does not depend on the tile; the fused
     # sweep takes its own, longer marches unless the caller gives tiles
     out = []
     for v in variants:

@@ -39,6 +39,15 @@ int fail(int code, const std::string& msg) {
                   std::string(#call) + ": " + cudaGetErrorString(err_));                          \
   } while (0)
 
+// Cells times members up to which the direct sweeps are the default in float32. us per step, direct
+// against the best fused shape (via transition, batch 2): 4.8 million 164 / 227, 9.6 million 268 /
+// 351, 10.8 million 320 / 378, 19.2 million 474 / 463, 27.2 million 638 / 622, 51.2 million 1139 /
+// 1055. Small fields stay in the 129 MB L2, where the fused sweep saves little, and its march over
+// the planes of a tile is a long serial chain on few blocks; large ones are bound by the memory
+// traffic it saves. In float64 the two float64 operations a clock and SM bound every variant, and the
+// fused sweep computes its tiles' halos twice: 853 against 1406 us at 161 x 143 x 88.
+constexpr double kDirectCells = 16e6;
+
 constexpr double kEps0 = 1.0 / (4e-7 * 3.14159265358979323846 * 299792458.0 * 299792458.0);
 constexpr double kMu0 = 4e-7 * 3.14159265358979323846;
 
@@ -72,7 +81,7 @@ struct EngineBase {
   int profiling = 0;
   int tile_z = 16;
   // 3: fused H + E sweep of the interior (two buffers per field), the rest as 2; 2: sweeps
-  // staged by TMA; 1: staged by cp.async; 0: register marching
+  // staged by TMA; 1: staged by cp.async; 0: the direct sweeps over the whole domain
   int staged = 2;
   bool tma_ok = false;  // the TMA descriptors were encoded (variant 2 available)
   bool fused_ok = false;  // the fused box is not empty and its descriptors were encoded
@@ -190,9 +199,11 @@ struct Engine final : EngineBase {
   int build(const oafdtd_problem& p);
   // parts: 1 the H half (H sweeps, ghosts, pre_e), 2 the E half (E sweeps, SIBC, edges, probe_e)
   int launch_step(int off, cudaEvent_t* ev, bool capturing = false, int parts = 3);
+  int direct_step(int off, cudaEvent_t* ev, unsigned rec);
   int step_half(int which) override;
   int plane(int comp, int k, double* out, const double* in) override;
   int plane_device(int comp, int k, void* dst, const void* src) override;
+  bool inject_direct = false;  // the direct sweeps take the edge list's edges with them
   bool half_pending = false;  // an H half ran and its E half has not
   int capture();
 
@@ -409,8 +420,8 @@ int Engine<real>::build(const oafdtd_problem& p) {
   timer.mark("ade_classify");
   // ---- combined table. Entry key: (category, material index, ADE row); categories 0 plain,
   // 1 dispersive, 2 dispersive with injection or surface impedance (deferred to the edge pass,
-  // after those). The map orders entries by category, so the kernels tell dispersive entries by
-  // an index range.
+  // after those), 3 plain with injection. The map orders entries by category, so the kernels tell
+  // dispersive and listed edges by index ranges.
   // Debye rows (cbe, beta_0..P-1) in the field precision. The edges are classified in parallel
   // parts; each part finds its rows (consecutive edges mostly share one, so the last is checked
   // first and a hash finds the others) and its table keys, then the parts are merged in order.
@@ -535,17 +546,55 @@ int Engine<real>::build(const oafdtd_problem& p) {
   for (int v = 0; v < p.n_mat; ++v)
     if (present[v]) entry[{0, v, -1}] = 0;
   if (entry.size() > 65536) return fail(OAFDTD_E_TABLE, "more than 65536 combined material entries");
+  // The direct sweeps take the edge list's edges with them (variant 0): the plain ones among them
+  // get entries of their own, category 3, so that the vector threads know them by their index. Not
+  // where a listed edge is set by the surface impedance first or lies in a CPML box (its psi is the
+  // vector threads'), nor where the entries would not fit (the fused sweep keeps kCoefSmem of them
+  // in shared memory): the edge pass then does it.
+  std::vector<std::pair<int, long long>> inj_plain;
+  {
+    std::vector<std::pair<int, long long>> def_sorted = deferred;
+    std::sort(def_sorted.begin(), def_sorted.end());
+    auto in_cpml = [&](int c, long long f) {
+      const int at[3] = {(int)(f % X), (int)(f / X % Y), (int)(f / ((long long)X * Y))};
+      for (int n = 0; n < p.n_corr; ++n) {
+        const oafdtd_correction& k = p.corr[n];
+        if (k.kind != 0 || k.c != c) continue;
+        bool in = true;
+        for (int ax = 0; ax < 3; ++ax) in = in && at[ax] >= k.lo[ax] && at[ax] < k.hi[ax];
+        if (in) return true;
+      }
+      return false;
+    };
+    inject_direct = true;
+    for (const std::pair<int, long long>& cf : def_sorted)
+      inject_direct = inject_direct && !on_sibc(cf.first, cf.second) && !in_cpml(cf.first, cf.second);
+    std::map<Key, int> extra;
+    for (size_t q = 0; q < inj_sorted.size(); ++q) {
+      if (q > 0 && inj_sorted[q] == inj_sorted[q - 1]) continue;
+      const std::pair<int, long long>& cf = inj_sorted[q];
+      inject_direct = inject_direct && !on_sibc(cf.first, cf.second) && !in_cpml(cf.first, cf.second);
+      if (std::binary_search(def_sorted.begin(), def_sorted.end(), cf)) continue;
+      inj_plain.push_back(cf);
+      extra[Key{3, p.idx[cf.first][cf.second], -1}] = 0;
+    }
+    const size_t total = entry.size() + extra.size();
+    inject_direct &= total <= 65536 && (total <= (size_t)oafdtd::kCoefSmem || entry.size() > (size_t)oafdtd::kCoefSmem);
+    if (inject_direct) entry.insert(extra.begin(), extra.end());
+    else inj_plain.clear();
+  }
   std::vector<oafdtd::Coef<real>> t_coef;
   std::vector<real> t_beta;
   std::vector<double> t_eps;
   std::vector<int> plain(p.n_mat, 0);
-  int ade_lo = -1, ade_hi = -1;
+  int ade_lo = -1, ade_hi = -1, edge_lo = -1;
   for (auto& kv : entry) {
     const int cat = std::get<0>(kv.first), v = std::get<1>(kv.first), rid = std::get<2>(kv.first);
     const int id = (int)t_coef.size();
     kv.second = id;
     if (cat == 1 && ade_lo < 0) ade_lo = id;
     if (cat == 1) ade_hi = id + 1;
+    if (cat >= 2 && edge_lo < 0) edge_lo = id;
     if (cat == 0) plain[v] = id;
     oafdtd::Coef<real> cf;
     cf.ca = (real)p.ca_tab[v];
@@ -557,6 +606,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
     t_eps.push_back(p.eps_tab[v] * kEps0);
   }
   if (ade_lo < 0) ade_lo = ade_hi = 0;
+  if (edge_lo < 0) edge_lo = (int)t_coef.size();
   // the index arrays: plain entries, then each dispersive edge's entry; kept on the host for the
   // traffic model
   std::vector<uint16_t> host_mat[3];
@@ -580,6 +630,8 @@ int Engine<real>::build(const oafdtd_problem& p) {
         m[ae[e].f] = (uint16_t)lid;
       }
     });
+    for (const std::pair<int, long long>& cf : inj_plain)
+      if (cf.first == c) m[cf.second] = (uint16_t)entry.find(Key{3, idx[cf.second], -1})->second;
     uint16_t* dm = nullptr;
     int rc = upload_vec(&dm, m);
     if (rc) return rc;
@@ -595,6 +647,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
     sw.n_coef = (int)t_coef.size();
     sw.ade_lo = ade_lo;
     sw.ade_hi = ade_hi;
+    sw.edge_lo = edge_lo;
     real* d = nullptr;
     if (t_beta.empty()) t_beta.push_back((real)0);
     rc = upload_vec(&d, t_beta);
@@ -856,7 +909,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
   ed.B = pr.B = en.B = B;
   if (int rc = alloc(&step_base, 1)) return rc;
   keep_state(step_base, 1);
-  ed.step_base = pr.step_base = step_base;
+  ed.step_base = pr.step_base = pr.counter = step_base;
 
   timer.mark("edges_sibc");
   // ---- probes
@@ -905,6 +958,10 @@ int Engine<real>::build(const oafdtd_problem& p) {
     keep_state(acc, (size_t)std::max(p.n_probe, 1) * B * std::max(p.n_freq, 1));
     pr.acc = acc;
     pr.max_steps = p.max_steps;
+    if ((rc = alloc(&dd, (size_t)std::max(p.n_probe, 1) * B * oafdtd::kChunk))) return rc;
+    pr.vals = dd;
+    if ((rc = alloc(&di, 1))) return rc;
+    pr.dft_done = di;
     pr.series = nullptr;
     if (p.record_series && p.n_probe > 0) {
       double* ser = nullptr;
@@ -995,7 +1052,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
       const int qa = std::min(((lo[0] + 3) / 4 + 1) & ~1, Q), qb = std::max(std::min(hi[0] / 4, Q), qa);
       const int ja = std::min(std::max(lo[1], 1), ny + 2), jb = std::max(std::min(hi[1], ny + 2), ja);
       const int ka = std::min(std::max(lo[2], 1), nz + 2), kb = std::max(std::min(hi[2], nz + 2), ka);
-      inner_staged[kind] = oafdtd::Span3{qa, qb, ja, jb, ka, kb};
+      inner_staged[kind] = sw.core[kind] = oafdtd::Span3{qa, qb, ja, jb, ka, kb};
       // the z-slab planes of the interior's x-y extent hold z corrections only: staged too
       zin_staged[kind][0] = oafdtd::Span3{qa, qb, ja, jb, 1, ka};
       zin_staged[kind][1] = oafdtd::Span3{qa, qb, ja, jb, kb, nz + 2};
@@ -1194,9 +1251,12 @@ int Engine<real>::build(const oafdtd_problem& p) {
     });
   }
   timer.mark("traffic_model");
-  // The fused sweep is the default where it applies and the device has room for the second
-  // field buffers; otherwise the staged sweeps run in place.
-  if (fused_ok && staged == 2) {
+  // The default variant. The direct sweeps (0) up to kDirectCells cells times members and for every
+  // float64 grid, the fused sweep above where it applies and the device has room for the second
+  // field buffers, else the staged sweeps in place.
+  if (sizeof(real) == 8 || (double)nx * ny * nz * B <= kDirectCells) {
+    if (int rc = set_variant(0)) return rc;
+  } else if (fused_ok && staged == 2) {
     size_t free_b = 0, total_b = 0;
     OA_CUDA(cudaMemGetInfo(&free_b, &total_b));
     if ((double)free_b > 1.05 * 6.0 * (double)bs * B * sizeof(real))
@@ -1244,6 +1304,34 @@ int Engine<real>::sweep_pair(int kind, cudaEvent_t* ev, int slot, unsigned rec, 
   return OAFDTD_OK;
 }
 
+// One time step of variant 0: the H sweep, the ghosts, the E sweep with the injection, the surface
+// impedance. The H sweep's first blocks sample the E probes of the step before, the E sweep's the H
+// probes of this one; the last E samples are taken by the DFT launch that ends the chunk. Where
+// the injection cannot ride along, pre_e and the edge pass run as in the other variants.
+template <typename real>
+int Engine<real>::direct_step(int off, cudaEvent_t* ev, unsigned rec) {
+  auto mark = [&](int k) { return ev ? cudaEventRecordWithFlags(ev[k], stream, rec) : cudaSuccess; };
+  cudaError_t err;
+  if ((err = mark(0)) != cudaSuccess || (err = mark(1)) != cudaSuccess ||
+      (err = oafdtd::launch_slab<real>(sw, 1, stream, nullptr, &pr, off)) != cudaSuccess ||
+      (err = mark(2)) != cudaSuccess)
+    return fail(OAFDTD_E_CUDA, std::string("h_slab: ") + cudaGetErrorString(err));
+  if (pmc_mask) err = oafdtd::launch_ghosts<real>(sw.Ho, pmc_mask, nx, ny, nz, X, Y, B, stream);
+  if (err != cudaSuccess || (err = mark(3)) != cudaSuccess)
+    return fail(OAFDTD_E_CUDA, std::string("ghosts: ") + cudaGetErrorString(err));
+  if (!inject_direct) err = oafdtd::launch_pre_e<real>(pr, off, stream);
+  if (err != cudaSuccess || (err = mark(4)) != cudaSuccess || (err = mark(5)) != cudaSuccess)
+    return fail(OAFDTD_E_CUDA, std::string("pre_e: ") + cudaGetErrorString(err));
+  err = oafdtd::launch_slab<real>(sw, 0, stream, inject_direct ? &ed : nullptr, inject_direct ? &pr : nullptr, off);
+  if (err != cudaSuccess || (err = mark(6)) != cudaSuccess)
+    return fail(OAFDTD_E_CUDA, std::string("e_slab: ") + cudaGetErrorString(err));
+  err = oafdtd::launch_sibc<real>(sb, stream);
+  if (err == cudaSuccess && !inject_direct) err = oafdtd::launch_edges<real>(ed, off, stream);
+  if (err != cudaSuccess || (err = mark(7)) != cudaSuccess || (err = mark(8)) != cudaSuccess)
+    return fail(OAFDTD_E_CUDA, std::string("edges: ") + cudaGetErrorString(err));
+  return OAFDTD_OK;
+}
+
 // One time step (parts 3) or one half of it (1: H, 2: E), from the current buffers. Profiling
 // records the class events of the step: ev[9] at its start, ev[0..8] after the fused sweep,
 // h_sweep, h_slab, ghosts, pre_e, e_sweep, e_slab, edges and probe_e. In the fused variant the
@@ -1269,6 +1357,7 @@ int Engine<real>::launch_step(int off, cudaEvent_t* ev, bool capturing, int part
   bind(p, p);
   const oafdtd::SweepMaps& mp = maps_p[p];
   if (ev) OA_CUDA(cudaEventRecordWithFlags(ev[9], stream, rec));
+  if (staged == 0 && parts == 3) return direct_step(off, ev, rec);
   if (fused) {
     if (ev) {
       err = oafdtd::launch_fused_sweep<real>(sw, fmaps[p], stream);
@@ -1356,7 +1445,7 @@ int Engine<real>::capture() {
   for (int o = 0; o < oafdtd::kChunk && rc == OAFDTD_OK; ++o)
     rc = launch_step(o, profiling ? &events[(size_t)o * (kClasses + 1)] : nullptr, true);
   if (rc == OAFDTD_OK) {
-    cudaError_t err = oafdtd::launch_bump(step_base, oafdtd::kChunk, stream);
+    cudaError_t err = oafdtd::launch_dft<real>(pr, oafdtd::kChunk, 3, staged == 0, oafdtd::kChunk, stream);
     if (err != cudaSuccess) rc = fail(OAFDTD_E_CUDA, cudaGetErrorString(err));
   }
   cur[0] = cur0[0];
@@ -1446,7 +1535,7 @@ int Engine<real>::enqueue(int64_t n) {
         int rc = launch_step(o, profiling ? &events[(size_t)o * (kClasses + 1)] : nullptr);
         if (rc) return rc;
       }
-      cudaError_t err = oafdtd::launch_bump(step_base, take, stream);
+      cudaError_t err = oafdtd::launch_dft<real>(pr, take, 3, staged == 0, take, stream);
       if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, cudaGetErrorString(err));
     }
     if (profiling) {
@@ -1569,11 +1658,12 @@ int Engine<real>::step_half(int which) {
     if (steps + 1 > max_steps) return fail(OAFDTD_E_RANGE, "step count exceeds max_steps (wave table length)");
     sw.tile_z = tile_z;
     if (int rc = launch_step(0, nullptr, false, 1)) return rc;
+    OA_CUDA(oafdtd::launch_dft<real>(pr, 1, 2, false, 0, stream));
     half_pending = true;
   } else {
     if (!half_pending) return fail(OAFDTD_E_INVALID, "an E half needs its H half first");
     if (int rc = launch_step(0, nullptr, false, 2)) return rc;
-    cudaError_t err = oafdtd::launch_bump(step_base, 1, stream);
+    cudaError_t err = oafdtd::launch_dft<real>(pr, 1, 1, false, 1, stream);
     if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, cudaGetErrorString(err));
     half_pending = false;
     steps += 1;
@@ -1781,9 +1871,8 @@ struct Batch final : BatchBase {
   oafdtd::SibcArgs<real>* d_sb[2] = {};
   oafdtd::EdgeArgs<real>* d_ed[2] = {};
   oafdtd::SlabLaunch* d_slab[2] = {};  // per kind (the same for both parities)
-  long long** d_step_base = nullptr;
   std::vector<oafdtd::SweepArgs<real>> h_sw[2];
-  std::vector<Launch> fused, h_inner, h_z, e_inner, e_z, slab_h, slab_e, pre_e, probe_e, edges, sibc;
+  std::vector<Launch> fused, h_inner, h_z, e_inner, e_z, slab_h, slab_e, pre_e, probe_e, edges, sibc, dft;
   bool tma = false;
   cudaGraphExec_t graph[2] = {};
 
@@ -1896,11 +1985,17 @@ struct Batch final : BatchBase {
     // launch geometry, from the parity-0 arguments (the boxes do not depend on the buffers)
     const std::vector<oafdtd::SweepArgs<real>>& a = h_sw[0];
     std::vector<dim3> g_fused(n), g_hi(n), g_hz(n), g_ei(n), g_ez(n), g_sh(n), g_se(n), g_pre(n), g_probe(n),
-        g_edge(n), g_sibc(n);
+        g_edge(n), g_sibc(n), g_dft(n);
     std::vector<int> k_pole(n), k_zero(n, 0), k_sibc(n);
     std::vector<oafdtd::SlabLaunch> slabs[2];
     slabs[0].resize(n);
     slabs[1].resize(n);
+    int planes[2];  // of the direct sweeps: one launch over every engine's vectors
+    for (int kind = 0; kind < 2; ++kind) {
+      long long vecs = 0;
+      for (int i = 0; i < n; ++i) vecs += oafdtd::slab_vecs(a[i], kind);
+      planes[kind] = oafdtd::slab_planes(vecs);
+    }
     for (int i = 0; i < n; ++i) {
       cudaError_t err = cudaSuccess;
       if (variant == 3 && (err = oafdtd::fused_grid(a[i], &g_fused[i])) != cudaSuccess)
@@ -1915,28 +2010,36 @@ struct Batch final : BatchBase {
       if (variant != 3) g_fused[i] = dim3(0, 0, 0);
       for (int kind = 0; kind < 2; ++kind) {
         long long blocks = 0;
-        if (oafdtd::slab_plan(a[i], kind, &slabs[kind][i], &blocks) != cudaSuccess)
+        if (oafdtd::slab_plan(a[i], kind, &slabs[kind][i], &blocks, planes[kind]) != cudaSuccess)
           return fail(OAFDTD_E_INVALID, "slab geometry of a batched engine");
+        if (variant == 0) {  // Engine::direct_step: the samples and the injection ride along
+          oafdtd::SlabLaunch& L = slabs[kind][i];
+          const bool inject = kind == 0 && eng[i]->inject_direct;
+          if (inject) L.inject = oafdtd::inject_blocks(eng[i]->ed);
+          if (kind == 1 || inject) L.extra = eng[i]->pr.n_kind[1 - kind] * eng[i]->B;
+          blocks += L.extra + L.inject;
+        }
         (kind == 0 ? g_se : g_sh)[i] = dim3((unsigned)blocks, 1, 1);
       }
       const Engine<real>& e = *eng[i];
       g_pre[i] = dim3((unsigned)oafdtd::pre_e_blocks(e.pr), 1, 1);
       g_probe[i] = dim3((unsigned)oafdtd::probe_e_blocks(e.pr), 1, 1);
       g_edge[i] = dim3((unsigned)oafdtd::edge_blocks(e.ed), 1, 1);
+      if (variant == 0) g_probe[i] = dim3(0, 0, 0);
+      if (variant == 0 && e.inject_direct) g_pre[i] = g_edge[i] = dim3(0, 0, 0);
       g_sibc[i] = dim3((unsigned)oafdtd::sibc_blocks(e.sb), 1, 1);
+      g_dft[i] = dim3((unsigned)oafdtd::dft_blocks(e.pr), 1, 1);
       k_pole[i] = a[i].ade_P > 1 ? 1 : 0;
       k_sibc[i] = oafdtd::sibc_variant(e.sb);
     }
     for (int kind = 0; kind < 2; ++kind)
       if (int rc = upload(&d_slab[kind], slabs[kind].data(), n)) return rc;
-    std::vector<long long*> bases(n);
-    for (int i = 0; i < n; ++i) bases[i] = eng[i]->step_base;
-    if (int rc = upload(&d_step_base, bases.data(), n)) return rc;
     const std::pair<std::vector<dim3>*, std::pair<std::vector<int>*, std::vector<Launch>*>> plans[] = {
         {&g_fused, {&k_pole, &fused}},  {&g_hi, {&k_zero, &h_inner}}, {&g_hz, {&k_zero, &h_z}},
         {&g_ei, {&k_pole, &e_inner}},   {&g_ez, {&k_pole, &e_z}},     {&g_sh, {&k_zero, &slab_h}},
         {&g_se, {&k_pole, &slab_e}},    {&g_pre, {&k_zero, &pre_e}},  {&g_probe, {&k_zero, &probe_e}},
         {&g_edge, {&k_zero, &edges}},   {&g_sibc, {&k_sibc, &sibc}},
+        {&g_dft, {&k_zero, &dft}},
     };
     for (const auto& q : plans)
       if (int rc = plan(*q.first, *q.second.first, q.second.second)) return rc;
@@ -1951,28 +2054,36 @@ struct Batch final : BatchBase {
     }
     return OAFDTD_OK;
   }
-  int slab_launches(int kind, int p, cudaStream_t s) {
+  int slab_launches(int kind, int p, int off, cudaStream_t s) {
     for (const Launch& L : kind == 0 ? slab_e : slab_h) {
-      const cudaError_t err =
-          oafdtd::launch_slab_batch<real>(d_sw[p], d_slab[kind], L.g, L.blocks, kind, L.key != 0, s);
+      const cudaError_t err = oafdtd::launch_slab_batch<real>(d_sw[p], d_slab[kind], d_ed[p], d_pr[p], L.g, L.blocks,
+                                                              kind, L.key != 0, off, s);
       if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, std::string("batched slab: ") + cudaGetErrorString(err));
     }
     return OAFDTD_OK;
   }
+  // the DFTs of the last n steps, and the step counters
+  int dft_launches(int n, int p) {
+    for (const Launch& L : dft) {
+      const cudaError_t err = oafdtd::launch_dft_batch<real>(d_pr[p], L.g, L.blocks, n, variant == 0, stream);
+      if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, std::string("batched dft: ") + cudaGetErrorString(err));
+    }
+    return OAFDTD_OK;
+  }
   // the staged sweep of one kind with its slab kernel beside it (Engine::sweep_pair)
-  int pair(int kind, int p) {
+  int pair(int kind, int p, int off) {
     const bool h = kind == 1;
     if (variant != 0) {
       OA_CUDA(cudaEventRecord(fork_ev, stream));
       OA_CUDA(cudaStreamWaitEvent(side, fork_ev, 0));
-      if (int rc = slab_launches(kind, p, side)) return rc;
+      if (int rc = slab_launches(kind, p, off, side)) return rc;
       OA_CUDA(cudaEventRecord(join_ev, side));
       if (int rc = sweep_launches(h ? h_inner : e_inner, h, false, p, stream)) return rc;
       if (int rc = sweep_launches(h ? h_z : e_z, h, true, p, stream)) return rc;
       OA_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
       return OAFDTD_OK;
     }
-    return slab_launches(kind, p, stream);
+    return slab_launches(kind, p, off, stream);
   }
 
   // One time step of every engine, from buffers p (Engine::launch_step with parts 3).
@@ -1986,10 +2097,10 @@ struct Batch final : BatchBase {
       OA_CUDA(cudaStreamWaitEvent(side, fork_ev, 0));
       if (int rc = sweep_launches(h_inner, true, false, p, side)) return rc;
       if (int rc = sweep_launches(h_z, true, true, p, side)) return rc;
-      if (int rc = slab_launches(1, p, side)) return rc;
+      if (int rc = slab_launches(1, p, off, side)) return rc;
       OA_CUDA(cudaEventRecord(join_ev, side));
       OA_CUDA(cudaStreamWaitEvent(stream, join_ev, 0));
-    } else if (int rc = pair(1, p)) {
+    } else if (int rc = pair(1, p, off)) {
       return rc;
     }
     for (size_t i = 0; i < eng.size(); ++i) {
@@ -2002,7 +2113,7 @@ struct Batch final : BatchBase {
     for (const Launch& L : pre_e)
       if ((err = oafdtd::launch_pre_e_batch<real>(d_pr[p], L.g, L.blocks, off, stream)) != cudaSuccess)
         return fail(OAFDTD_E_CUDA, std::string("batched pre_e: ") + cudaGetErrorString(err));
-    if (int rc = pair(0, p)) return rc;
+    if (int rc = pair(0, p, off)) return rc;
     for (const Launch& L : sibc)
       if ((err = oafdtd::launch_sibc_batch<real>(d_sb[p], L.g, L.blocks, L.key, stream)) != cudaSuccess)
         return fail(OAFDTD_E_CUDA, std::string("batched sibc: ") + cudaGetErrorString(err));
@@ -2025,8 +2136,7 @@ struct Batch final : BatchBase {
       if (variant == 3) q ^= 1;
     }
     if (rc == OAFDTD_OK) {
-      const cudaError_t err = oafdtd::launch_bump_batch(d_step_base, (int)eng.size(), oafdtd::kChunk, stream);
-      if (err != cudaSuccess) rc = fail(OAFDTD_E_CUDA, cudaGetErrorString(err));
+      rc = dft_launches(oafdtd::kChunk, q);
     }
     const cudaError_t err = cudaStreamEndCapture(stream, &g);
     if (rc != OAFDTD_OK) {
@@ -2079,8 +2189,7 @@ struct Batch final : BatchBase {
           if (int rc = launch_step(o, q)) return rc;
           if (variant == 3) q ^= 1;
         }
-        const cudaError_t err = oafdtd::launch_bump_batch(d_step_base, (int)eng.size(), take, stream);
-        if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, cudaGetErrorString(err));
+        if (int rc = dft_launches(take, q)) return rc;
       }
       for (Engine<real>* e : eng) {
         e->steps += take;

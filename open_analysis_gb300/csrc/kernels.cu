@@ -1,13 +1,13 @@
-// FDTD time-step kernels for sm_103a.
+// FDTD time-step kernels for sm_103a beside the sweeps (fused.cu, staged.cu, slab.cu).
 //
-// One time step is: h_sweep -> [ghosts] -> [pre_e] -> e_sweep -> [edges] -> [probe_e].
-//  * h_sweep, e_sweep: the Yee sweeps with CPML, and Debye ADE fused (sweeps.cu).
-//  * ghosts: PMC mirror planes, one launch per wall in wall order.
-//  * pre_e: H probe sums + running DFT at (n + 1/2) dt; saves E^n of dispersive edges that also
-//    receive injection (their ADE update runs after the injection, in the edge pass).
+//  * ghosts: PMC mirror planes, every wall in one launch.
+//  * pre_e: H probe samples at (n + 1/2) dt; saves E^n of dispersive edges that also receive
+//    injection (their ADE update runs after the injection, in the edge pass).
 //  * sibc, edges: surface impedance on its edge list, then injection and the deferred Debye
 //    updates on theirs.
-//  * probe_e: E probe sums + running DFT at (n + 1) dt.
+//  * probe_e: E probe samples at (n + 1) dt.
+//  * dft: the running DFTs of a chunk's samples, and the step counter.
+// In variant 0 the direct sweeps take the samples and the injection with them (slab.cu).
 //
 // Arithmetic follows the reference engine (packages/oa-fdtd/src/oa_fdtd/reference.py:115-249)
 // operation by operation; the library is built with -fmad=false, so float32 fields agree bit for
@@ -15,78 +15,168 @@
 // order (bulk update, then the corrections in ascending derivative axis, each rounded to the field
 // precision), so fusion changes no rounding.
 
+#include <algorithm>
+
 #include "oafdtd_internal.cuh"
+#include "probe.cuh"
 
 namespace oafdtd {
 
 // ----------------------------------------------------------------------------- PMC ghosts
-// h[dst plane] = -h[src plane] over the whole plane (every storage index of the other axes).
+// h[dst plane] = -h[src plane] for both components tangential to a PMC wall, over the whole plane
+// (every storage index of the other axes), wall after wall in the order x low, x high, y low, ...
+// One launch for every wall (blockIdx.y): where planes of two walls meet, the last wall's value
+// follows from reflecting the point across each earlier wall it lies on, so no wall waits for
+// another.
 template <typename real>
-__global__ void ghost_kernel(real* H0, real* H1, int axis, int dst, int src, int X, int Y, int Z,
-                             int B) {
-  const int ext[3] = {X, Y, Z};
-  const int u_ax = axis == 0 ? 1 : 0;
-  const int v_ax = axis == 2 ? 1 : 2;
-  const long long nu = ext[u_ax], nv = ext[v_ax];
-  const long long total = nu * nv * B;
-  const long long st[3] = {1, X, (long long)X * Y};
-  const long long bs = (long long)X * Y * Z;
+struct GhostArgs {
+  real* H[3];
+  int mask, n[3], ext[3], B;
+};
+
+template <typename real>
+__device__ __forceinline__ void ghost_wall(const GhostArgs<real>& g, int wall, int v, int u, int b) {
+  const int axis = wall >> 1;
+  const int u_ax = axis == 0 ? 1 : 0, v_ax = axis == 2 ? 1 : 2;
+  const long long base = (long long)b * g.ext[0] * g.ext[1] * g.ext[2];
+  for (int c = 0; c < 3; ++c) {
+    if (c == axis) continue;
+    int p[3];
+    p[axis] = (wall & 1) ? g.n[axis] + 1 : 0;
+    p[u_ax] = u;
+    p[v_ax] = v;
+    bool later = false;  // a later wall writes this point
+    for (int w = wall + 1; w < 6; ++w)
+      later |= ((g.mask >> w) & 1) && c != (w >> 1) && p[w >> 1] == ((w & 1) ? g.n[w >> 1] + 1 : 0);
+    if (later) continue;
+    const long long dst = base + ((long long)p[2] * g.ext[1] + p[1]) * g.ext[0] + p[0];
+    bool neg = false;
+    for (int w = wall; w >= 0; --w) {
+      const int ax = w >> 1;
+      if (!((g.mask >> w) & 1) || c == ax || p[ax] != ((w & 1) ? g.n[ax] + 1 : 0)) continue;
+      p[ax] = (w & 1) ? g.n[ax] : 1;
+      neg = !neg;
+    }
+    const real s = g.H[c][base + ((long long)p[2] * g.ext[1] + p[1]) * g.ext[0] + p[0]];
+    g.H[c][dst] = neg ? -s : s;
+  }
+}
+
+template <typename real>
+__global__ void __launch_bounds__(256) ghost_kernel(const __grid_constant__ GhostArgs<real> g) {
+  const int wall = blockIdx.y, axis = wall >> 1;
+  if (!((g.mask >> wall) & 1)) return;
+  const int nu = g.ext[axis == 0 ? 1 : 0], nv = g.ext[axis == 2 ? 1 : 2];
+  const long long total = (long long)nu * nv * g.B;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    const long long u = t % nu;
     const long long r = t / nu;
-    const long long v = r % nv;
-    const long long b = r / nv;
-    const long long off = b * bs + u * st[u_ax] + v * st[v_ax];
-    const long long pd = off + dst * st[axis], ps = off + src * st[axis];
-    H0[pd] = -H0[ps];
-    H1[pd] = -H1[ps];
+    ghost_wall(g, wall, (int)(r % nv), (int)(t - r * nu), (int)(r / nv));
   }
 }
 
 // ----------------------------------------------------------------------------- probes
-// Weighted float64 sum of one probe for one batch member (fixed-order reduction), then the
-// running DFT acc[f] += exp(-j w t) dt V with t = (n + offset) dt.
+// Every step's probe samples (probe_sample) are kept for the chunk; one launch at its end adds
+// them to the running DFTs, acc[f] += exp(-j w t) dt V with t = (n + offset) dt, step after step as
+// the reference does, and advances the step counter. A DFT per step put 256 float64 sincos of one
+// block on the path of every step (8 us a step for the E probes at 64 to 256 frequencies: GB300
+// issues two float64 operations a clock and SM); here a block takes four frequencies, one thread
+// per (frequency, step) for the phases, which all probes of a kind share, then one thread per
+// (probe, member, frequency) for the sums.
+constexpr int kDftF = 4;
+
 template <typename real>
-__device__ void probe_block(const ProbeArgs<real>& a, int pid, int b, long long step, double toff) {
-  __shared__ double warp_sum[32];
-  const real* F = a.F[(a.kind[pid] == 0 ? 0 : 3) + a.comp[pid]] + (long long)b * a.bs;
-  double acc = 0.0;
-  for (long long e = a.off[pid] + threadIdx.x; e < a.off[pid + 1]; e += blockDim.x)
-    acc += (double)F[a.flat[e]] * a.w[e];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) warp_sum[warp] = acc;
-  __syncthreads();
-  __shared__ double total;
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += warp_sum[w];
-    total = s;
-    if (a.series != nullptr) a.series[((long long)pid * a.B + b) * a.max_steps + step] = s;
+__host__ __device__ __forceinline__ int dft_blocks_of(const ProbeArgs<real>& a) {
+  return a.n_probe > 0 && a.n_freq > 0 ? 2 * ((a.n_freq + kDftF - 1) / kDftF) : 1;
+}
+
+// Steps base .. base + n - 1 of the probes of the kinds in `kinds` (bit 0 E, bit 1 H). tail: the last
+// step's E samples are not in yet and taken here (by every block: a few points each).
+template <typename real>
+__device__ __forceinline__ void dft_body(const ProbeArgs<real>& a, int block, int n, int kinds, bool tail, int bump) {
+  __shared__ double2 ph[kDftF][kChunk];
+  __shared__ double tails[kChunk];
+  const long long base = *a.step_base;
+  const int nfb = (a.n_freq + kDftF - 1) / kDftF;
+  const int kind = nfb > 0 ? block / nfb : 0, f0 = nfb > 0 ? (block % nfb) * kDftF : 0;
+  const int pairs = kind < 2 && ((kinds >> kind) & 1) ? a.n_kind[kind] * a.B : 0;
+  if (pairs > 0 && a.n_freq > 0) {
+    const int fi = threadIdx.x / kChunk, o = threadIdx.x % kChunk;
+    if (o < n && f0 + fi < a.n_freq) {
+      const double t = ((double)(base + o) + (kind == 0 ? 1.0 : 0.5)) * a.dt;
+      double sn, cs;
+      sincos(a.omega[f0 + fi] * t, &sn, &cs);
+      ph[fi][o] = make_double2(cs * a.dt, -(sn * a.dt));
+    }
+    const bool last = tail && kind == 0;
+    for (int p0 = 0; p0 < pairs; p0 += kChunk) {
+      if (last) {
+        for (int q = p0; q < min(pairs, p0 + kChunk); ++q) {
+          const int pid = a.list[0][q / a.B], b = q % a.B;
+          const double s = probe_sum(a, 0, pid, b);
+          if (threadIdx.x == 0) {
+            tails[q - p0] = s;
+            if (f0 == 0 && a.series != nullptr)
+              a.series[((long long)pid * a.B + b) * a.max_steps + base + n - 1] = s;
+          }
+        }
+      }
+      __syncthreads();
+      const int q = p0 + (int)threadIdx.x / kDftF, f = (int)threadIdx.x % kDftF;
+      if (q < pairs && f0 + f < a.n_freq) {
+        const long long pb = (long long)a.list[kind][q / a.B] * a.B + q % a.B;
+        const double* v = a.vals + pb * kChunk;
+        double2* out = a.acc + pb * a.n_freq + f0 + f;
+        double2 cur = *out;
+        const int m = last ? n - 1 : n;
+#pragma unroll 8
+        for (int s = 0; s < m; ++s) {
+          const double x = v[s];
+          cur.x += ph[f][s].x * x;
+          cur.y += ph[f][s].y * x;
+        }
+        if (last) {
+          cur.x += ph[f][n - 1].x * tails[q - p0];
+          cur.y += ph[f][n - 1].y * tails[q - p0];
+        }
+        *out = cur;
+      }
+      __syncthreads();
+    }
   }
+  if (bump == 0) return;
+  // the last block to get here advances the counter: every block has read it
   __syncthreads();
-  const double v = total;
-  const double t = ((double)step + toff) * a.dt;
-  double2* out = a.acc + ((long long)pid * a.B + b) * a.n_freq;
-  for (int f = threadIdx.x; f < a.n_freq; f += blockDim.x) {
-    double sn, cs;
-    sincos(a.omega[f] * t, &sn, &cs);
-    double2 cur = out[f];
-    cur.x += (cs * a.dt) * v;
-    cur.y += (-(sn * a.dt)) * v;
-    out[f] = cur;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(a.dft_done, 1) == dft_blocks_of(a) - 1) {
+      *a.dft_done = 0;
+      *a.counter += bump;
+    }
   }
 }
 
 template <typename real>
+__global__ void __launch_bounds__(kDftF* kChunk) dft_kernel(const __grid_constant__ ProbeArgs<real> a, int n, int kinds,
+                                                            int tail, int bump) {
+  dft_body(a, (int)blockIdx.x, n, kinds, tail != 0, bump);
+}
+
+// Several engines' DFTs (and step counters) in one launch.
+template <typename real>
+__global__ void __launch_bounds__(kDftF* kChunk)
+    dft_batch_kernel(const ProbeArgs<real>* __restrict__ A, const BatchGrid G, int n, int tail) {
+  __shared__ __align__(16) unsigned char args[sizeof(ProbeArgs<real>)];
+  int e;
+  const uint3 bid = G.block(&e);
+  dft_body(stage_args(A + e, args), (int)bid.x, n, 3, tail != 0, n);
+}
+
+template <typename real>
 __device__ __forceinline__ void pre_e_body(const ProbeArgs<real>& a, int off, int block) {
-  const long long step = *a.step_base + off;
   const int nprobe_blocks = a.n_kind[1] * a.B;
   if (block < nprobe_blocks) {
-    const int pi = block / a.B, b = block % a.B;
-    probe_block(a, a.list[1][pi], b, step, 0.5);
+    probe_sample(a, 1, block, off);
     return;
   }
   const int t = (block - nprobe_blocks) * blockDim.x + threadIdx.x;
@@ -101,18 +191,11 @@ __global__ void __launch_bounds__(256) pre_e_kernel(const __grid_constant__ Prob
 }
 
 template <typename real>
-__device__ __forceinline__ void probe_e_body(const ProbeArgs<real>& a, int off, int block) {
-  const long long step = *a.step_base + off;
-  const int pi = block / a.B, b = block % a.B;
-  probe_block(a, a.list[0][pi], b, step, 1.0);
-}
-
-template <typename real>
 __global__ void __launch_bounds__(256) probe_e_kernel(const __grid_constant__ ProbeArgs<real> a, int off) {
-  probe_e_body(a, off, (int)blockIdx.x);
+  probe_sample(a, 0, (int)blockIdx.x, off);
 }
 
-// Several engines' deferred-E saves and H-probe DFTs, and E-probe DFTs, in one launch each.
+// Several engines' deferred-E saves and H-probe samples, and E-probe samples, in one launch each.
 template <typename real>
 __global__ void __launch_bounds__(256) pre_e_batch_kernel(const ProbeArgs<real>* __restrict__ A, const BatchGrid G,
                                                           int off) {
@@ -128,7 +211,7 @@ __global__ void __launch_bounds__(256) probe_e_batch_kernel(const ProbeArgs<real
   __shared__ __align__(16) unsigned char args[sizeof(ProbeArgs<real>)];
   int e;
   const uint3 bid = G.block(&e);
-  probe_e_body(stage_args(A + e, args), off, (int)bid.x);
+  probe_sample(stage_args(A + e, args), 0, (int)bid.x, off);
 }
 
 // ----------------------------------------------------------------------------- surface impedance
@@ -437,34 +520,22 @@ __global__ void energy_final_kernel(const double* partial, int nblocks, double* 
   out[cc] = s;
 }
 
-__global__ void bump_kernel(long long* step_base, int n) { *step_base += n; }
-
-__global__ void bump_batch_kernel(long long* const* step_base, int n_eng, int n) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < n_eng) *step_base[e] += n;
-}
-
 // ----------------------------------------------------------------------------- launchers
 static inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
 template <typename real>
 cudaError_t launch_ghosts(real* const H[3], int pmc_mask, int nx, int ny, int nz, int X, int Y, int B,
                           cudaStream_t s) {
-  const int n[3] = {nx, ny, nz};
-  const int Z = nz + 2;
-  for (int axis = 0; axis < 3; ++axis) {
-    for (int side = 0; side < 2; ++side) {
-      if (!(pmc_mask & (1 << (2 * axis + side)))) continue;
-      const int dst = side == 0 ? 0 : n[axis] + 1;
-      const int src = side == 0 ? 1 : n[axis];
-      real* h0 = H[axis == 0 ? 1 : 0];
-      real* h1 = H[axis == 2 ? 1 : 2];
-      ghost_kernel<real><<<152 * 4, 256, 0, s>>>(h0, h1, axis, dst, src, X, Y, Z, B);
-      cudaError_t err = cudaGetLastError();
-      if (err != cudaSuccess) return err;
+  GhostArgs<real> g{{H[0], H[1], H[2]}, pmc_mask, {nx, ny, nz}, {X, Y, nz + 2}, B};
+  long long most = 0;
+  for (int w = 0; w < 6; ++w)
+    if ((pmc_mask >> w) & 1) {
+      const int axis = w >> 1;
+      most = std::max(most, (long long)g.ext[axis == 0 ? 1 : 0] * g.ext[axis == 2 ? 1 : 2] * B);
     }
-  }
-  return cudaSuccess;
+  if (most == 0) return cudaSuccess;
+  ghost_kernel<real><<<dim3(std::min(ceil_div(most, 256), 152u * 8u), 6), 256, 0, s>>>(g);
+  return cudaGetLastError();
 }
 
 template <typename real>
@@ -536,14 +607,22 @@ cudaError_t launch_energy(const EnergyArgs<real>& a, double* partial, int nblock
   return cudaGetLastError();
 }
 
-cudaError_t launch_bump(long long* step_base, int n, cudaStream_t s) {
-  bump_kernel<<<1, 1, 0, s>>>(step_base, n);
+template <typename real>
+int dft_blocks(const ProbeArgs<real>& a) {
+  return dft_blocks_of(a);
+}
+
+template <typename real>
+cudaError_t launch_dft(const ProbeArgs<real>& a, int n, int kinds, bool tail, int bump, cudaStream_t s) {
+  dft_kernel<real><<<dft_blocks_of(a), kDftF * kChunk, 0, s>>>(a, n, kinds, tail ? 1 : 0, bump);
   return cudaGetLastError();
 }
 
-cudaError_t launch_bump_batch(long long* const* step_base, int n_eng, int n, cudaStream_t s) {
-  if (n_eng <= 0) return cudaSuccess;
-  bump_batch_kernel<<<(unsigned)ceil_div(n_eng, 128), 128, 0, s>>>(step_base, n_eng, n);
+template <typename real>
+cudaError_t launch_dft_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int n, bool tail,
+                             cudaStream_t s) {
+  if (blocks <= 0) return cudaSuccess;
+  dft_batch_kernel<real><<<blocks, kDftF * kChunk, 0, s>>>(A, G, n, tail ? 1 : 0);
   return cudaGetLastError();
 }
 
@@ -554,6 +633,10 @@ cudaError_t launch_bump_batch(long long* const* step_base, int n_eng, int n, cud
   template cudaError_t launch_probe_e<real>(const ProbeArgs<real>&, int, cudaStream_t);            \
   template cudaError_t launch_edges<real>(const EdgeArgs<real>&, int, cudaStream_t);               \
   template cudaError_t launch_sibc<real>(const SibcArgs<real>&, cudaStream_t, int, int);            \
+  template int dft_blocks<real>(const ProbeArgs<real>&);                                            \
+  template cudaError_t launch_dft<real>(const ProbeArgs<real>&, int, int, bool, int, cudaStream_t); \
+  template cudaError_t launch_dft_batch<real>(const ProbeArgs<real>*, const BatchGrid&, int, int, bool, \
+                                              cudaStream_t);                                        \
   template int pre_e_blocks<real>(const ProbeArgs<real>&);                                          \
   template int probe_e_blocks<real>(const ProbeArgs<real>&);                                        \
   template int edge_blocks<real>(const EdgeArgs<real>&);                                            \
@@ -585,8 +668,8 @@ cudaError_t preload_kernels() {
       reinterpret_cast<const void*>(edge_kernel<real>),
       reinterpret_cast<const void*>(energy_kernel<real>),
       reinterpret_cast<const void*>(energy_final_kernel),
-      reinterpret_cast<const void*>(bump_kernel),
-      reinterpret_cast<const void*>(bump_batch_kernel),
+      reinterpret_cast<const void*>(dft_kernel<real>),
+      reinterpret_cast<const void*>(dft_batch_kernel<real>),
       reinterpret_cast<const void*>(pre_e_batch_kernel<real>),
       reinterpret_cast<const void*>(probe_e_batch_kernel<real>),
       reinterpret_cast<const void*>(sibc_batch_kernel<real, 2, 16>),

@@ -70,6 +70,7 @@ struct SweepArgs {
   const Coef<real>* coef;   // [entry]; entries [ade_lo, ade_hi) are dispersive, then deferred ones
   int n_coef;               // entries in the table
   int ade_lo, ade_hi;
+  int edge_lo;              // first entry of the edges the edge list holds (n_coef: none)
   const real* ade_beta;     // [entry * P + p]
   const real* ade_kp;       // [p]
   const real* ade_onekp;    // [p]: 1 + kp in the field precision
@@ -102,6 +103,7 @@ struct SweepArgs {
   int zsd[2][2][2];  // [kind][low/high][component 0/1]: side of the z-term psi, -1 if none
   Span3 slab[2][6];
   int n_slab[2];
+  Span3 core[2];     // the interior box of each kind, whatever the variant sweeps it with
 };
 
 // TMA descriptors of the staged sweeps: per component, the field arrays as 4-D tensors
@@ -207,6 +209,9 @@ struct ProbeArgs {
   double dt;
   double2* acc;              // (n_probe, B, F)
   double* series;            // (n_probe, B, max_steps) or nullptr
+  double* vals;              // (n_probe, B, kChunk): the samples of the steps of a chunk
+  int* dft_done;             // blocks of the DFT launch that have read the step counter
+  long long* counter;        // the step counter the DFT launch advances (step_base)
   int max_steps;
   long long bs;
   int B;
@@ -235,13 +240,25 @@ struct EnergyArgs {
 constexpr int kEnergyWShift = 40;  // weights scaled by 2^40 ...
 constexpr int kEnergyVShift = 32;  // ... and fields by 2^32 (squares by 2^64) in the float-float sum
 
-// Launch geometry of the slab kernel: the boxes of one kind with their first block.
+// A divisor of a launch geometry: m = ceil(2^32 / d) where the high half of a multiplication by it
+// divides exactly for every operand of the launch, 0 elsewhere.
+struct FastDiv {
+  int d;
+  unsigned m;
+};
+
+// Launch geometry of the direct sweeps: the boxes of one kind with their first block.
 struct SlabLaunch {
   Span3 box[6];
   int n;
   int first[7];  // first block of each box; first[n] = total blocks
-  int cblk[6];   // column blocks per (box, chunk, member)
-  int nch[6];    // z chunks per box
+  int planes;       // planes marched per thread
+  FastDiv cblk[6];  // column blocks per (box, chunk, member)
+  FastDiv nch[6];   // z chunks per box
+  FastDiv nv[6];    // vector columns per row
+  Span3 core;    // holds no correction cell (quads, rows, planes)
+  int extra;     // leading blocks that sample probes (variant 0)
+  int inject;    // blocks after those that update the edge list's edges (variant 0, E)
 };
 
 // The blocks of one launch that covers several engines (a batched sweep): block b of the launch
@@ -284,7 +301,12 @@ cudaError_t fused_grid(const SweepArgs<real>& a, dim3* grid);
 template <typename real>
 cudaError_t staged_grids(const SweepArgs<real>& a, int kind, dim3* inner, dim3* z);
 template <typename real>
-cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long long* blocks);
+cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long long* blocks, int planes = 0);
+// Vectors of one kind's boxes, and the planes a thread marches in a launch over that many (0 to
+// slab_plan: its own).
+template <typename real>
+long long slab_vecs(const SweepArgs<real>& a, int kind);
+int slab_planes(long long vecs);
 template <typename real>
 int pre_e_blocks(const ProbeArgs<real>& a);
 template <typename real>
@@ -303,8 +325,9 @@ template <typename real>
 cudaError_t launch_staged_batch(const SweepArgs<real>* A, const SweepMaps* M, const BatchGrid& G, int blocks, bool h,
                                 bool tma, bool z, bool multi_pole, cudaStream_t s);
 template <typename real>
-cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const BatchGrid& G, int blocks, int kind,
-                              bool multi_pole, cudaStream_t s);
+cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
+                              const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
+                              int off, cudaStream_t s);
 template <typename real>
 cudaError_t launch_pre_e_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int off, cudaStream_t s);
 template <typename real>
@@ -313,16 +336,31 @@ template <typename real>
 cudaError_t launch_edges_batch(const EdgeArgs<real>* A, const BatchGrid& G, int blocks, int off, cudaStream_t s);
 template <typename real>
 cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int blocks, int variant, cudaStream_t s);
-// step_base[e] += n for the n_eng engines' device step counters (an array of device pointers)
-cudaError_t launch_bump_batch(long long* const* step_base, int n_eng, int n, cudaStream_t s);
+// The running DFTs of the n steps from the step counter on, for the probe kinds in `kinds` (bit 0
+// E, bit 1 H), which then advances by `bump`. tail: the E samples of the last step are taken here.
+template <typename real>
+int dft_blocks(const ProbeArgs<real>& a);
+template <typename real>
+cudaError_t launch_dft(const ProbeArgs<real>& a, int n, int kinds, bool tail, int bump, cudaStream_t s);
+// Several engines' n steps, both kinds; every counter advances by n.
+template <typename real>
+cudaError_t launch_dft_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int n, bool tail,
+                             cudaStream_t s);
 
 // kernel launchers (kernels.cu)
 template <typename real>
 cudaError_t launch_h_sweep(const SweepArgs<real>& a, const SweepMaps& m, cudaStream_t s);
 template <typename real>
 cudaError_t launch_e_sweep(const SweepArgs<real>& a, const SweepMaps& m, cudaStream_t s);
+// Blocks of the direct E sweep that take the edge list's edges (one thread per edge and member).
 template <typename real>
-cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s);
+int inject_blocks(const EdgeArgs<real>& ed);
+// The direct sweep of one kind over its boxes. ed: the E sweep takes the edge list's edges with it;
+// pr: its first blocks sample the probes that are due (E launch: H probes of step off; H launch: E
+// probes of step off - 1).
+template <typename real>
+cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, const EdgeArgs<real>* ed = nullptr,
+                        const ProbeArgs<real>* pr = nullptr, int off = 0);
 template <typename real>
 cudaError_t launch_ghosts(real* const H[3], int pmc_mask, int nx, int ny, int nz, int X, int Y, int B,
                           cudaStream_t s);
@@ -338,7 +376,6 @@ cudaError_t launch_probe_e(const ProbeArgs<real>& a, int off, cudaStream_t s);
 template <typename real>
 cudaError_t launch_energy(const EnergyArgs<real>& a, double* partial, int nblocks, double* out,
                           cudaStream_t s);
-cudaError_t launch_bump(long long* step_base, int n, cudaStream_t s);
 template <typename real>
 cudaError_t launch_staged_sweep(const SweepArgs<real>& a, const SweepMaps& m, cudaStream_t s, bool h);
 // The fused H + E sweep of a.fused (variant 3, two buffers per field).

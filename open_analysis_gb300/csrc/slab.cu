@@ -1,21 +1,34 @@
-// The slab kernel: everything outside the interior box of a sweep.
+// The direct kernels: H and E updates read straight from global memory, no staging.
 //
 // The update domain of each sweep is split into an interior box, which holds no CPML correction
-// cell and is swept by the staged kernels (staged.cu), and up to six disjoint boxes around it:
-// the z slabs (whole planes), then the y slabs and the x slabs of the remaining planes. This
-// kernel marches those boxes. With the staged sweeps off (variant 0) its one box is the whole
-// domain.
+// cell and is swept by the staged or fused kernels (staged.cu, fused.cu), and up to six disjoint
+// boxes around it: these kernels march those boxes. In variant 0 their one box is the whole
+// domain; it is the default where the fields of a grid stay in the L2 cache or are float64.
 //
-// Each thread owns a "quad" (four consecutive x cells of one storage row) and marches a chunk of
-// z planes, carrying the neighbouring plane in registers. For every cell it does, in the
-// reference's order (packages/oa-fdtd/src/oa_fdtd/reference.py:152-207, :115-127):
+// Each thread owns one component of one 16-byte vector of x cells (four float32 or two float64) of one
+// storage row and marches a few z planes, carrying the plane its z derivative needs again; the three
+// components of a column sit in one block, so the sources they share are read once into its L1.
+// Per plane every load is issued first (sources, field, index, Debye current, psi), then the
+// arithmetic, then the stores, so no load waits behind a store it cannot be proven not to alias; and
+// the next plane's lines are prefetched into L2, which needs no registers. What bounds these kernels
+// is the latency of those loads at 24 warps per SM (80 registers): at 400x400x120, batch 2, over the
+// whole grid H takes 0.31 ms and E 0.49 ms (4.5 and 4.1 TB/s of the measured 6.8; 0.32 and 0.52
+// without the prefetch at 16 planes). Three shapes measured and left: every component in one thread
+// (168 registers, 0.62 and 1.53 ms), one plane per thread (set-up dominates: 0.59 and 0.88 ms), one
+// body for all three components (600 instead of 300 instructions per vector in E).
+//
+// For every cell, in the reference's order (packages/oa-fdtd/src/oa_fdtd/reference.py:152-207,
+// :115-127):
 //   1. the bulk update (E: ca E + cb curl H; H: H + dt/mu0 curl E);
 //   2. the CPML corrections of the component in ascending derivative axis, each
 //      psi <- b psi + c d; F <- F + (sign k)(ek d + psi), with d the derivative the bulk update
 //      used and k = cb of the edge (E) or dt/mu0 (H);
 //   3. (E) the Debye update of dispersive edges: jt = 1/2 sum_p (1 + k_p) J_p;
-//      E^{n+1} = E - cbe jt; J_p = k_p J_p + beta_p (E^{n+1} - E^n). Dispersive edges that take an
-//      injection keep it for the edge pass, after the surface impedance and the injection.
+//      E^{n+1} = E - cbe jt; J_p = k_p J_p + beta_p (E^{n+1} - E^n);
+// In variant 0 the E launch also takes the edge list's edges (injection, and the Debye update of the
+// dispersive ones): a few blocks of one thread per edge do their whole update, and the vector
+// threads, which know those edges by table entries of their own past edge_lo, leave them out.
+// Elsewhere the edge pass does this after the sweeps.
 // The library is compiled without FMA contraction, so each product and sum rounds as in NumPy.
 //
 // psi layout, one array per (kind, component, axis, side): (B, Z', Y', X') with the slab width
@@ -24,465 +37,689 @@
 #include <algorithm>
 
 #include "device_common.cuh"
+#include "probe.cuh"
 
 namespace oafdtd {
 
-constexpr int kSlabThreads = 256;
-// Planes marched per thread. The slab boxes are thin (CPML slabs of ~10 cells): short marches
-// give the kernel enough independent threads to hide its load latency.
-constexpr int kSlabPlanes = 4;
+// A block: vector columns x 3 components (threadIdx.x, y).
+constexpr int kSlabCols = 64, kSlabThreads = 3 * kSlabCols;
 
-
+// One 16-byte vector of consecutive x cells: the cells a thread owns.
 template <typename real>
-__device__ __forceinline__ long long psi_index(const CpmlSide<real>& s, int ax, int b, int k, int j, int i, int X,
-                                               int Y, int Z) {
-  if (ax == 0) {
-    const int w = s.hi[0] - s.lo[0];
-    return (((long long)b * Z + k) * Y + j) * w + (i - s.lo[0]);
-  }
-  if (ax == 1) {
-    const int w = s.hi[1] - s.lo[1];
-    return (((long long)b * Z + k) * w + (j - s.lo[1])) * X + i;
-  }
-  const int w = s.hi[2] - s.lo[2];
-  return (((long long)b * w + (k - s.lo[2])) * Y + j) * X + i;
-}
-
-// psi of one correction term on one quad: the side whose box holds the quad's row (-1: none) and
-// the values. y and z slabs keep psi rows at the field pitch, so their quads are whole 16-byte
-// vectors (elements outside the box are written back unchanged); x slabs are read per element.
-template <typename real>
-struct PsiQuad {
-  Quad<real> v;
-  int sd;
+struct Vec {
+  static constexpr int n = 16 / (int)sizeof(real);
+  real v[n];
 };
-
 template <typename real>
-__device__ __forceinline__ const CpmlSide<real>& side_of(const CpmlTerm<real>& T, int sd) {
-  return sd == 0 ? T.side[0] : T.side[1];
+constexpr int kVec = Vec<real>::n;
+
+__device__ __forceinline__ Vec<float> ldv(const float* p) {
+  const float4 t = *reinterpret_cast<const float4*>(p);
+  return Vec<float>{{t.x, t.y, t.z, t.w}};
 }
-
+__device__ __forceinline__ Vec<double> ldv(const double* p) {
+  const double2 t = *reinterpret_cast<const double2*>(p);
+  return Vec<double>{{t.x, t.y}};
+}
+__device__ __forceinline__ void stv(float* p, const Vec<float>& q) {
+  *reinterpret_cast<float4*>(p) = make_float4(q.v[0], q.v[1], q.v[2], q.v[3]);
+}
+__device__ __forceinline__ void stv(double* p, const Vec<double>& q) {
+  *reinterpret_cast<double2*>(p) = make_double2(q.v[0], q.v[1]);
+}
+// The material indices of one vector of cells, packed.
 template <typename real>
-__device__ __forceinline__ void psi_load(const CpmlTerm<real>& T, PsiQuad<real>& P, int b, int k, int j, int i0,
-                                         int X, int Y, int Z) {
-  P.sd = -1;
-#pragma unroll
-  for (int sd = 0; sd < 2; ++sd) {
-    const CpmlSide<real>& s = T.side[sd];
-    if (P.sd >= 0 || s.psi == nullptr) continue;
-    if (j < s.lo[1] || j >= s.hi[1] || k < s.lo[2] || k >= s.hi[2] || i0 + 3 < s.lo[0] || i0 >= s.hi[0]) continue;
-    P.sd = sd;
-    if (T.axis == 0) {
-      const long long pq = psi_index(s, 0, b, k, j, i0, X, Y, Z);
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        P.v.v[e] = (i0 + e >= s.lo[0] && i0 + e < s.hi[0]) ? s.psi[pq + e] : (real)0;
-    } else {
-      P.v = ld4(s.psi + psi_index(s, T.axis, b, k, j, i0, X, Y, Z));
-    }
+struct Mats {
+  uint32_t w[kVec<real> / 2];
+  __device__ __forceinline__ int operator[](int e) const { return (int)((w[e / 2] >> (16 * (e & 1))) & 0xffffu); }
+  __device__ __forceinline__ bool same() const {
+    return w[0] == w[kVec<real> / 2 - 1] && (w[0] >> 16) == (w[0] & 0xffffu);
   }
+};
+__device__ __forceinline__ void ld_mat(const uint16_t* p, Mats<float>& m) {
+  const uint2 t = *reinterpret_cast<const uint2*>(p);
+  m.w[0] = t.x, m.w[1] = t.y;
 }
-
+__device__ __forceinline__ void ld_mat(const uint16_t* p, Mats<double>& m) { m.w[0] = *reinterpret_cast<const uint32_t*>(p); }
 template <typename real>
-__device__ __forceinline__ void psi_store(const CpmlTerm<real>& T, const PsiQuad<real>& P, int b, int k, int j,
-                                          int i0, int X, int Y, int Z) {
-  if (P.sd < 0) return;
-  const CpmlSide<real>& s = side_of(T, P.sd);
-  const long long pq = psi_index(s, T.axis, b, k, j, i0, X, Y, Z);
-  if (T.axis == 0) {
+__device__ __forceinline__ Vec<real> zerov() {
+  Vec<real> z;
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (i0 + e >= s.lo[0] && i0 + e < s.hi[0]) s.psi[pq + e] = P.v.v[e];
-  } else {
-    st4(s.psi + pq, P.v);
-  }
+  for (int e = 0; e < kVec<real>; ++e) z.v[e] = (real)0;
+  return z;
 }
 
-// One correction on a quad: psi <- b psi + c d; F <- F + (sign k)(ek d + psi) for the cells of
-// the box. The coefficient arrays are read-only for the whole run.
-template <typename real>
-__device__ __forceinline__ void psi_apply(const CpmlTerm<real>& T, PsiQuad<real>& P, const real* const (&co)[3][3],
-                                          Quad<real>& f, const real (&d)[4], const real (&kf)[4], int k, int j,
-                                          int i0) {
-  if (P.sd < 0) return;
-  const CpmlSide<real>& s = side_of(T, P.sd);
-  const int ax = T.axis;
-  const real* cb_ = co[ax][0];
-  const real* cc_ = co[ax][1];
-  const real* ck_ = co[ax][2];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = i0 + e;
-    if (i < s.lo[0] || i >= s.hi[0]) continue;
-    const int ia = ax == 0 ? i : (ax == 1 ? j : k);
-    real ps = P.v.v[e] * __ldg(cb_ + ia);
-    ps = ps + __ldg(cc_ + ia) * d[e];
-    P.v.v[e] = ps;
-    const real upd = __ldg(ck_ + ia) * d[e] + ps;
-    f.v[e] = f.v[e] + (T.sign * kf[e]) * upd;
-  }
+// n / f.d for n >= 0, by a multiplication where it is exact (the host sets m to 0 where it is not).
+__device__ __forceinline__ int fast_div(const FastDiv& f, int n) {
+  return f.m ? (int)__umulhi((unsigned)n, f.m) : n / f.d;
 }
 
-// Where a thread works: field component, member, box, quad column and plane range. The
-// component is the fastest-varying block index, so the three components of a region run side by
-// side and share their source-field reads through L1 and L2.
+// Where a thread works: member, storage row, first cell of its vector, planes; core: its cells lie in
+// no correction box.
 struct SlabWork {
-  int comp, b, j, i0, k0, k1;
-  bool live;
+  int b, j, i0, k0, k1;
+  bool live, core;
 };
 
-__device__ __forceinline__ SlabWork slab_work(const SlabLaunch& L, int nx, int block) {
-  const int blk = block / 3;
+template <typename real>
+__device__ __forceinline__ SlabWork slab_work(const SlabLaunch& L, int nx, int blk) {
+  constexpr int V = kVec<real>;
   int s = 0;
   while (s + 1 < L.n && blk >= L.first[s + 1]) ++s;
   const Span3 bx = L.box[s];
-  int r = blk - L.first[s];
-  const int cb = r % L.cblk[s];
-  r /= L.cblk[s];
-  const int ch = r % L.nch[s];
+  const int r = blk - L.first[s];
+  const int t = fast_div(L.cblk[s], r), cb = r - t * L.cblk[s].d;
   SlabWork w;
-  w.comp = block % 3;
-  w.b = r / L.nch[s];
-  const int nq = bx.q1 - bx.q0;
-  const int col = cb * kSlabThreads + (int)threadIdx.x;
-  const int ncol = nq * (bx.j1 - bx.j0);
-  const int c = min(col, ncol - 1);
-  w.j = bx.j0 + c / nq;
-  w.i0 = 4 * (bx.q0 + c % nq);
-  w.k0 = bx.k0 + ch * kSlabPlanes;
-  w.k1 = min(w.k0 + kSlabPlanes, bx.k1);
-  w.live = col < ncol && w.i0 <= nx + 1;
+  w.b = fast_div(L.nch[s], t);
+  const int ch = t - w.b * L.nch[s].d;
+  const int c = cb * kSlabCols + (int)threadIdx.x;
+  const int row = fast_div(L.nv[s], c);
+  w.j = bx.j0 + row;
+  w.i0 = 4 * bx.q0 + V * (c - row * L.nv[s].d);
+  w.k0 = bx.k0 + ch * L.planes;
+  w.k1 = min(w.k0 + L.planes, bx.k1);
+  w.live = w.j < bx.j1 && w.i0 <= nx + 1;
+  const Span3& o = L.core;
+  w.core = w.i0 >= 4 * o.q0 && w.i0 + V <= 4 * o.q1 && w.j >= o.j0 && w.j < o.j1 && w.k0 >= o.k0 && w.k1 <= o.k1;
   return w;
 }
 
-// ------------------------------------------------------------------------------------- E
-// Index of the Debye current of pole 0 at (b, k, j, i) in the dense (P, B, nzA, Y, X) array.
+// The cells of a vector from i0 on that lie in 1 .. last, one bit each.
 template <typename real>
-__device__ __forceinline__ long long jindex(const SweepArgs<real>& a, int c, int b, int k, int j, int i) {
-  return (((long long)b * a.jnk[c] + (k - a.jk0[c])) * a.Y + j) * a.X + i;
+__device__ __forceinline__ unsigned valid_cells(int i0, int last) {
+  constexpr int V = kVec<real>;
+  const int n = last - i0 + 1;  // cells up to the last
+  unsigned m = n >= V ? (1u << V) - 1u : (1u << n) - 1u;
+  return i0 == 0 ? m & ~1u : m;
 }
 
-// One E component on one quad column. Per plane: every load first (H, E, index, Debye current,
-// psi), then the arithmetic, then every store, so no load waits behind a store it cannot be proven
-// not to alias. C: 0 Ex (terms y +Hz, z -Hy), 1 Ey (z +Hx, x -Hz), 2 Ez (x +Hy, y -Hx); d0 is
-// the derivative along the first axis in ascending order, d1 along the second.
-// kMulti: more than one Debye pole (the general update, a call); single-pole runs compile without
-// it, so their registers never spill around the call.
-template <typename real, int C, bool kMulti>
-__device__ __forceinline__ void slab_e_column(const SweepArgs<real>& a, const SlabWork& w) {
-  const int X = a.X, Y = a.Y, Z = a.nz + 2, nx = a.nx, b = w.b, j = w.j, i0 = w.i0;
-  const long long sz = (long long)X * Y;
-  const long long base = (long long)b * a.bs;
-  const real* Hx = a.Ho[0] + base;  // H^{n+1/2}
-  const real* Hy = a.Ho[1] + base;
-  const real* Hz = a.Ho[2] + base;
-  const real* E = a.E[C] + base;     // E^n
-  real* Eo = a.Eo[C] + base;         // E^{n+1}
-  const Quad<real> idx4 = ld4(a.idd[0] + i0);
-  const real idy = a.idd[1][j];
-  long long q = (long long)w.k0 * sz + (long long)j * X + i0;  // offset within one member
-  // the z-derivative source at plane k - 1, carried (Ex: Hy, Ey: Hx)
-  Quad<real> hm = zero4<real>();
-  if (C == 0) hm = ld4(Hy + q - sz);
-  if (C == 1) hm = ld4(Hx + q - sz);
-  for (int k = w.k0; k < w.k1; ++k, q += sz) {
-    // ---- loads
-    Quad<real> s0, s1, s2;  // sources of the two derivatives
-    real sl = (real)0;      // x - 1 neighbour of element 0
-    if (C == 0) {
-      s0 = ld4(Hz + q);
-      s1 = ld4(Hz + q - X);
-      s2 = ld4(Hy + q);
-    } else if (C == 1) {
-      s0 = ld4(Hz + q);
-      if (i0 > 0) sl = Hz[q - 1];  // cell 0 is never updated: no neighbour from the row before
-      s2 = ld4(Hx + q);
-    } else {
-      s0 = ld4(Hy + q);
-      if (i0 > 0) sl = Hy[q - 1];
-      s2 = ld4(Hx + q);
-      s1 = ld4(Hx + q - X);
-    }
-    const Quad<uint16_t> m = ld4(a.mat[C] + q);
-    Quad<real> e4 = ld4(E + q);
-    const bool jrange = a.ade_P == 1 && k >= a.jk0[C] && k < a.jk0[C] + a.jnk[C];
-    Quad<real> j4 = zero4<real>();
-    if (jrange) j4 = ld4(a.J[C] + jindex(a, C, b, k, j, i0));
-    PsiQuad<real> ps[2];
-    ps[0].sd = ps[1].sd = -1;
-    if (a.has_cpml) {
-      psi_load<real>(a.ecorr[C][0], ps[0], b, k, j, i0, X, Y, Z);
-      psi_load<real>(a.ecorr[C][1], ps[1], b, k, j, i0, X, Y, Z);
-    }
-    // ---- arithmetic
-    real d0[4], d1[4];
-    const real idz = a.idd[2][k];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (C == 0) {
-        d0[e] = (s0.v[e] - s1.v[e]) * idy;  // y: Hz
-        d1[e] = (s2.v[e] - hm.v[e]) * idz;  // z: Hy
-      } else if (C == 1) {
-        const real l = e > 0 ? s0.v[e - 1] : sl;
-        d0[e] = (s0.v[e] - l) * idx4.v[e];  // x: Hz
-        d1[e] = (s2.v[e] - hm.v[e]) * idz;  // z: Hx
-      } else {
-        const real l = e > 0 ? s0.v[e - 1] : sl;
-        d0[e] = (s0.v[e] - l) * idx4.v[e];  // x: Hy
-        d1[e] = (s2.v[e] - s1.v[e]) * idy;  // y: Hx
-      }
-    }
-    const bool first_plus = C != 1;  // the reference's term order: (d0, -d1), for Ey (d1, -d0)
-    const Quad<real> e0 = e4;
-    real kf[4];
-    bool valid[4], dis[4];
-    bool disp = false;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + e;
-      const Coef<real> cf = ldg_coef(a.coef + m.v[e]);
-      kf[e] = cf.cb;
-      valid[e] = i >= 1 && i <= nx + 1;
-      const real acc = first_plus ? d0[e] + (-d1[e]) : d1[e] + (-d0[e]);
-      if (valid[e]) e4.v[e] = cf.ca * e4.v[e] + cf.cb * acc;
-      dis[e] = valid[e] && m.v[e] >= a.ade_lo && m.v[e] < a.ade_hi;
-      disp |= dis[e];
-    }
-    psi_apply<real>(a.ecorr[C][0], ps[0], a.pe, e4, d0, kf, k, j, i0);
-    psi_apply<real>(a.ecorr[C][1], ps[1], a.pe, e4, d1, kf, k, j, i0);
-    if (disp) {
-      if constexpr (!kMulti) {
-        const real onekp = a.ade_onekp[0], kp = a.ade_kp[0];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (!dis[e]) continue;
-          const Coef<real> cf = ldg_coef(a.coef + m.v[e]);  // the Debye coefficients (cbe, beta_0)
-          const real jt = (real)0.5 * (onekp * j4.v[e]);
-          const real en = e4.v[e] - cf.cbe * jt;
-          const real de = en - e0.v[e];
-          j4.v[e] = kp * j4.v[e] + cf.beta0 * de;
-          e4.v[e] = en;
-        }
-      } else {
-        const long long jstride = (long long)a.B * a.jnk[C] * Y * X;
-        const long long jq = jindex(a, C, b, k, j, i0);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (!dis[e]) continue;
-          const Coef<real> cf = ldg_coef(a.coef + m.v[e]);
-          e4.v[e] = ade_cell(e4.v[e], e0.v[e], cf.cbe, cf.beta0, m.v[e], a.J[C], jq + e, jstride, a.ade_kp,
-                             a.ade_onekp, a.ade_beta, a.ade_P);
-        }
-      }
-    }
-    // ---- stores
-    st4(Eo + q, e4);
-    if (!kMulti && disp) st4(a.J[C] + jindex(a, C, b, k, j, i0), j4);
-    psi_store<real>(a.ecorr[C][0], ps[0], b, k, j, i0, X, Y, Z);
-    psi_store<real>(a.ecorr[C][1], ps[1], b, k, j, i0, X, Y, Z);
-    if (C == 0) hm = s2;
-    if (C == 1) hm = s2;
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
+// ------------------------------------------------------------------------------------- CPML
+// One correction term of a component (AX: its derivative axis) on a thread's column, worked out once
+// for the march: psi of the march's first plane is at p, of the next a stride further on; `mask` holds
+// the vector's cells inside the box (low bits) and, from bit 8, the march's planes inside it (0: no
+// slab of this term holds the column). A march meets at most one side of an axis (slab_plan sees to
+// it in z). y and z slabs keep psi rows at the field pitch, so their vectors are whole 16 bytes
+// (elements outside the box are written back unchanged); x slabs are read per element.
+template <typename real>
+struct PsiCol {
+  real* p;
+  int stride;
+  unsigned mask;
+};
+
+template <typename real, int AX>
+__device__ __forceinline__ void psi_column(const CpmlTerm<real>& T, PsiCol<real>& c, const SlabWork& w, int X, int Y,
+                                           int Z) {
+  constexpr int V = kVec<real>;
+  c.mask = 0;
+  c.p = nullptr;
+  c.stride = 0;
+  if (w.core) return;
+#pragma unroll 1
+  for (int sd = 0; sd < 2; ++sd) {
+    const CpmlSide<real>& s = T.side[sd];
+    if (s.psi == nullptr || w.i0 + V <= s.lo[0] || w.i0 >= s.hi[0] || w.j < s.lo[1] || w.j >= s.hi[1] ||
+        w.k1 <= s.lo[2] || w.k0 >= s.hi[2])
+      continue;
+    const int wd = s.hi[AX] - s.lo[AX];
+    c.stride = AX == 0 ? Y * wd : (AX == 1 ? wd * X : Y * X);
+    c.p = AX == 0   ? s.psi + (((long long)w.b * Z + w.k0) * Y + w.j) * wd + (w.i0 - s.lo[0])
+          : AX == 1 ? s.psi + (((long long)w.b * Z + w.k0) * wd + (w.j - s.lo[1])) * X + w.i0
+                    : s.psi + (((long long)w.b * wd + w.k0 - s.lo[2]) * Y + w.j) * X + w.i0;
+    const int lo = max(s.lo[0] - w.i0, 0), hi = min(s.hi[0] - w.i0, V);
+    const int klo = max(s.lo[2] - w.k0, 0), khi = min(s.hi[2], w.k1) - w.k0;
+    c.mask = (((1u << hi) - 1u) & ~((1u << lo) - 1u)) | ((((1u << khi) - 1u) & ~((1u << klo) - 1u)) << 8);
+    return;
   }
 }
 
+// psi of plane t of the march (false: the plane has none of this term); the march moves p on by the
+// stride after each plane.
+template <typename real, int AX>
+__device__ __forceinline__ bool psi_load(const PsiCol<real>& c, Vec<real>& v, int t) {
+  if (!((c.mask >> (8 + t)) & 1)) return false;
+  if constexpr (AX == 0) {
+#pragma unroll
+    for (int e = 0; e < kVec<real>; ++e) v.v[e] = ((c.mask >> e) & 1) ? c.p[e] : (real)0;
+  } else {
+    v = ldv(c.p);
+  }
+  return true;
+}
+
+// psi <- b psi + c d; F <- F + (sign k)(ek d + psi) for the cells of the box, kf(e) the factor k of
+// cell e; the updated psi back. The coefficient arrays are read-only for the whole run.
+template <typename real, int AX, typename KF>
+__device__ __forceinline__ void psi_apply(const PsiCol<real>& c, Vec<real>& v, const real* const (&co)[3], real sign,
+                                          Vec<real>& f, const Vec<real>& d, KF kf, const SlabWork& w, int k) {
+  Vec<real> cb, cc, ck;
+  if constexpr (AX == 0) {
+    cb = ldv(co[0] + w.i0), cc = ldv(co[1] + w.i0), ck = ldv(co[2] + w.i0);
+  } else {
+    const int ia = AX == 1 ? w.j : k;
+    const real b = __ldg(co[0] + ia), cv = __ldg(co[1] + ia), kv = __ldg(co[2] + ia);
+#pragma unroll
+    for (int e = 0; e < kVec<real>; ++e) cb.v[e] = b, cc.v[e] = cv, ck.v[e] = kv;
+  }
+#pragma unroll
+  for (int e = 0; e < kVec<real>; ++e) {
+    if (!((c.mask >> e) & 1)) continue;
+    real ps = v.v[e] * cb.v[e];
+    ps = ps + cc.v[e] * d.v[e];
+    v.v[e] = ps;
+    const real upd = ck.v[e] * d.v[e] + ps;
+    f.v[e] = f.v[e] + (sign * kf(e)) * upd;
+  }
+  if constexpr (AX == 0) {
+#pragma unroll
+    for (int e = 0; e < kVec<real>; ++e)
+      if ((c.mask >> e) & 1) c.p[e] = v.v[e];
+  } else {
+    stv(c.p, v);
+  }
+}
+
+// ------------------------------------------------------------------------------------- E
+// One edge of the edge list for one member, whole: bulk update, injection (reference.py:223-234),
+// Debye update. The vector threads leave these edges (and their currents) alone, so nothing else
+// writes them; the host keeps edges in CPML boxes and on copper to the edge pass.
+template <typename real>
+__device__ __forceinline__ void list_edge(const SweepArgs<real>& a, const EdgeArgs<real>& ed, int off, int t) {
+  const int n = t % ed.n, b = t / ed.n;
+  const int c = ed.comp[n], X = a.X;
+  const int q = (int)ed.flat[n], sz = X * a.Y;
+  const int k = q / sz, j = (q - k * sz) / X, i = q - k * sz - j * X;
+  const long long base = (long long)b * a.bs;
+  const real* Hx = a.Ho[0] + base + q;
+  const real* Hy = a.Ho[1] + base + q;
+  const real* Hz = a.Ho[2] + base + q;
+  const int m = a.mat[c][q];
+  const Coef<real> cf = ldg_coef(a.coef + m);
+  const real e0 = a.E[c][base + q];
+  real val = e0;
+  if (i >= 1 && i <= a.nx + 1 && j >= 1 && j <= a.ny + 1 && k >= 1 && k <= a.nz + 1) {
+    real d0, d1;
+    if (c == 0) {
+      d0 = (Hz[0] - Hz[-X]) * a.idd[1][j];
+      d1 = (Hy[0] - Hy[-sz]) * a.idd[2][k];
+    } else if (c == 1) {
+      d0 = (Hz[0] - Hz[-1]) * a.idd[0][i];
+      d1 = (Hx[0] - Hx[-sz]) * a.idd[2][k];
+    } else {
+      d0 = (Hy[0] - Hy[-1]) * a.idd[0][i];
+      d1 = (Hx[0] - Hx[-X]) * a.idd[1][j];
+    }
+    const real acc = c != 1 ? d0 + (-d1) : d1 + (-d0);
+    val = cf.ca * val + cf.cb * acc;
+  }
+  const long long step = *ed.step_base + off;
+  const int ie = ed.inj_end[n];
+#pragma unroll 1
+  for (int s = ed.inj_beg[n]; s < ie; ++s) {
+    const int ch = ed.i_chan[s];
+    const double w = ed.wave[(long long)ch * ed.max_steps + step];
+    val = val + (real)((ed.drive[b * ed.n_chan + ch] * w) * ed.i_amp[s]);
+  }
+  if (ed.def_slot[n] >= 0) {
+    const int P = a.ade_P;
+    const long long js = (long long)a.B * a.jnk[c] * sz;
+    real* J = a.J[c] + ((long long)b * a.jnk[c] - a.jk0[c]) * sz + q;
+    real jt = (real)0;
+#pragma unroll 1
+    for (int p = 0; p < P; ++p) jt = jt + a.ade_onekp[p] * J[p * js];
+    jt = (real)0.5 * jt;
+    const real en = val - cf.cbe * jt;
+    const real de = en - e0;
+#pragma unroll 1
+    for (int p = 0; p < P; ++p) {
+      const real bp = p == 0 ? cf.beta0 : a.ade_beta[(long long)m * P + p];
+      J[p * js] = a.ade_kp[p] * J[p * js] + bp * de;
+    }
+    val = en;
+  }
+  a.Eo[c][base + q] = val;
+}
+
+// Stores a vector; the elements of the edge list's edges stay out (listed: there are some).
+template <typename real>
+__device__ __forceinline__ void st_unlisted(real* p, const Vec<real>& v, const Mats<real>& m, int edge_lo, bool listed) {
+  if (!listed) {
+    stv(p, v);
+  } else {
+#pragma unroll
+    for (int e = 0; e < kVec<real>; ++e)
+      if (m[e] < edge_lo) p[e] = v.v[e];
+  }
+}
+
+// One E component on one vector column. Per plane every load first (H, E, indices, Debye current,
+// psi), then the arithmetic, then every store. C: 0 Ex (terms y +Hz, z -Hy), 1 Ey (z +Hx, x -Hz),
+// 2 Ez (x +Hy, y -Hx). kMulti: more than one Debye pole; the currents of each pole are then read
+// twice (the second time from the L1 cache).
+template <typename real, int C, bool kMulti>
+__device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inject, const SlabWork& w) {
+  constexpr int V = kVec<real>;
+  constexpr int A0 = C == 0 ? 1 : 0, A1 = C == 2 ? 1 : 2;  // the derivative axes, ascending
+  // Vectors whose cells have several table entries: a branch of their own in float32 (one gather and
+  // four registers serve the rest); in float64 both branches would issue their arithmetic wherever
+  // a warp holds both, and the two float64 operations a clock and SM bound the kernel (0.51 against
+  // 0.46 ms for E at 161x143x88, batch 2): there every cell has its entry.
+  constexpr bool kBranch = sizeof(real) == 4;
+  const int X = a.X, Y = a.Y, i0 = w.i0, sz = X * Y;
+  const long long base = (long long)w.b * a.bs;
+  const real* const s0 = a.Ho[C == 2 ? 1 : 2] + base;  // sources along A0 and A1: H^{n+1/2}
+  const real* const s1 = a.Ho[C == 0 ? 1 : 0] + base;
+  const real* const E = a.E[C] + base;                 // E^n
+  real* const Eo = a.Eo[C] + base;                     // E^{n+1}
+  real* const J = a.J[C] + (long long)(w.b * a.jnk[C] - a.jk0[C]) * sz;
+  const int jlo = a.ade_P > 0 ? a.jk0[C] : 1 << 30, jhi = a.jk0[C] + a.jnk[C];
+  const uint16_t* const mat = a.mat[C];
+  Vec<real> wx;
+  if (C != 0) wx = ldv(a.idd[0] + i0);
+  const real wy = a.idd[1][w.j];
+  const unsigned vm = valid_cells<real>(i0, a.nx + 1);
+  PsiCol<real> c0, c1;
+  psi_column<real, A0>(a.ecorr[C][0], c0, w, X, Y, a.nz + 2);
+  psi_column<real, A1>(a.ecorr[C][1], c1, w, X, Y, a.nz + 2);
+  int q = (w.k0 * Y + w.j) * X + i0;  // offset within one member (below 2^31)
+  Vec<real> below;                    // the z-derivative's source on the plane below, carried
+  if (C != 2) below = ldv(s1 + (q - sz));
+#pragma unroll 1
+  for (int k = w.k0; k < w.k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride) {
+    // ---- loads
+    Mats<real> m;
+    ld_mat(mat + q, m);
+    const Vec<real> e0 = ldv(E + q);
+    const Vec<real> u0 = ldv(s0 + q), u1 = ldv(s1 + q);
+    Vec<real> n0, n1;      // the neighbours one down along A0 (y) and A1 (y); z is carried
+    real x0 = (real)0;     // along x only element 0's; cell 0 is never updated: none from the row before
+    if (C == 0) n0 = ldv(s0 + (q - X));
+    else if (i0 > 0) x0 = s0[q - 1];
+    if (C == 2) n1 = ldv(s1 + (q - X));
+    else n1 = below;
+    Vec<real> j4, p0, p1;
+    const bool debye = k >= jlo && k < jhi;
+    if (!kMulti && debye) j4 = ldv(J + q);
+    const bool on0 = psi_load<real, A0>(c0, p0, k - w.k0), on1 = psi_load<real, A1>(c1, p1, k - w.k0);
+    const real w1 = C == 2 ? wy : a.idd[2][k];
+    if (k + 1 < w.k1) {
+      prefetch_l2(mat + (q + sz));
+      prefetch_l2(E + (q + sz));
+      prefetch_l2(s0 + (q + sz));
+      prefetch_l2(s1 + (q + sz));
+      if (k + 1 >= jlo && k + 1 < jhi) prefetch_l2(J + (q + sz));
+    }
+    if (C != 2) below = u1;
+    // ---- bulk update: d0 along A0, d1 along A1. The cells of a vector mostly share a table entry: one
+    // gather then serves all of them
+    Vec<real> d0, d1, f = e0;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      d0.v[e] = C == 0 ? (u0.v[e] - n0.v[e]) * wy : (u0.v[e] - (e > 0 ? u0.v[e > 0 ? e - 1 : 0] : x0)) * wx.v[e];
+      d1.v[e] = (u1.v[e] - n1.v[e]) * w1;
+    }
+    auto acc = [&](int e) { return C != 1 ? d0.v[e] + (-d1.v[e]) : d1.v[e] + (-d0.v[e]); };
+    const int m0 = m[0];
+    const Coef<real> cf0 = ldg_coef(a.coef + m0);
+    const bool same = m.same();
+    unsigned dis = m0 >= a.ade_lo && m0 < a.ade_hi ? vm : 0u;
+    bool listed = m0 >= a.edge_lo;
+    Coef<real> cfd[kBranch ? 1 : V];
+    if constexpr (!kBranch) {
+      cfd[0] = cf0;
+#pragma unroll
+      for (int e = 1; e < V; ++e) {
+        cfd[e] = cf0;
+        if (m[e] != m0) cfd[e] = ldg_coef(a.coef + m[e]);
+      }
+    }
+    auto coef = [&](int e) {
+      if constexpr (!kBranch) return cfd[e];
+      else return same ? cf0 : ldg_coef(a.coef + m[e]);
+    };
+    if (same || !kBranch) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const Coef<real> cf = kBranch ? cf0 : cfd[kBranch ? 0 : e];
+        if ((vm >> e) & 1) f.v[e] = cf.ca * f.v[e] + cf.cb * acc(e);
+      }
+    }
+    if (!same) {
+      dis = 0;
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        if constexpr (kBranch) {
+          const Coef<real> cf = ldg_coef(a.coef + m[e]);
+          if ((vm >> e) & 1) f.v[e] = cf.ca * f.v[e] + cf.cb * acc(e);
+        }
+        if (m[e] >= a.ade_lo && m[e] < a.ade_hi) dis |= vm & (1u << e);
+        listed |= m[e] >= a.edge_lo;
+      }
+    }
+    listed = listed && inject;
+    // ---- corrections
+    auto kf = [&](int e) { return coef(e).cb; };
+    if (on0) psi_apply<real, A0>(c0, p0, a.pe[A0], a.ecorr[C][0].sign, f, d0, kf, w, k);
+    if (on1) psi_apply<real, A1>(c1, p1, a.pe[A1], a.ecorr[C][1].sign, f, d1, kf, w, k);
+    // ---- Debye
+    if (dis) {
+      if constexpr (!kMulti) {
+        const real onekp = a.ade_onekp[0], kp = a.ade_kp[0];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          if (!((dis >> e) & 1)) continue;
+          const Coef<real> cf = coef(e);
+          const real jt = (real)0.5 * (onekp * j4.v[e]);
+          const real en = f.v[e] - cf.cbe * jt;
+          const real de = en - e0.v[e];
+          j4.v[e] = kp * j4.v[e] + cf.beta0 * de;
+          f.v[e] = en;
+        }
+        st_unlisted<real>(J + q, j4, m, a.edge_lo, listed);
+      } else {
+        const long long js = (long long)a.B * a.jnk[C] * sz;
+        const int P = a.ade_P;
+        Vec<real> jt = zerov<real>(), de;
+#pragma unroll 4
+        for (int p = 0; p < P; ++p) {
+          const Vec<real> jp = ldv(J + q + p * js);
+          const real onekp = a.ade_onekp[p];
+#pragma unroll
+          for (int e = 0; e < V; ++e) jt.v[e] = jt.v[e] + onekp * jp.v[e];
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const real en = f.v[e] - coef(e).cbe * ((real)0.5 * jt.v[e]);
+          de.v[e] = en - e0.v[e];
+          if ((dis >> e) & 1) f.v[e] = en;
+        }
+#pragma unroll 2
+        for (int p = 0; p < P; ++p) {
+          Vec<real> jp = ldv(J + q + p * js);
+          const real kp = a.ade_kp[p], b0 = __ldg(a.ade_beta + m0 * P + p);
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            real bp = b0;
+            if (e > 0 && m[e] != m0) bp = __ldg(a.ade_beta + m[e] * P + p);
+            if ((dis >> e) & 1) jp.v[e] = kp * jp.v[e] + bp * de.v[e];
+          }
+          st_unlisted<real>(J + q + p * js, jp, m, a.edge_lo, listed);
+        }
+      }
+    }
+    st_unlisted<real>(Eo + q, f, m, a.edge_lo, listed);
+  }
+}
+
+// The E boxes; the first L.extra blocks sample the H probes of the step instead (H is complete), the
+// next L.inject blocks take the edge list's edges.
 template <typename real, bool kMulti>
-__device__ __forceinline__ void slab_e_body(const SweepArgs<real>& a, const SlabLaunch& L, int block) {
-  const SlabWork w = slab_work(L, a.nx, block);
-  if (!w.live || w.k0 >= w.k1) return;
-  if (w.comp == 0)
-    slab_e_column<real, 0, kMulti>(a, w);
-  else if (w.comp == 1)
-    slab_e_column<real, 1, kMulti>(a, w);
-  else
-    slab_e_column<real, 2, kMulti>(a, w);
+__device__ __forceinline__ void slab_e_body(const SweepArgs<real>& a, const SlabLaunch& L, const EdgeArgs<real>& ed,
+                                            const ProbeArgs<real>& pr, int off, int block) {
+  if (block < L.extra) {
+    probe_sample(pr, 1, block, off);
+    return;
+  }
+  block -= L.extra;
+  if (block < L.inject) {
+    const int t = block * kSlabThreads + (int)(threadIdx.x + kSlabCols * threadIdx.y);
+    if (t < ed.n * a.B) list_edge<real>(a, ed, off, t);
+    return;
+  }
+  const SlabWork w = slab_work<real>(L, a.nx, block - L.inject);
+  if (!w.live) return;
+  const bool inject = L.inject > 0;
+  if (threadIdx.y == 0) slab_e_march<real, 0, kMulti>(a, inject, w);
+  else if (threadIdx.y == 1) slab_e_march<real, 1, kMulti>(a, inject, w);
+  else slab_e_march<real, 2, kMulti>(a, inject, w);
 }
 
 template <typename real, bool kMulti>
-__global__ void __launch_bounds__(kSlabThreads, 3)
-    slab_e_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L) {
-  slab_e_body<real, kMulti>(a, L, (int)blockIdx.x);
+__global__ void __launch_bounds__(kSlabThreads, 4)
+    slab_e_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L,
+                  const __grid_constant__ EdgeArgs<real> ed, const __grid_constant__ ProbeArgs<real> pr, int off) {
+  slab_e_body<real, kMulti>(a, L, ed, pr, off, (int)blockIdx.x);
 }
 
-// Several engines' E slab updates in one launch: engine e's arguments at A[e] and L[e].
+// Several engines' E updates in one launch: engine e's arguments at A[e], L[e], ED[e] and PR[e].
 template <typename real, bool kMulti>
-__global__ void __launch_bounds__(kSlabThreads, 3)
-    slab_e_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L, const BatchGrid G) {
+__global__ void __launch_bounds__(kSlabThreads, 4)
+    slab_e_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L,
+                        const EdgeArgs<real>* __restrict__ ED, const ProbeArgs<real>* __restrict__ PR, const BatchGrid G,
+                        int off) {
   __shared__ __align__(16) unsigned char args[sizeof(SweepArgs<real>)];
   __shared__ __align__(16) unsigned char launch[sizeof(SlabLaunch)];
   int e;
   const uint3 bid = G.block(&e);
   const SlabLaunch& l = stage_args(L + e, launch);
-  slab_e_body<real, kMulti>(stage_args(A + e, args), l, (int)bid.x);
+  slab_e_body<real, kMulti>(stage_args(A + e, args), l, ED[e], PR[e], off, (int)bid.x);
 }
 
 // ------------------------------------------------------------------------------------- H
-// One H component on one quad column. C: 0 Hx (terms y -Ez, z +Ey), 1 Hy (z -Ex, x +Ez),
-// 2 Hz (x -Ey, y +Ex); d0 along the first axis in ascending order, d1 along the second.
+// One H component on one vector column. C: 0 Hx (terms y -Ez, z +Ey), 1 Hy (z -Ex, x +Ez), 2 Hz
+// (x -Ey, y +Ex). The cells each updates: Hx i in 1..nx+1, j <= ny, k <= nz; Hy i <= nx, k <= nz; Hz
+// i <= nx, j <= ny.
 template <typename real, int C>
-__device__ __forceinline__ void slab_h_column(const SweepArgs<real>& a, const SlabWork& w) {
-  const int X = a.X, Y = a.Y, Z = a.nz + 2, nx = a.nx, ny = a.ny, nz = a.nz, b = w.b, j = w.j, i0 = w.i0;
-  // the cells this component updates: Hx i in 1..nx+1, j <= ny, k <= nz; Hy i <= nx, k <= nz;
-  // Hz i <= nx, j <= ny
-  if ((C == 0 || C == 2) && j > ny) return;
-  const int ilast = C == 0 ? nx + 1 : nx;
-  const long long sz = (long long)X * Y;
-  const long long base = (long long)b * a.bs;
-  const real* Ex = a.E[0] + base;
-  const real* Ey = a.E[1] + base;
-  const real* Ez = a.E[2] + base;
-  const real* H = a.H[C] + base;  // H^{n-1/2}
-  real* Ho = a.Ho[C] + base;      // H^{n+1/2}
-  const Quad<real> ipx = ld4(a.ip[0] + i0);
-  const real ipy = a.ip[1][j];
-  const bool right = i0 + 4 < X;  // the x + 1 neighbour of element 3 is in the row
+__device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const SlabWork& w) {
+  constexpr int V = kVec<real>;
+  constexpr int A0 = C == 0 ? 1 : 0, A1 = C == 2 ? 1 : 2;  // the derivative axes, ascending
+  if (C != 1 && w.j > a.ny) return;
+  const int k1 = C == 2 ? w.k1 : min(w.k1, a.nz + 1);
+  const int X = a.X, Y = a.Y, i0 = w.i0, sz = X * Y;
+  const long long base = (long long)w.b * a.bs;
+  const real* const s0 = a.E[C == 2 ? 1 : 2] + base;  // sources along A0 and A1
+  const real* const s1 = a.E[C == 0 ? 1 : 0] + base;
+  const real* const H = a.H[C] + base;                // H^{n-1/2}
+  real* const Ho = a.Ho[C] + base;                    // H^{n+1/2}
+  Vec<real> wx;
+  if (C != 0) wx = ldv(a.ip[0] + i0);
+  const real wy = a.ip[1][w.j];
+  const bool right = i0 + V < X;  // the x + 1 neighbour of the last element is in the row
+  const unsigned vm = valid_cells<real>(i0, C == 0 ? a.nx + 1 : a.nx);
   const real dtmu = a.dtmu;
-  long long q = (long long)w.k0 * sz + (long long)j * X + i0;
-  // the z-derivative source at plane k, carried from the previous plane's k + 1 (Hx: Ey, Hy: Ex)
-  Quad<real> sc = zero4<real>();
-  if (C == 0) sc = ld4(Ey + q);
-  if (C == 1) sc = ld4(Ex + q);
-  for (int k = w.k0; k < w.k1; ++k, q += sz) {
-    if (C != 2 && k > nz) break;
+  PsiCol<real> c0, c1;
+  psi_column<real, A0>(a.hcorr[C][0], c0, w, X, Y, a.nz + 2);
+  psi_column<real, A1>(a.hcorr[C][1], c1, w, X, Y, a.nz + 2);
+  int q = (w.k0 * Y + w.j) * X + i0;
+  Vec<real> here;  // the z-derivative's source on this plane, carried from the last one's plane above
+  if (C != 2) here = ldv(s1 + q);
+#pragma unroll 1
+  for (int k = w.k0; k < k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride) {
     // ---- loads
-    Quad<real> s0, s1, s2;
-    real sr = (real)0;  // x + 1 neighbour of element 3
-    if (C == 0) {
-      s0 = ld4(Ez + q + X);   // y: Ez(j + 1)
-      s1 = ld4(Ez + q);
-      s2 = ld4(Ey + q + sz);  // z: Ey(k + 1)
-    } else if (C == 1) {
-      s0 = ld4(Ez + q);       // x: Ez
-      sr = right ? Ez[q + 4] : (real)0;
-      s2 = ld4(Ex + q + sz);  // z: Ex(k + 1)
+    Vec<real> h = ldv(H + q);
+    const Vec<real> u0 = ldv(s0 + q);
+    Vec<real> n0, u1, n1;  // the neighbours one up along A0 (y) and A1 (z, y)
+    real x0 = (real)0;     // along x only the last element's
+    if (C == 0) n0 = ldv(s0 + (q + X));
+    else if (right) x0 = s0[q + V];
+    if (C == 2) {
+      u1 = ldv(s1 + q);
+      n1 = ldv(s1 + (q + X));
     } else {
-      s0 = ld4(Ey + q);       // x: Ey
-      sr = right ? Ey[q + 4] : (real)0;
-      s2 = ld4(Ex + q + X);   // y: Ex(j + 1)
-      s1 = ld4(Ex + q);
+      u1 = here;
+      n1 = ldv(s1 + (q + sz));
+      here = n1;
     }
-    Quad<real> h = ld4(H + q);
-    PsiQuad<real> ps[2];
-    ps[0].sd = ps[1].sd = -1;
-    if (a.has_cpml) {
-      psi_load<real>(a.hcorr[C][0], ps[0], b, k, j, i0, X, Y, Z);
-      psi_load<real>(a.hcorr[C][1], ps[1], b, k, j, i0, X, Y, Z);
+    Vec<real> p0, p1;
+    const bool on0 = psi_load<real, A0>(c0, p0, k - w.k0), on1 = psi_load<real, A1>(c1, p1, k - w.k0);
+    const real w1 = C == 2 ? wy : a.ip[2][k];
+    if (k + 1 < k1) {
+      prefetch_l2(H + (q + sz));
+      prefetch_l2(s0 + (q + sz));
+      if (C == 2) prefetch_l2(s1 + (q + sz));
+      else if (k + 2 < a.nz + 2) prefetch_l2(s1 + (q + 2 * sz));
     }
-    // ---- arithmetic
-    const real ipz = a.ip[2][k];
-    real d0[4], d1[4], kf[4];
+    // ---- arithmetic: d0 along A0, d1 along A1
+    Vec<real> d0, d1;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      real acc;
-      if (C == 0) {
-        d0[e] = (s0.v[e] - s1.v[e]) * ipy;  // y
-        d1[e] = (s2.v[e] - sc.v[e]) * ipz;  // z
-        acc = (-d0[e]) + d1[e];
-      } else if (C == 1) {
-        const real r = e < 3 ? s0.v[e + 1] : sr;
-        d0[e] = (r - s0.v[e]) * ipx.v[e];   // x
-        d1[e] = (s2.v[e] - sc.v[e]) * ipz;  // z
-        acc = (-d1[e]) + d0[e];
-      } else {
-        const real r = e < 3 ? s0.v[e + 1] : sr;
-        d0[e] = (r - s0.v[e]) * ipx.v[e];   // x
-        d1[e] = (s2.v[e] - s1.v[e]) * ipy;  // y
-        acc = (-d0[e]) + d1[e];
-      }
-      const int i = i0 + e;
-      kf[e] = dtmu;
-      if (i >= 1 && i <= ilast) h.v[e] = h.v[e] + dtmu * acc;
+    for (int e = 0; e < V; ++e) {
+      d0.v[e] = C == 0 ? (n0.v[e] - u0.v[e]) * wy
+                       : ((e < V - 1 ? u0.v[e < V - 1 ? e + 1 : e] : x0) - u0.v[e]) * wx.v[e];
+      d1.v[e] = (n1.v[e] - u1.v[e]) * w1;
+      const real acc = C == 1 ? (-d1.v[e]) + d0.v[e] : (-d0.v[e]) + d1.v[e];
+      if ((vm >> e) & 1) h.v[e] = h.v[e] + dtmu * acc;
     }
-    psi_apply<real>(a.hcorr[C][0], ps[0], a.ph, h, d0, kf, k, j, i0);
-    psi_apply<real>(a.hcorr[C][1], ps[1], a.ph, h, d1, kf, k, j, i0);
-    // ---- stores
-    st4(Ho + q, h);
-    psi_store<real>(a.hcorr[C][0], ps[0], b, k, j, i0, X, Y, Z);
-    psi_store<real>(a.hcorr[C][1], ps[1], b, k, j, i0, X, Y, Z);
-    if (C != 2) sc = s2;
+    auto kf = [&](int) { return dtmu; };
+    if (on0) psi_apply<real, A0>(c0, p0, a.ph[A0], a.hcorr[C][0].sign, h, d0, kf, w, k);
+    if (on1) psi_apply<real, A1>(c1, p1, a.ph[A1], a.hcorr[C][1].sign, h, d1, kf, w, k);
+    stv(Ho + q, h);
   }
 }
 
 template <typename real>
 __device__ __forceinline__ void slab_h_body(const SweepArgs<real>& a, const SlabLaunch& L, int block) {
-  const SlabWork w = slab_work(L, a.nx, block);
-  if (!w.live || w.k0 >= w.k1) return;
-  if (w.comp == 0)
-    slab_h_column<real, 0>(a, w);
-  else if (w.comp == 1)
-    slab_h_column<real, 1>(a, w);
-  else
-    slab_h_column<real, 2>(a, w);
+  const SlabWork w = slab_work<real>(L, a.nx, block);
+  if (!w.live) return;
+  if (threadIdx.y == 0) slab_h_march<real, 0>(a, w);
+  else if (threadIdx.y == 1) slab_h_march<real, 1>(a, w);
+  else slab_h_march<real, 2>(a, w);
 }
 
+// The H boxes; the first L.extra blocks sample the E probes of the previous step instead (the H
+// update leaves E alone; off - 1 is that step).
 template <typename real>
 __global__ void __launch_bounds__(kSlabThreads, 4)
-    slab_h_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L) {
-  slab_h_body<real>(a, L, (int)blockIdx.x);
+    slab_h_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L,
+                  const __grid_constant__ ProbeArgs<real> pr, int off) {
+  if ((int)blockIdx.x < L.extra) {
+    probe_sample(pr, 0, (int)blockIdx.x, off - 1);
+    return;
+  }
+  slab_h_body<real>(a, L, (int)blockIdx.x - L.extra);
 }
 
-// Several engines' H slab updates in one launch.
+// Several engines' H updates in one launch. The E probes of a step before the first of a group
+// (off 0) are already in: those blocks return.
 template <typename real>
 __global__ void __launch_bounds__(kSlabThreads, 4)
-    slab_h_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L, const BatchGrid G) {
+    slab_h_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L,
+                        const ProbeArgs<real>* __restrict__ PR, const BatchGrid G, int off) {
   __shared__ __align__(16) unsigned char args[sizeof(SweepArgs<real>)];
   __shared__ __align__(16) unsigned char launch[sizeof(SlabLaunch)];
   int e;
   const uint3 bid = G.block(&e);
   const SlabLaunch& l = stage_args(L + e, launch);
-  slab_h_body<real>(stage_args(A + e, args), l, (int)bid.x);
+  if ((int)bid.x < l.extra) {
+    if (off > 0) probe_sample(PR[e], 0, (int)bid.x, off - 1);
+    return;
+  }
+  slab_h_body<real>(stage_args(A + e, args), l, (int)bid.x - l.extra);
 }
 
 // ------------------------------------------------------------------------------------- launch
+// The divisor d for operands below `limit`: ceil(2^32 / d) divides exactly by the high half of a
+// multiplication where limit * (its excess over 2^32) stays below 2^32.
+static FastDiv fast_divisor(long long d, long long limit) {
+  FastDiv f{(int)d, 0};
+  const unsigned long long m = ((1ull << 32) + (unsigned long long)d - 1) / (unsigned long long)d;
+  const unsigned long long excess = m * (unsigned long long)d - (1ull << 32);
+  if (d > 1 && (unsigned long long)limit * std::max(excess, 1ull) < (1ull << 32)) f.m = (unsigned)m;
+  return f;
+}
+
+// Vectors of the boxes of one kind, all members.
 template <typename real>
-cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long long* blocks) {
+long long slab_vecs(const SweepArgs<real>& a, int kind) {
+  long long n = 0;
+  for (int s = 0; s < a.n_slab[kind]; ++s) {
+    const Span3& bx = a.slab[kind][s];
+    const long long q = std::min(bx.q1, (a.nx + 1) / 4 + 1) - bx.q0;
+    if (q > 0 && bx.j1 > bx.j0 && bx.k1 > bx.k0) n += q * (4 / kVec<real>)*(bx.j1 - bx.j0) * (bx.k1 - bx.k0) * a.B;
+  }
+  return n;
+}
+
+// Planes a thread marches in a launch over `vecs` vectors. A thread's set-up (its place, the CPML
+// columns) costs about one plane's work, so long marches pay as long as the blocks still fill the
+// chip: 4 blocks of 192 threads per SM, 608 of them, run at once. us per step by planes (1, 2, 4, 8,
+// 16), both sweeps over the whole grid: 6.7 thousand vectors 11 / 12 / 15 / 22 / 35; 155 thousand
+// 28 / 23 / 22 / 26 / 39; 510 thousand 93 / 76 / 71 / 71 / 80; 1.2 million 224 / 182 / 159 / 150 /
+// 154; 9.9 million 1632 / 1234 / 1013 / 920 / 886; a batch of 16 instances, 4.9 million together,
+// 1138 / 812 / 642 / 552 / 521.
+int slab_planes(long long vecs) {
+  const long long blocks = vecs / kSlabCols;  // with one plane each
+  return blocks >= 16 * 2400 ? 16 : (blocks >= 8 * 900 ? 8 : (blocks >= 4 * 600 ? 4 : (blocks >= 2 * 600 ? 2 : 1)));
+}
+
+template <typename real>
+cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long long* blocks, int planes) {
   *L = SlabLaunch{};
-  L->n = 0;
   *blocks = 0;
+  L->core = a.core[kind];
+  L->planes = planes > 0 ? planes : slab_planes(slab_vecs(a, kind));
+  // no march may meet both z slabs of a term (a thread keeps one side's psi)
+  for (int c = 0; c < 3; ++c)
+    for (int t = 0; t < 2; ++t) {
+      const CpmlTerm<real>& T = kind == 0 ? a.ecorr[c][t] : a.hcorr[c][t];
+      if (T.axis != 2 || T.side[0].psi == nullptr || T.side[1].psi == nullptr) continue;
+      const int gap = std::max(T.side[1].lo[2] - T.side[0].hi[2], T.side[0].lo[2] - T.side[1].hi[2]);
+      L->planes = std::max(1, std::min(L->planes, gap + 1));
+    }
+  constexpr int kPerQuad = 4 / kVec<real>;
   long long total = 0;
   for (int n = 0; n < a.n_slab[kind]; ++n) {
     Span3 bx = a.slab[kind][n];
     bx.q1 = std::min(bx.q1, (a.nx + 1) / 4 + 1);  // quads past the last updated cell hold no work
-    const long long cols = (long long)(bx.q1 - bx.q0) * (bx.j1 - bx.j0);
+    const long long cols = (long long)(bx.q1 - bx.q0) * kPerQuad * (bx.j1 - bx.j0);
     if (cols <= 0 || bx.k1 <= bx.k0) continue;
     L->box[L->n] = bx;
     L->first[L->n] = (int)total;
-    L->cblk[L->n] = (int)((cols + kSlabThreads - 1) / kSlabThreads);
-    L->nch[L->n] = (bx.k1 - bx.k0 + kSlabPlanes - 1) / kSlabPlanes;
-    total += (long long)L->cblk[L->n] * L->nch[L->n] * a.B;
+    const long long cblk = (cols + kSlabCols - 1) / kSlabCols;
+    const int nch = (bx.k1 - bx.k0 + L->planes - 1) / L->planes;
+    const long long blocks_here = cblk * nch * a.B;
+    L->cblk[L->n] = fast_divisor(cblk, blocks_here);
+    L->nch[L->n] = fast_divisor(nch, (long long)nch * a.B);
+    L->nv[L->n] = fast_divisor((bx.q1 - bx.q0) * kPerQuad, cblk * kSlabCols);
+    total += blocks_here;
     ++L->n;
   }
-  if (L->n == 0) return cudaSuccess;
-  if (3 * total > 2147483647LL) return cudaErrorInvalidConfiguration;
+  if (total > 2147483647LL) return cudaErrorInvalidConfiguration;
   L->first[L->n] = (int)total;
-  *blocks = 3 * total;  // one block per component of every column block
+  *blocks = total;
   return cudaSuccess;
 }
 
 template <typename real>
-cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s) {
+int inject_blocks(const EdgeArgs<real>& ed) {
+  return (int)(((long long)ed.n * ed.B + kSlabThreads - 1) / kSlabThreads);
+}
+
+template <typename real>
+cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, const EdgeArgs<real>* ed,
+                        const ProbeArgs<real>* pr, int off) {
   SlabLaunch L;
   long long blocks = 0;
   if (const cudaError_t e = slab_plan(a, kind, &L, &blocks)) return e;
+  if (pr != nullptr) L.extra = kind == 0 ? pr->n_kind[1] * a.B : (off > 0 ? pr->n_kind[0] * a.B : 0);
+  if (ed != nullptr) L.inject = inject_blocks(*ed);
+  blocks += L.extra + L.inject;
   if (blocks == 0) return cudaSuccess;
+  const EdgeArgs<real> no_ed{};
+  const ProbeArgs<real> no_pr{};
+  const EdgeArgs<real>& e = ed ? *ed : no_ed;
+  const ProbeArgs<real>& p = pr ? *pr : no_pr;
   if (kind == 0 && a.ade_P > 1)
-    slab_e_kernel<real, true><<<(unsigned)blocks, kSlabThreads, 0, s>>>(a, L);
+    slab_e_kernel<real, true><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, e, p, off);
   else if (kind == 0)
-    slab_e_kernel<real, false><<<(unsigned)blocks, kSlabThreads, 0, s>>>(a, L);
+    slab_e_kernel<real, false><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, e, p, off);
   else
-    slab_h_kernel<real><<<(unsigned)blocks, kSlabThreads, 0, s>>>(a, L);
+    slab_h_kernel<real><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, p, off);
   return cudaGetLastError();
 }
 
 template <typename real>
-cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const BatchGrid& G, int blocks, int kind,
-                              bool multi_pole, cudaStream_t s) {
+cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
+                              const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
+                              int off, cudaStream_t s) {
   if (blocks <= 0) return cudaSuccess;
   if (kind == 0 && multi_pole)
-    slab_e_batch_kernel<real, true><<<blocks, kSlabThreads, 0, s>>>(A, L, G);
+    slab_e_batch_kernel<real, true><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, ED, PR, G, off);
   else if (kind == 0)
-    slab_e_batch_kernel<real, false><<<blocks, kSlabThreads, 0, s>>>(A, L, G);
+    slab_e_batch_kernel<real, false><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, ED, PR, G, off);
   else
-    slab_h_batch_kernel<real><<<blocks, kSlabThreads, 0, s>>>(A, L, G);
+    slab_h_batch_kernel<real><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, PR, G, off);
   return cudaGetLastError();
 }
 
@@ -504,15 +741,17 @@ cudaError_t preload_slab() {
   return cudaSuccess;
 }
 
-template cudaError_t preload_slab<float>();
-template cudaError_t preload_slab<double>();
-template cudaError_t slab_plan<float>(const SweepArgs<float>&, int, SlabLaunch*, long long*);
-template cudaError_t slab_plan<double>(const SweepArgs<double>&, int, SlabLaunch*, long long*);
-template cudaError_t launch_slab_batch<float>(const SweepArgs<float>*, const SlabLaunch*, const BatchGrid&, int, int,
-                                              bool, cudaStream_t);
-template cudaError_t launch_slab_batch<double>(const SweepArgs<double>*, const SlabLaunch*, const BatchGrid&, int, int,
-                                               bool, cudaStream_t);
-template cudaError_t launch_slab<float>(const SweepArgs<float>&, int, cudaStream_t);
-template cudaError_t launch_slab<double>(const SweepArgs<double>&, int, cudaStream_t);
+#define OAFDTD_SLAB(real)                                                                                             \
+  template int inject_blocks<real>(const EdgeArgs<real>&);                                                            \
+  template cudaError_t preload_slab<real>();                                                                          \
+  template cudaError_t slab_plan<real>(const SweepArgs<real>&, int, SlabLaunch*, long long*, int);                    \
+  template long long slab_vecs<real>(const SweepArgs<real>&, int);                                                    \
+  template cudaError_t launch_slab_batch<real>(const SweepArgs<real>*, const SlabLaunch*, const EdgeArgs<real>*,      \
+                                               const ProbeArgs<real>*, const BatchGrid&, int, int, bool, int,         \
+                                               cudaStream_t);                                                         \
+  template cudaError_t launch_slab<real>(const SweepArgs<real>&, int, cudaStream_t, const EdgeArgs<real>*,            \
+                                         const ProbeArgs<real>*, int);
+OAFDTD_SLAB(float)
+OAFDTD_SLAB(double)
 
 }  // namespace oafdtd

@@ -27,9 +27,9 @@ def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_serie
     ``estimate_bytes`` (``engine.py:29-40``), which the run driver checks against free device
     memory before it builds the engine, counted from this engine's own buffers.
 
-    * six field arrays ``(B, Z, Y, X)`` twice (the fused sweep, the default wherever the grid has
-      an interior free of CPML cells, reads one set and writes the other) and the three uint16
-      index arrays ``(Z, Y, X)``;
+    * six field arrays ``(B, Z, Y, X)`` twice (the fused sweep, the default of large float32 grids
+      and open to every grid with an interior free of CPML cells, reads one set and writes the
+      other) and the three uint16 index arrays ``(Z, Y, X)``;
     * dense Debye currents ``(P, B, nk, Y, X)`` per component over the z range ``nk`` of its
       dispersive edges;
     * one CPML psi array per correction: the slab width on its derivative axis, the full storage
@@ -388,7 +388,7 @@ class Gb300Engine:
 
     def set_tuning(self, tile_z: int = 0, variant: int = -1) -> None:
         """Planes marched per block (0 keeps) and the sweep variant (3 the fused H + E sweep of
-        the interior, 2 staged by TMA, 1 staged by cp.async, 0 register marching, -1 keeps)."""
+        the interior, 2 staged by TMA, 1 staged by cp.async, 0 the direct sweeps, -1 keeps)."""
         native.check(self._lib.oafdtd_set_tuning(self._h, int(tile_z), int(variant)), "set_tuning")
 
     def get_tuning(self) -> tuple[int, int]:
