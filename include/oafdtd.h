@@ -408,12 +408,13 @@ int oafdtd_mlp_adam(float* w, void* w16, const float* grad, float* m1, float* m2
  * row-major N x K (both K-contiguous), BF16 operands, FP32 accumulation, the epilogues of
  * oafdtd_mlp_gemm (ldc for C32, C16 and mask). Group g's operands start strideA, strideB, strideC
  * (C32, C16 and mask), strideCT (C16T) and strideBias elements after group g - 1's (ignored for
- * one group). Problems with M a multiple of 128, N and K multiples of 64, leading dimensions and
- * strides multiples of 8, 16-byte aligned pointers and beta 0 run on the fifth-generation tensor
- * cores (tcgen05.mma, accumulators in tensor memory, operand tiles and results moved by TMA tensor
+ * one group). Problems of any size whose leading dimensions and strides are multiples of 8 (with a
+ * mask, N too), with 16-byte aligned pointers and beta 0, run on the fifth-generation tensor cores
+ * (tcgen05.mma, accumulators in tensor memory, operand tiles and results moved by TMA tensor
  * copies; one persistent launch for all groups); the others on the mma.sync kernel, one launch.
  * C16T (BF16, nullable) receives the result transposed, N x M with leading dimension ldct (the next
- * layer's weight gradient reads it K-contiguous); off the tcgen05 shapes it needs C16 as well.
+ * layer's weight gradient reads it K-contiguous); off those layouts, ldct included, it needs C16 as
+ * well.
  * status (device int32, nullable): bit 0 is set when a bounded wait of the tcgen05 kernel gave up
  * (that launch's C is then incomplete). */
 int oafdtd_mlp_gemm_tn(const void* A, const void* B, float* C32, void* C16, void* C16T, const float* bias,

@@ -478,18 +478,22 @@ int oafdtd_mlp_gemm_tn(const void* A, const void* B, float* C32, void* C16, void
   const cudaStream_t s = static_cast<cudaStream_t>(stream);
   oafdtd::UmmaProblem p{A, B, C32, C16, C16T, bias, mask, M, N, K, lda, ldb, ldc, ldct, act, groups,
                         strideA, strideB, strideC, strideCT, strideBias, beta, status};
+  // a transposed result whose rows TMA cannot address (ldct not a multiple of 8) is made from C16
+  const bool own_t = C16T && C16 && !oafdtd::umma_shape_ok(p);
+  if (own_t) p.C16T = nullptr;
   if (oafdtd::umma_shape_ok(p)) {
     std::string why;
     const cudaError_t err = oafdtd::launch_umma_gemm(p, s, &why);
-    if (err != cudaSuccess) {
+    if (err == cudaSuccess)
+      return own_t ? oafdtd_mlp_transpose(C16, M, N, ldc, C16T, ldct, groups, strideC, strideCT, stream) : 0;
+    if (err != cudaErrorNotSupported) {
       oafdtd::set_last_error(std::string("oafdtd_mlp_gemm_tn: ") + (why.empty() ? cudaGetErrorString(err) : why));
-      return err == cudaErrorInvalidValue ? -1 : -3;
+      return -3;
     }
-    return 0;
   }
   // other shapes: the mma.sync kernels (B transposed), then the transposed copy of the BF16 result
   if (C16T && !C16) {
-    oafdtd::set_last_error("oafdtd_mlp_gemm_tn: a transposed result off the tcgen05 shapes needs C16 as well");
+    oafdtd::set_last_error("oafdtd_mlp_gemm_tn: a transposed result off the tcgen05 layouts needs C16 as well");
     return -1;
   }
   oafdtd::GemmArgs g;

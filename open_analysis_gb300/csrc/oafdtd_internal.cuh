@@ -277,6 +277,29 @@ struct BatchGrid {
 };
 
 #ifdef __CUDACC__
+// Programmatic dependent launch. A kernel launched by launch_pdl may start once every block of the
+// kernel before it in the stream has called pdl_launch() or ended; pdl_wait() then waits for that
+// kernel's completion, all its writes included. So a launch's set-up (indices, barriers, descriptors)
+// runs in the tail of the kernel before it. Every thread calls pdl_wait() before its first access to
+// memory that another kernel writes or reads.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // A batched kernel's arguments of this block's engine, copied once per block from device memory
 // into shared memory (buf: sizeof(T) bytes, 16-byte aligned), so that the kernel body reads them
 // as cheaply as launch parameters instead of holding them in registers.
@@ -406,8 +429,8 @@ struct UmmaProblem {
   float beta;
   int* status;         // set nonzero when a bounded wait gave up (nullable)
 };
-// Whether a problem suits the kernel: M a multiple of 128, N of 64, K of 64; leading dimensions
-// and group strides multiples of 8 elements; 16-byte aligned operands; beta 0.
+// Whether a problem suits the kernel: any M, N and K (with a mask, N a multiple of 8); leading
+// dimensions and group strides multiples of 8 elements; 16-byte aligned operands; beta 0.
 bool umma_shape_ok(const UmmaProblem& p);
 cudaError_t launch_umma_gemm(const UmmaProblem& p, cudaStream_t s, std::string* why);
 cudaError_t preload_umma();

@@ -24,6 +24,12 @@
 //     epilogue, stages the 32 x 32 chunk in shared memory in the TMA's swizzled layout and stores
 //     it with cp.async.bulk.tensor (FP32: 128-byte swizzle; BF16: 64-byte; transposed BF16:
 //     plain rows of 64 bytes), so the epilogue of one tile overlaps the MMAs of the next.
+// Ragged extents: TMA fills a box's part past the matrix with zeros on loads and leaves it out on
+// stores, so any M, N and K run here; the results are bit for bit the mma.sync kernel's (the same K
+// steps of 16). The training and prediction shapes are bound by latency, not by the tensor pipe (one
+// tile per CTA: launch, descriptors, two rounds of TMA, epilogue): the launches are programmatic
+// dependents, so a kernel sets up in the tail of the one before (8 x 256x512x512: 10.5 to 7.5 us;
+// 32 x 64x512x512, on mma.sync before: 8.5 us).
 // Every mbarrier wait is bounded (about two seconds, and a poll count); a wait that gives up sets
 // the caller's status word and a flag the other roles poll, every role leaves its loop, copies
 // and MMAs in flight are waited for (bounded again) and TMEM is freed, so no launch hangs.
@@ -184,7 +190,9 @@ __global__ void __launch_bounds__(kUThreads, 1)
   UStage<BN>* st = reinterpret_cast<UStage<BN>*>(base);
   EpiStage* ep = reinterpret_cast<EpiStage*>(base + kUStages * sizeof(UStage<BN>));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int MT = g.M / kUM, NT = g.N / BN, KT = g.K / kUK;
+  // the last tiles of each extent may reach past it: TMA fills loads there with zeros (a K step of
+  // zeros adds nothing) and leaves stores out
+  const int MT = (g.M + kUM - 1) / kUM, NT = (g.N + BN - 1) / BN, KT = (g.K + kUK - 1) / kUK;
   const int tiles = g.groups * MT * NT;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kUStages; ++s) {
@@ -212,6 +220,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   const uint32_t tmem = tmem_base;
+  pdl_launch();
+  pdl_wait();  // operands, bias and mask may come from the kernel before; it may read what C replaces
   int issued = 0;  // the producer's count of K steps whose copies it issued
   if (warp == 0) {
     if (lane == 0) {
@@ -290,7 +300,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
           if (lane == 0) ubar_arrive(&tempty[acc]);
         }
         const int col0 = nt * BN + c;  // the chunk's first column
-        const float bl = g.bias ? g.bias[gi * g.sBias + col0 + lane] : 0.f;
+        if (row0 >= g.M || col0 >= g.N) continue;  // nothing of the chunk lies in C
+        const float bl = g.bias && col0 + lane < g.N ? g.bias[gi * g.sBias + col0 + lane] : 0.f;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bl, j);
@@ -304,7 +315,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
           const uint4* mp = reinterpret_cast<const uint4*>(g.mask + gi * g.sC + (long long)row * g.ldc + col0);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            const uint4 w = mp[k];
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (row < g.M && col0 + 8 * k < g.N) w = mp[k];
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
@@ -395,16 +407,16 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
   CUtensorMap amap, bmap, c32map{}, c16map{}, c16tmap{};
   if (!group_map(&amap, BF, 2, p.A, p.M, p.K, p.lda, p.sA, p.groups, kUK, kUM, CU_TENSOR_MAP_SWIZZLE_128B, "A", why) ||
       !group_map(&bmap, BF, 2, p.B, p.N, p.K, p.ldb, p.sB, p.groups, kUK, BN, CU_TENSOR_MAP_SWIZZLE_128B, "B", why))
-    return cudaErrorInvalidValue;
+    return cudaErrorNotSupported;
   if (p.C32 && !group_map(&c32map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.C32, p.M, p.N, p.ldc, p.sC, p.groups, 32, 32,
                           CU_TENSOR_MAP_SWIZZLE_128B, "C32", why))
-    return cudaErrorInvalidValue;
+    return cudaErrorNotSupported;
   if (p.C16 && !group_map(&c16map, BF, 2, p.C16, p.M, p.N, p.ldc, p.sC, p.groups, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B,
                           "C16", why))
-    return cudaErrorInvalidValue;
+    return cudaErrorNotSupported;
   if (p.C16T && !group_map(&c16tmap, BF, 2, p.C16T, p.N, p.M, p.ldct, p.sCT, p.groups, 32, 32,
                            CU_TENSOR_MAP_SWIZZLE_NONE, "C16T", why))
-    return cudaErrorInvalidValue;
+    return cudaErrorNotSupported;
   UmmaArgs g{};
   g.bias = p.bias;
   g.mask = static_cast<const __nv_bfloat16*>(p.mask);
@@ -423,10 +435,9 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
       sms = 148;
   }
-  const long long tiles = (long long)p.groups * (p.M / kUM) * (p.N / BN);
+  const long long tiles = (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + BN - 1) / BN);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  umma_gemm_kernel<BN><<<grid, kUThreads, bytes, s>>>(g, amap, bmap, c32map, c16map, c16tmap);
-  return cudaGetLastError();
+  return launch_pdl(umma_gemm_kernel<BN>, dim3(grid), dim3(kUThreads), bytes, s, g, amap, bmap, c32map, c16map, c16tmap);
 }
 
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
@@ -434,8 +445,7 @@ bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 
 }  // namespace
 
 bool umma_shape_ok(const UmmaProblem& p) {
-  const bool tiles = p.M > 0 && p.N > 0 && p.K > 0 && p.M % kUM == 0 && p.N % 64 == 0 && p.K % kUK == 0 &&
-                     p.groups >= 1;
+  const bool sizes = p.M > 0 && p.N > 0 && p.K > 0 && p.groups >= 1 && (!p.mask || p.N % 8 == 0);
   const bool lds = p.lda % 8 == 0 && p.ldb % 8 == 0 && p.ldc % 8 == 0 && (!p.C16T || p.ldct % 8 == 0) &&
                    p.lda >= p.K && p.ldb >= p.K && p.ldc >= p.N && (!p.C16T || p.ldct >= p.M);
   const bool strides = p.groups == 1 || (p.sA % 8 == 0 && p.sB % 8 == 0 && p.sC % 8 == 0 && p.sCT % 8 == 0 &&
@@ -443,12 +453,13 @@ bool umma_shape_ok(const UmmaProblem& p) {
                                          p.sC >= (long long)p.M * p.ldc && (!p.C16T || p.sCT >= (long long)p.N * p.ldct));
   const bool ptrs = aligned16(p.A) && aligned16(p.B) && aligned16(p.C32) && aligned16(p.C16) && aligned16(p.C16T) &&
                     aligned16(p.mask);
-  return tiles && lds && strides && ptrs && p.beta == 0.f;
+  return sizes && lds && strides && ptrs && p.beta == 0.f;
 }
 
 cudaError_t launch_umma_gemm(const UmmaProblem& p, cudaStream_t s, std::string* why) {
   // 128-column tiles unless they would leave most SMs without a tile
-  const long long tiles128 = p.N % 128 == 0 ? (long long)p.groups * (p.M / kUM) * (p.N / 128) : 0;
+  const long long tiles128 =
+      p.N > 64 ? (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + 127) / 128) : 0;
   if (tiles128 >= 96) return launch_bn<128>(p, s, why);
   return launch_bn<64>(p, s, why);
 }

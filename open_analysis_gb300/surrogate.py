@@ -323,8 +323,8 @@ class Mlp:
     floats, the members' blocks side by side. Every GEMM is C = A . B^T with both operands
     K-contiguous (``oafdtd_mlp_gemm_tn``): the forward reads the transposed weights, the weight
     gradients the transposed activations and output gradients, which the epilogues and a small
-    transpose kernel write. Problems with M a multiple of 128 and N, K multiples of 64 (batch 256,
-    widths of 512) run on the tcgen05 tensor cores, all members in one persistent launch. Every
+    transpose kernel write. They run on the tcgen05 tensor cores, all members in one persistent
+    launch, where the layout allows (batches that are multiples of 8; predictions of any size). Every
     width is padded to a multiple of 8 (the input with zero columns, so the extra weights see zero
     inputs and zero gradients)."""
 
