@@ -398,6 +398,10 @@ int oafdtd_mlp_colsum(const float* X, int32_t M, int32_t N, int32_t ld, float* o
 int oafdtd_mlp_mse_grad(const float* Y, const float* T, int32_t M, int32_t N, float* G32, void* G16,
                         float* row_loss, int32_t groups, void* stream);
 
+/* The same, and the BF16 gradient transposed within each group into G16T (groups x N x M / groups). */
+int oafdtd_mlp_mse_grad_t(const float* Y, const float* T, int32_t M, int32_t N, float* G32, void* G16, void* G16T,
+                          float* row_loss, int32_t groups, void* stream);
+
 /* One Adam step on n FP32 weights w (moments m1, m2), refreshing the BF16 copy w16 (nullable).
  * The learning rate is read from *lr (device float) and the step number for the bias corrections
  * from *step (device int32, >= 1), so a captured step replays with both moving on. */
@@ -426,6 +430,22 @@ int oafdtd_mlp_gemm_tn(const void* A, const void* B, float* C32, void* C16, void
  * for g < groups, src_g and dst_g src_stride and dst_stride elements after group g - 1's. */
 int oafdtd_mlp_transpose(const void* src, int32_t rows, int32_t cols, int32_t lds, void* dst, int32_t ldd,
                          int32_t groups, int64_t src_stride, int64_t dst_stride, void* stream);
+
+/* One Adam step on a network of n_layers (at most 32) of every member, with its BF16 weights w16 and
+ * their transposes w16t, in one launch: member k's parameters start k * stride elements into each
+ * buffer; layers (host) holds per layer the weights' offset, fan_in, fan_out (row-major fan_in x
+ * fan_out; w16t the transpose at the same offset) and the biases' offset. Offsets, widths and stride
+ * multiples of 8, buffers 16-byte aligned. lr, step and the arithmetic as oafdtd_mlp_adam. */
+int oafdtd_mlp_adam_net(float* w, void* w16, void* w16t, const float* grad, float* m1, float* m2, int32_t n_layers,
+                        const int64_t* layers, int32_t members, int64_t stride, const float* lr, float b1, float b2,
+                        float eps, const int32_t* step, void* stream);
+
+/* One training batch of every group in one launch: rows idx[g * rows + r] of x (n_in columns) as
+ * BF16 into x16 (groups x rows x n_in) and transposed into x16t (groups x n_in x rows), and of t
+ * (n_out columns, a multiple of 4, 16-byte aligned) into t32 (groups x rows x n_out). *counter
+ * (device int32, nullable) += 1. */
+int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out, const int32_t* idx, int32_t rows,
+                     int32_t groups, void* x16, void* x16t, float* t32, int32_t* counter, void* stream);
 
 /* *counter += 1 on the device (the Adam step number inside a captured training step). */
 int oafdtd_mlp_count(int32_t* counter, void* stream);

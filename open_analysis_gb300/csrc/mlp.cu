@@ -372,6 +372,46 @@ __global__ void mse_grad_kernel(const float* Y, const float* T, int Mg, int N, f
   }
 }
 
+// The same with the BF16 gradient transposed too (per group, N x M_g), in one pass: a block takes
+// kMseRows rows of a group, a warp each, and walks the columns 128 at a time, the transposed part of
+// kMseRows rows (16 bytes per column) going out through shared memory. 9 us for 2048 x 752 (24 MB, in
+// L2; 6 steps in a row bound it); the two launches that this replaces took 17.
+constexpr int kMseRows = 8, kMseCols = 128;
+
+__global__ void __launch_bounds__(256) mse_grad_t_kernel(const float* Y, const float* T, int Mg, int N, float* G32,
+                                                         __nv_bfloat16* G16, __nv_bfloat16* G16T, float* row_loss) {
+  __shared__ __align__(16) __nv_bfloat16 tile[2][kMseCols][kMseRows];
+  const int tid = threadIdx.x, ty = tid / 32, lane = tid % 32;
+  const int r0 = blockIdx.x * kMseRows;  // Mg is a multiple of 8: every row is in
+  const long long row = (long long)blockIdx.y * Mg + r0 + ty;
+  const float scale = 2.f / ((float)Mg * (float)N);
+  float s = 0.f;
+  int half = 0;
+  for (int c0 = 0; c0 < N; c0 += kMseCols, half ^= 1) {  // two tiles in turn: one barrier per step
+    const int c = c0 + 4 * lane;
+    if (c < N) {
+      const long long o = row * N + c;
+      const float4 y = *reinterpret_cast<const float4*>(Y + o), t = *reinterpret_cast<const float4*>(T + o);
+      const float d[4] = {y.x - t.x, y.y - t.y, y.z - t.z, y.w - t.w};
+      s += d[0] * d[0] + d[1] * d[1] + d[2] * d[2] + d[3] * d[3];
+      const float4 g = make_float4(scale * d[0], scale * d[1], scale * d[2], scale * d[3]);
+      *reinterpret_cast<float4*>(G32 + o) = g;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(g.x, g.y), hi = __floats2bfloat162_rn(g.z, g.w);
+      *reinterpret_cast<uint2*>(G16 + o) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      __nv_bfloat16(*q)[kMseRows] = &tile[half][4 * lane];
+      q[0][ty] = lo.x, q[1][ty] = lo.y, q[2][ty] = hi.x, q[3][ty] = hi.y;
+    }
+    __syncthreads();
+    if (tid < kMseCols && c0 + tid < N)
+      *reinterpret_cast<uint4*>(G16T + ((long long)blockIdx.y * N + c0 + tid) * Mg + r0) =
+          *reinterpret_cast<const uint4*>(&tile[half][tid][0]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) row_loss[row] = s;
+}
+
 // Adam on FP32 master weights, with the BF16 copy the GEMMs read. The learning rate and the step
 // number (for the bias corrections) are read from device memory, so that a captured training step
 // replays unchanged while both move on.
@@ -392,6 +432,126 @@ __global__ void adam_kernel(float* w, __nv_bfloat16* w16, const float* grad, flo
 }
 
 __global__ void count_kernel(int* counter) { *counter += 1; }
+
+// Adam on a whole network of every member, with its BF16 weights and their transposes: one launch in
+// place of Adam, and a transpose per layer that read the BF16 weights back (8 members of 1.8 million
+// parameters: 118 + 7 x 5 us before, of which two powf per parameter took Adam from its 66 us of
+// memory traffic to 118). A block takes a 64 x 64 tile of one layer's weights (fan_in x fan_out): 16
+// loads of 16 bytes per thread in flight, the updated tile through shared memory for the transpose.
+// The blocks after a layer's tiles take its biases. blockIdx.y is the member. 80 us now, 7.0 TB/s. Run
+// layer by layer beside the backward GEMMs it cost the step 20 us more than behind them: both want the
+// same memory.
+constexpr int kAdamLayers = 32, kAdamTile = 64;
+struct AdamNet {
+  int n;
+  long long w[kAdamLayers], b[kAdamLayers];  // offsets of the weights and biases in a member's block
+  int rows[kAdamLayers], cols[kAdamLayers];
+  int first[kAdamLayers + 1];  // first block of each layer
+};
+
+struct AdamStep {
+  float lr, b1, b2, eps, c1, c2;
+};
+__device__ __forceinline__ float adam_update(const AdamStep& t, float w, float g, float& m1, float& m2) {
+  m1 = t.b1 * m1 + (1.f - t.b1) * g;
+  m2 = t.b2 * m2 + (1.f - t.b2) * g * g;
+  return w - t.lr * (m1 / t.c1) / (sqrtf(m2 / t.c2) + t.eps);
+}
+
+__global__ void __launch_bounds__(256) adam_net_kernel(const __grid_constant__ AdamNet net, float* w, __nv_bfloat16* w16,
+                                                       __nv_bfloat16* w16t, const float* grad, float* m1, float* m2,
+                                                       long long stride, const float* lr_dev, float b1, float b2,
+                                                       float eps, const int* step) {
+  __shared__ __align__(16) __nv_bfloat16 tile[kAdamTile][kAdamTile + 8];
+  __shared__ AdamStep sh;
+  const int tid = threadIdx.x;
+  int l = 0;
+  while (l + 1 < net.n && (int)blockIdx.x >= net.first[l + 1]) ++l;
+  const int rows = net.rows[l], cols = net.cols[l];
+  const int tc = (cols + kAdamTile - 1) / kAdamTile, tiles = tc * ((rows + kAdamTile - 1) / kAdamTile);
+  const int blk = (int)blockIdx.x - net.first[l];
+  const long long base = blockIdx.y * stride;
+  // the step's constants (two powers: some microseconds of one thread) come behind the loads
+  auto constants = [&] {
+    if (tid == 0) {
+      const float t = (float)*step;
+      sh = AdamStep{*lr_dev, b1, b2, eps, 1.f - powf(b1, t), 1.f - powf(b2, t)};
+    }
+    __syncthreads();
+    return sh;
+  };
+  if (blk >= tiles) {  // biases
+    const AdamStep st = constants();
+    const int i = (blk - tiles) * 256 + tid;
+    if (i >= cols) return;
+    const long long o = base + net.b[l] + i;
+    float a = m1[o], b = m2[o];
+    const float v = adam_update(st, w[o], grad[o], a, b);
+    m1[o] = a, m2[o] = b, w[o] = v;
+    w16[o] = __float2bfloat16(v);
+    return;
+  }
+  const int r0 = blk / tc * kAdamTile, c0 = blk % tc * kAdamTile;
+  const int tx = tid % 16, ty = tid / 16, c = c0 + 4 * tx;  // cols is a multiple of 8: a quad is in or out
+  const long long o0 = base + net.w[l] + c;
+  float4 g4[4], a4[4], b4[4], w4[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const int r = r0 + ty + 16 * p;
+    if (r >= rows || c >= cols) continue;
+    const long long o = o0 + (long long)r * cols;
+    g4[p] = *reinterpret_cast<const float4*>(grad + o);
+    a4[p] = *reinterpret_cast<const float4*>(m1 + o);
+    b4[p] = *reinterpret_cast<const float4*>(m2 + o);
+    w4[p] = *reinterpret_cast<const float4*>(w + o);
+  }
+  const AdamStep st = constants();
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const int r = r0 + ty + 16 * p;
+    if (r >= rows || c >= cols) continue;
+    const long long o = o0 + (long long)r * cols;
+    w4[p].x = adam_update(st, w4[p].x, g4[p].x, a4[p].x, b4[p].x);
+    w4[p].y = adam_update(st, w4[p].y, g4[p].y, a4[p].y, b4[p].y);
+    w4[p].z = adam_update(st, w4[p].z, g4[p].z, a4[p].z, b4[p].z);
+    w4[p].w = adam_update(st, w4[p].w, g4[p].w, a4[p].w, b4[p].w);
+    *reinterpret_cast<float4*>(m1 + o) = a4[p];
+    *reinterpret_cast<float4*>(m2 + o) = b4[p];
+    *reinterpret_cast<float4*>(w + o) = w4[p];
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(w4[p].x, w4[p].y), hi = __floats2bfloat162_rn(w4[p].z, w4[p].w);
+    *reinterpret_cast<uint2*>(w16 + o) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    const int row = ty + 16 * p;
+    tile[4 * tx][row] = lo.x, tile[4 * tx + 1][row] = lo.y, tile[4 * tx + 2][row] = hi.x, tile[4 * tx + 3][row] = hi.y;
+  }
+  __syncthreads();
+  // the transpose: column tid / 4 of the tile, 16 of its rows (rows is a multiple of 8)
+  const int col = tid / 4, seg = tid % 4 * 16;
+#pragma unroll
+  for (int h = 0; h < 16; h += 8)
+    if (c0 + col < cols && r0 + seg + h < rows)
+      *reinterpret_cast<uint4*>(w16t + base + net.w[l] + (long long)(c0 + col) * rows + r0 + seg + h) =
+          *reinterpret_cast<const uint4*>(&tile[col][seg + h]);
+}
+
+// One training batch in one launch, a block per (member, row): row idx[row] of the inputs as BF16, in
+// rows and transposed (per member), and of the targets as FP32. Moves the step number on by one.
+__global__ void __launch_bounds__(128) batch_kernel(const float* x, int n_in, const float* t, int n_out, const int* idx,
+                                                    int rows, __nv_bfloat16* x16, __nv_bfloat16* x16t, float* t32,
+                                                    int* counter) {
+  const long long r = blockIdx.x;
+  if (counter && r == 0 && threadIdx.x == 0) *counter += 1;
+  const int member = (int)(r / rows), k = (int)(r - (long long)member * rows);
+  const long long src = idx[r];
+  for (int c = threadIdx.x; c < n_in; c += blockDim.x) {
+    const __nv_bfloat16 v = __float2bfloat16(x[src * n_in + c]);
+    x16[r * n_in + c] = v;
+    x16t[((long long)member * n_in + c) * rows + k] = v;
+  }
+  const float4* s = reinterpret_cast<const float4*>(t + src * n_out);
+  float4* d = reinterpret_cast<float4*>(t32 + r * n_out);
+  for (int c = threadIdx.x; c < n_out / 4; c += blockDim.x) d[c] = s[c];
+}
 
 // Rows idx[0..rows) of an FP32 matrix with `cols` columns, into FP32 and/or BF16 copies.
 __global__ void gather_kernel(const float* src, int cols, const int* idx, int rows, float* d32,
@@ -550,11 +710,73 @@ int oafdtd_mlp_mse_grad(const float* Y, const float* T, int32_t M, int32_t N, fl
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+int oafdtd_mlp_mse_grad_t(const float* Y, const float* T, int32_t M, int32_t N, float* G32, void* G16, void* G16T,
+                          float* row_loss, int32_t groups, void* stream) {
+  if (!Y || !T || !G32 || !G16 || !G16T || !row_loss || M < 1 || N < 1 || groups < 1 || groups > 65535 ||
+      M % groups != 0)
+    return -1;
+  const int Mg = M / groups;
+  bool fast = Mg % 8 == 0 && N % 8 == 0;
+  for (const void* p : {static_cast<const void*>(Y), static_cast<const void*>(T), static_cast<const void*>(G32),
+                        static_cast<const void*>(G16), static_cast<const void*>(G16T)})
+    fast = fast && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+  if (!fast) {
+    if (const int rc = oafdtd_mlp_mse_grad(Y, T, M, N, G32, G16, row_loss, groups, stream)) return rc;
+    return oafdtd_mlp_transpose(G16, Mg, N, N, G16T, Mg, groups, (int64_t)Mg * N, (int64_t)Mg * N, stream);
+  }
+  oafdtd::mse_grad_t_kernel<<<dim3(Mg / oafdtd::kMseRows, groups), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      Y, T, Mg, N, G32, static_cast<__nv_bfloat16*>(G16), static_cast<__nv_bfloat16*>(G16T), row_loss);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 int oafdtd_mlp_adam(float* w, void* w16, const float* grad, float* m1, float* m2, int64_t n, const float* lr,
                     float b1, float b2, float eps, const int32_t* step, void* stream) {
   if (!w || !grad || !m1 || !m2 || !lr || !step || n < 1) return -1;
   oafdtd::adam_kernel<<<(unsigned)((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       w, static_cast<__nv_bfloat16*>(w16), grad, m1, m2, n, lr, b1, b2, eps, step);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+int oafdtd_mlp_adam_net(float* w, void* w16, void* w16t, const float* grad, float* m1, float* m2, int32_t n_layers,
+                        const int64_t* layers, int32_t members, int64_t stride, const float* lr, float b1, float b2,
+                        float eps, const int32_t* step, void* stream) {
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  bool ok = w && w16 && w16t && grad && m1 && m2 && layers && lr && step && n_layers >= 1 &&
+            n_layers <= oafdtd::kAdamLayers && members >= 1 && members <= 65535 && stride % 8 == 0 && aligned(w) &&
+            aligned(w16) && aligned(w16t) && aligned(grad) && aligned(m1) && aligned(m2);
+  oafdtd::AdamNet net{};
+  long long blocks = 0;
+  for (int l = 0; ok && l < n_layers; ++l) {
+    const int64_t* q = layers + 4 * l;  // weight offset, fan_in, fan_out, bias offset
+    ok = q[0] >= 0 && q[0] % 8 == 0 && q[1] >= 1 && q[1] % 8 == 0 && q[2] >= 1 && q[2] % 8 == 0 && q[3] >= 0 &&
+         q[0] + q[1] * q[2] <= stride && q[3] + q[2] <= stride && q[1] <= (1 << 20) && q[2] <= (1 << 20);
+    net.w[l] = q[0], net.rows[l] = (int)q[1], net.cols[l] = (int)q[2], net.b[l] = q[3];
+    net.first[l] = (int)blocks;
+    blocks += ((q[1] + 63) / 64) * ((q[2] + 63) / 64) + (q[2] + 255) / 256;
+    ok = ok && blocks <= 2147483647LL;
+  }
+  if (!ok) {
+    oafdtd::set_last_error("oafdtd_mlp_adam_net: bad arguments");
+    return -1;
+  }
+  net.n = n_layers;
+  net.first[n_layers] = (int)blocks;
+  oafdtd::adam_net_kernel<<<dim3((unsigned)blocks, members), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      net, w, static_cast<__nv_bfloat16*>(w16), static_cast<__nv_bfloat16*>(w16t), grad, m1, m2, stride, lr, b1, b2, eps,
+      step);
+  return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out, const int32_t* idx, int32_t rows,
+                     int32_t groups, void* x16, void* x16t, float* t32, int32_t* counter, void* stream) {
+  if (!x || !t || !idx || !x16 || !x16t || !t32 || n_in < 1 || n_out < 4 || n_out % 4 != 0 || rows < 1 || groups < 1 ||
+      (reinterpret_cast<uintptr_t>(t) & 15) || (reinterpret_cast<uintptr_t>(t32) & 15) ||
+      (long long)rows * groups > 2147483647LL) {
+    oafdtd::set_last_error("oafdtd_mlp_batch: bad arguments");
+    return -1;
+  }
+  oafdtd::batch_kernel<<<(unsigned)(rows * groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
+      x, n_in, t, n_out, idx, rows, static_cast<__nv_bfloat16*>(x16), static_cast<__nv_bfloat16*>(x16t), t32, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

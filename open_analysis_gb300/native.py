@@ -217,6 +217,12 @@ SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
         C.c_int,
         [C.c_void_p] * 5 + [_i64, C.c_void_p] + [C.c_float] * 3 + [C.c_void_p, C.c_void_p],
     ),
+    "oafdtd_mlp_adam_net": (
+        C.c_int,
+        [C.c_void_p] * 6 + [_i32, C.c_void_p, _i32, _i64, C.c_void_p] + [C.c_float] * 3 + [C.c_void_p] * 2,
+    ),
+    "oafdtd_mlp_batch": (C.c_int, [C.c_void_p, _i32, C.c_void_p, _i32, C.c_void_p, _i32, _i32] + [C.c_void_p] * 5),
+    "oafdtd_mlp_mse_grad_t": (C.c_int, [C.c_void_p, C.c_void_p, _i32, _i32] + [C.c_void_p] * 4 + [_i32, C.c_void_p]),
     "oafdtd_mlp_count": (C.c_int, [C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_gather": (C.c_int, [C.c_void_p, _i32, C.c_void_p, _i32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_gemm_tn": (

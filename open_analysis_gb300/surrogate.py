@@ -34,6 +34,7 @@ measure is taken relative to full scale.
 
 from __future__ import annotations
 
+import ctypes as C
 import math
 import time
 from collections.abc import Sequence
@@ -354,6 +355,7 @@ class Mlp:
             self.layout.append((wo, a, b, off))
             off = _align(off + b)
         self.n_params = off
+        self._layers = (C.c_int64 * (4 * len(self.layout)))(*[v for q in self.layout for v in q])
         flat = np.zeros((self.members, off), np.float32)
         n_layers = len(self.layout)
         gain = 2.0 if act == "relu" else 1.0  # He / Glorot-style variance per fan-in
@@ -381,6 +383,7 @@ class Mlp:
         self.lr = torch.full((1,), 1e-3, dtype=f32, device=self.dev)
         self.gen = torch.Generator(device=self.dev)
         self.gen.manual_seed(seed + 1)
+        self.side = torch.cuda.Stream(self.dev)  # bias gradients, beside the backward GEMMs
         self._train: dict[str, Any] | None = None
         self.graph: Any = None
 
@@ -498,32 +501,39 @@ class Mlp:
             "row_loss": z(m, dt=f32),
         }
 
-    def _backward(self, buf: dict[str, Any], m: int, s: int) -> None:
+    def _backward(self, buf: dict[str, Any], m: int, s: int, x_t: bool = False) -> None:
+        """Gradients of one batch: the GEMMs one after the other on the current stream, each layer's
+        bias gradient beside them on ``self.side``. ``x_t``: the transposed inputs are in ``buf``
+        already."""
         lib, g, p = self.lib, self.members, self.n_params
         y, t = buf["y"], buf["t"]
         out, n_in = self.sizes[-1], self.sizes[0]
-        native.check(lib.oafdtd_mlp_mse_grad(y.data_ptr(), t.data_ptr(), g * m, out, buf["g32"].data_ptr(),
-                                             buf["g16"].data_ptr(), buf["row_loss"].data_ptr(), g, s), "mse_grad")
+        cur, side = self.torch.cuda.current_stream(self.dev), self.side
+        s2 = int(side.cuda_stream)
         g32, g16, gT = buf["g32"].data_ptr(), buf["g16"].data_ptr(), buf["g16T"].data_ptr()
-        native.check(lib.oafdtd_mlp_transpose(g16, m, out, out, gT, m, g, m * out, out * m, s), "transpose")
-        native.check(lib.oafdtd_mlp_transpose(buf["x16"].data_ptr(), m, n_in, n_in, buf["x16T"].data_ptr(), m, g,
-                                              m * n_in, n_in * m, s), "transpose")
+        native.check(lib.oafdtd_mlp_mse_grad_t(y.data_ptr(), t.data_ptr(), g * m, out, g32, g16, gT,
+                                               buf["row_loss"].data_ptr(), g, s), "mse_grad")
+        if not x_t:
+            native.check(lib.oafdtd_mlp_transpose(buf["x16"].data_ptr(), m, n_in, n_in, buf["x16T"].data_ptr(), m, g,
+                                                  m * n_in, n_in * m, s), "transpose")
         for l in range(len(self.layout) - 1, -1, -1):
             _, a, b, _ = self.layout[l]
             inp = buf["x16"].data_ptr() if l == 0 else buf["acts"][l - 1].data_ptr()
             inp_t = buf["x16T"].data_ptr() if l == 0 else buf["actsT"][l - 1].data_ptr()
+            dz32 = dz16 = dzt = 0
+            if l:
+                # dZ[l-1] = (g . W^T) times the activation's derivative at the layer input  (m x a);
+                # W (a x b) is the B operand (N x K) as stored; the transposed dZ feeds layer l-1's dW
+                dz32, dz16 = buf["dz32"][l - 1].data_ptr(), buf["dz16"][l - 1].data_ptr()
+                dzt = buf["dz16T"][l - 1].data_ptr()
+                self._gemm_tn(g16, self._w(l), dz32, dz16, dzt, 0, inp, m, a, b, b, b, a, m, self.dact, s,
+                              m * b, p, m * a, a * m, 0)
             # dW = inp^T . g = (inp^T) . (g^T)^T  (a x b), from the transposed activations and g
             self._gemm_tn(inp_t, gT, self._gw(l), 0, 0, 0, 0, a, b, m, m, m, b, a, 0, s, a * m, b * m, p, 0, 0)
-            native.check(lib.oafdtd_mlp_colsum(g32, m, b, b, self._gb(l), g, m * b, p, s), "colsum")
-            if l == 0:
-                break
-            # dZ[l-1] = (g . W^T) times the activation's derivative at the layer input  (m x a);
-            # W (a x b) is the B operand (N x K) as stored; the transposed dZ feeds layer l-1's dW
-            dz32, dz16 = buf["dz32"][l - 1].data_ptr(), buf["dz16"][l - 1].data_ptr()
-            dzt = buf["dz16T"][l - 1].data_ptr()
-            self._gemm_tn(g16, self._w(l), dz32, dz16, dzt, 0, inp, m, a, b, b, b, a, m, self.dact, s,
-                          m * b, p, m * a, a * m, 0)
+            side.wait_stream(cur)
+            native.check(lib.oafdtd_mlp_colsum(g32, m, b, b, self._gb(l), g, m * b, p, s2), "colsum")
             g32, g16, gT = dz32, dz16, dzt
+        cur.wait_stream(side)
 
     def _per_member(self, v: npt.ArrayLike) -> npt.NDArray[np.float32]:
         """Host rows ``(m, c)`` for every member alike, or ``(members, m, c)`` per member."""
@@ -562,18 +572,21 @@ class Mlp:
                 [flat[bo : bo + b] for _, _, b, bo in self.layout])
 
     def _adam(self, s: int, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8) -> None:
-        lib = self.lib
-        native.check(lib.oafdtd_mlp_count(self.step_no.data_ptr(), s), "count")
-        native.check(lib.oafdtd_mlp_adam(self.p32.data_ptr(), self.p16.data_ptr(), self.grad.data_ptr(),
-                                         self.m1.data_ptr(), self.m2.data_ptr(), self.members * self.n_params,
-                                         self.lr.data_ptr(), b1, b2, eps, self.step_no.data_ptr(), s), "adam")
-        self._refresh_t(s)
+        """Adam on every layer of every member, with the BF16 weights and their transposes (one launch
+        per 32 layers)."""
+        for l in range(0, len(self.layout), 32):
+            native.check(self.lib.oafdtd_mlp_adam_net(
+                self.p32.data_ptr(), self.p16.data_ptr(), self.p16T.data_ptr(), self.grad.data_ptr(), self.m1.data_ptr(),
+                self.m2.data_ptr(), min(32, len(self.layout) - l), C.byref(self._layers, 32 * l), self.members,
+                self.n_params, self.lr.data_ptr(), b1, b2, eps, self.step_no.data_ptr(), s), "adam")
 
     def adam_step(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8) -> None:
         """One Adam step of every member on the current gradient buffer (the step number moves on
         by one)."""
         self.lr.fill_(lr)
-        self._adam(self._stream(), b1, b2, eps)
+        s = self._stream()
+        native.check(self.lib.oafdtd_mlp_count(self.step_no.data_ptr(), s), "count")
+        self._adam(s, b1, b2, eps)
 
     def check_status(self) -> None:
         """Raise when a bounded wait of a tcgen05 GEMM gave up since the last check (its result
@@ -588,12 +601,11 @@ class Mlp:
         lib, m, g = self.lib, self.batch, self.members
         idx = tr["perm"].data_ptr() + j * g * m * 4
         buf = tr["buf"]
-        native.check(lib.oafdtd_mlp_gather(tr["x"].data_ptr(), self.sizes[0], idx, g * m, None, buf["x16"].data_ptr(),
-                                           s), "gather")
-        native.check(lib.oafdtd_mlp_gather(tr["t"].data_ptr(), self.sizes[-1], idx, g * m, buf["t"].data_ptr(), None,
-                                           s), "gather")
+        native.check(lib.oafdtd_mlp_batch(tr["x"].data_ptr(), self.sizes[0], tr["t"].data_ptr(), self.sizes[-1], idx, m,
+                                          g, buf["x16"].data_ptr(), buf["x16T"].data_ptr(), buf["t"].data_ptr(),
+                                          self.step_no.data_ptr(), s), "batch")
         self._forward(buf["x16"].data_ptr(), buf["acts"], buf["y"].data_ptr(), m, s, buf["actsT"])
-        self._backward(buf, m, s)
+        self._backward(buf, m, s, x_t=True)
         self._adam(s)
 
     def prepare(self, x: npt.ArrayLike, t: npt.ArrayLike, graph: bool = True,
@@ -612,13 +624,13 @@ class Mlp:
         nb = min(len(r) for r in subsets) // self.batch
         if nb < 1:
             raise ValueError(f"{min(len(r) for r in subsets)} training rows are fewer than one batch of {self.batch}")
-        self.stream = torch.cuda.Stream(self.dev)
+        self.stream, self.draw = torch.cuda.Stream(self.dev), torch.cuda.Stream(self.dev)
         tr = {
             "n": n,
             "nb": nb,
             "x": torch.from_numpy(x).to(self.dev),
             "t": torch.from_numpy(t).to(self.dev),
-            "rows": [torch.from_numpy(r.astype(np.int64)).to(self.dev) for r in subsets],
+            "rows": [None if rows is None else torch.from_numpy(r.astype(np.int64)).to(self.dev) for r in subsets],
             # batch j of member k: perm[j, k, :]
             "perm": torch.zeros((nb, self.members, self.batch), dtype=torch.int32, device=self.dev),
             "buf": self._buffers(self.batch),
@@ -648,11 +660,18 @@ class Mlp:
         tr = self._train
         assert tr is not None
         nb, m = tr["nb"], self.batch
+        # the shuffles are drawn on a stream of their own, beside the epoch before
+        with torch.cuda.stream(self.draw):
+            picks = []
+            for r in tr["rows"]:
+                pick = torch.randperm(tr["n"] if r is None else r.numel(), generator=self.gen, device=self.dev)[: nb * m]
+                picks.append(pick if r is None else r[pick])
+            perm = torch.stack(picks).view(self.members, nb, m).transpose(0, 1)
         with torch.cuda.stream(self.stream):
             self.lr.fill_(lr)
-            for k, r in enumerate(tr["rows"]):
-                pick = r[torch.randperm(r.numel(), generator=self.gen, device=self.dev)[: nb * m]]
-                tr["perm"][:, k, :].copy_(pick.view(nb, m).to(torch.int32))
+            self.stream.wait_stream(self.draw)
+            tr["perm"].copy_(perm)
+            perm.record_stream(self.stream)
             if self.graph is not None:
                 self.graph.replay()
             else:

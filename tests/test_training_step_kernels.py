@@ -1,0 +1,85 @@
+"""The kernels that a training step takes in one pass each, against the separate ones they stand for."""
+
+import ctypes as C
+
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+def _lib():
+    from open_analysis_gb300 import native
+
+    return native, native.load()
+
+
+@pytest.mark.parametrize("sizes,members", [([8, 8], 1), ([24, 72, 8], 3), ([64, 128, 64], 2), ([8, 1032, 200], 1)])
+def test_adam_of_a_whole_net_matches_adam_and_a_transpose(sizes, members):
+    # tiles of 64 x 64: whole ones, ragged ones (72, 200), single 8-wide ones; > 256 biases (1032)
+    native, lib = _lib()
+    layers, off = [], 0
+    for a, b in zip(sizes, sizes[1:]):
+        layers.append((off, a, b, off + a * b))
+        off += a * b + b
+    gen = torch.Generator("cuda").manual_seed(1)
+    r = lambda: torch.randn(members * off, generator=gen, device="cuda")  # noqa: E731
+    w, grad, m1, m2 = r(), r(), r(), r().abs()
+    lr = torch.full((1,), 1e-3, device="cuda")
+    step = torch.full((1,), 3, dtype=torch.int32, device="cuda")
+    w16 = torch.zeros(members * off, dtype=torch.bfloat16, device="cuda")
+    ref = [t.clone() for t in (w, w16, m1, m2)]
+    w16t = torch.zeros_like(w16)
+    s = int(torch.cuda.current_stream().cuda_stream)
+    native.check(lib.oafdtd_mlp_adam(ref[0].data_ptr(), ref[1].data_ptr(), grad.data_ptr(), ref[2].data_ptr(),
+                                     ref[3].data_ptr(), members * off, lr.data_ptr(), 0.9, 0.999, 1e-8,
+                                     step.data_ptr(), s), "adam")
+    table = (C.c_int64 * (4 * len(layers)))(*[v for q in layers for v in q])
+    native.check(lib.oafdtd_mlp_adam_net(w.data_ptr(), w16.data_ptr(), w16t.data_ptr(), grad.data_ptr(),
+                                         m1.data_ptr(), m2.data_ptr(), len(layers), table, members, off,
+                                         lr.data_ptr(), 0.9, 0.999, 1e-8, step.data_ptr(), s), "adam_net")
+    for have, want in zip((w, w16, m1, m2), ref):
+        assert torch.equal(have, want)
+    for k in range(members):
+        for wo, a, b, _ in layers:
+            at = slice(k * off + wo, k * off + wo + a * b)
+            assert torch.equal(w16t[at].view(b, a), w16[at].view(a, b).T)
+
+
+@pytest.mark.parametrize("m,n,groups", [(8, 8, 1), (24, 136, 3), (256, 752, 2), (5, 9, 2)])
+def test_loss_gradient_and_its_transpose(m, n, groups):
+    # columns 128 at a time: less, a remainder, several; (5, 9) takes the separate kernels
+    native, lib = _lib()
+    gen = torch.Generator("cuda").manual_seed(2)
+    y, t = (torch.randn(groups * m, n, generator=gen, device="cuda") for _ in range(2))
+    g32, ref32 = torch.zeros_like(y), torch.zeros_like(y)
+    g16, ref16 = (torch.zeros_like(y, dtype=torch.bfloat16) for _ in range(2))
+    g16t = torch.zeros(groups, n, m, dtype=torch.bfloat16, device="cuda")
+    loss, ref_loss = (torch.zeros(groups * m, device="cuda") for _ in range(2))
+    s = int(torch.cuda.current_stream().cuda_stream)
+    native.check(lib.oafdtd_mlp_mse_grad(y.data_ptr(), t.data_ptr(), groups * m, n, ref32.data_ptr(),
+                                         ref16.data_ptr(), ref_loss.data_ptr(), groups, s), "mse_grad")
+    native.check(lib.oafdtd_mlp_mse_grad_t(y.data_ptr(), t.data_ptr(), groups * m, n, g32.data_ptr(), g16.data_ptr(),
+                                           g16t.data_ptr(), loss.data_ptr(), groups, s), "mse_grad_t")
+    assert torch.equal(g32, ref32) and torch.equal(g16, ref16)
+    assert torch.equal(g16t, ref16.view(groups, m, n).transpose(1, 2))
+    # a sum of n squares in another order: (n + 1) roundings each, of 2^-24
+    assert torch.all((loss - ref_loss).abs() <= 2 * (n + 1) * 2.0**-24 * ref_loss)
+
+
+@pytest.mark.parametrize("n_in,n_out,rows,groups", [(8, 8, 1, 1), (24, 200, 40, 3), (264, 752, 256, 2)])
+def test_a_batch_is_its_gathered_rows(n_in, n_out, rows, groups):
+    native, lib = _lib()
+    gen = torch.Generator("cuda").manual_seed(3)
+    x, t = (torch.randn(97, c, generator=gen, device="cuda") for c in (n_in, n_out))
+    idx = torch.randint(97, (groups, rows), generator=gen, device="cuda", dtype=torch.int32)
+    x16 = torch.zeros(groups, rows, n_in, dtype=torch.bfloat16, device="cuda")
+    x16t = torch.zeros(groups, n_in, rows, dtype=torch.bfloat16, device="cuda")
+    t32 = torch.zeros(groups, rows, n_out, device="cuda")
+    step = torch.full((1,), 6, dtype=torch.int32, device="cuda")
+    s = int(torch.cuda.current_stream().cuda_stream)
+    native.check(lib.oafdtd_mlp_batch(x.data_ptr(), n_in, t.data_ptr(), n_out, idx.data_ptr(), rows, groups,
+                                      x16.data_ptr(), x16t.data_ptr(), t32.data_ptr(), step.data_ptr(), s), "batch")
+    assert torch.equal(x16, x[idx.long()].bfloat16()) and torch.equal(x16t, x16.transpose(1, 2))
+    assert torch.equal(t32, t[idx.long()]) and step.item() == 7
