@@ -432,73 +432,103 @@ __device__ __forceinline__ float2 ff_add(float2 a, float2 b) {
   return make_float2(h, lo - (h - s));
 }
 
+// The sum of v^2 w over four cells, as a float-float pair. Products are exact to 2^-46, their rounded
+// parts are summed with the errors gathered apart (four of them: the gathered part needs no carry).
+__device__ __forceinline__ float2 ff_quad(const float v[4], const float2 w[4]) {
+  float hi = 0.0f, lo = 0.0f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const float p = v[e] * v[e];
+    const float h = w[e].x * p;
+    lo = __fmaf_rn(w[e].y, p, __fmaf_rn(w[e].x, __fmaf_rn(v[e], v[e], -p), lo)) + __fmaf_rn(w[e].x, p, -h);
+    const float s = hi + h, bb = s - hi;
+    lo += (hi - (s - bb)) + (h - bb);
+    hi = s;
+  }
+  const float s = hi + lo;
+  return make_float2(s, lo - (s - hi));
+}
+
 // Energy sums 1/2 sum eps E^2 V (and sum H^2 V) per component, in float64 or, for float32
 // fields, in float-float: GB300's float64 rate is a small fraction of its float32 rate, and a
-// float64 product chain per cell made this kernel compute-bound (3.3 ms at 400x400x120, batch
+// float64 product chain per cell makes this kernel compute-bound (3.3 ms at 400x400x120, batch
 // 2; the fields are read in 0.15 ms). A float32 field value squares exactly into a float-float
 // pair; the weights come as float-float pairs; the terms of a thread are summed in float-float
 // and the thread's sum converted to float64 once. Each term is then exact to about 1e-13 relative,
 // so the sum is too (every term is positive). The fields are scaled by 2^32 and the weights by
 // 2^40 (exact) so that squares of fields down to 1e-28 and weights down to 1e-30 stay normal;
 // the thread's sum is scaled back by 2^-104. Fields above 4e9 would overflow the square.
+// Field and weights of 38 million cells (1.1 GB, 0.16 ms) take 0.45 ms, 0.61 before: bound by the
+// instructions of the pairs (about 130 per quad).
+// A thread takes a quad (four cells of a row) per turn. The y-z weight, and the permittivity where
+// the four cells have one, multiply the quad's sum instead of each cell: a third of the float-float
+// operations. The quads of a thread lie a grid apart, and row and column move on by adding.
 template <typename real>
-__global__ void __launch_bounds__(256) energy_kernel(const __grid_constant__ EnergyArgs<real> a,
-                                                     double* partial) {
+__global__ void __launch_bounds__(256, 4) energy_kernel(const __grid_constant__ EnergyArgs<real> a,
+                                                        double* partial) {
   __shared__ double warp_sum[8];
   const int cc = blockIdx.y;  // 0..2 E, 3..5 H
   const real* F = a.F[cc];
-  const double* wx = a.w[cc][0];
-  const double* wy = a.w[cc][1];
-  const double* wz = a.w[cc][2];
-  const long long rows = (long long)a.B * a.Z * a.Y;
-  const long long bs = (long long)a.Z * a.Y * a.X;
+  const ushort4* M = cc < 3 ? reinterpret_cast<const ushort4*>(a.mat[cc]) : nullptr;
+  const int Q = a.X / 4;
+  const long long rows = (long long)a.Z * a.Y, per = rows * Q, quads = per * a.B;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long dr = stride / Q;
+  const int dq = (int)(stride - dr * Q);
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  long long r = t / Q;  // row of the member
+  int i = (int)(t - r * Q);
+  long long base = 0;  // first quad of the member
   double acc = 0.0;
+  auto settle = [&] {  // r into its member
+    while (r >= rows) r -= rows, base += per;
+  };
+  auto advance = [&] {
+    t += stride, r += dr, i += dq;
+    if (i >= Q) i -= Q, ++r;
+    settle();
+  };
+  settle();
   if constexpr (sizeof(real) == 4) {
-    // one quad (four cells, 16-byte loads) per thread and iteration, quads of consecutive rows
-    // on consecutive threads: enough loads in flight to stream the fields
     const float vscale = ldexpf(1.0f, kEnergyVShift);
-    const float2* wxf = a.wxf[cc];
+    const float4* wx4 = reinterpret_cast<const float4*>(a.wxf[cc]);
     const float2* wyzf = a.wyzf[cc];
-    const int Q = a.X / 4;
-    const long long quads = rows * Q;
     float2 sum = make_float2(0.0f, 0.0f);
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < quads;
-         t += (long long)gridDim.x * blockDim.x) {
-      const long long r = t / Q;
-      const int i0 = 4 * (int)(t - r * Q);
-      const long long plane = r % ((long long)a.Z * a.Y);
-      const long long q = r * a.X + i0;
-      const float4 f4 = *reinterpret_cast<const float4*>(F + q);
-      const float2 wyz = wyzf[plane];
-      ushort4 m4 = make_ushort4(0, 0, 0, 0);
-      if (cc < 3) m4 = *reinterpret_cast<const ushort4*>(a.mat[cc] + (q % bs));
-      const float fv[4] = {f4.x, f4.y, f4.z, f4.w};
-      const unsigned short mv[4] = {m4.x, m4.y, m4.z, m4.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float v = fv[e] * vscale;
-        const float p = v * v;
-        const float2 v2 = make_float2(p, __fmaf_rn(v, v, -p));
-        float2 w = ff_mul(wxf[i0 + e], wyz);
-        if (cc < 3) w = ff_mul(w, a.epsf[mv[e]]);
-        sum = ff_add(sum, ff_mul(w, v2));
+    for (; t < quads; advance()) {
+      const float4 f = reinterpret_cast<const float4*>(F)[t], w01 = wx4[2 * i], w23 = wx4[2 * i + 1];
+      const float2 wyz = wyzf[r];
+      const float v[4] = {f.x * vscale, f.y * vscale, f.z * vscale, f.w * vscale};
+      float2 w[4] = {{w01.x, w01.y}, {w01.z, w01.w}, {w23.x, w23.y}, {w23.z, w23.w}};
+      float2 q;
+      if (M) {
+        const ushort4 m = M[t - base];
+        if (m.x == m.y && m.x == m.z && m.x == m.w) {
+          q = ff_mul(ff_quad(v, w), a.epsf[m.x]);
+        } else {
+          w[0] = ff_mul(w[0], a.epsf[m.x]), w[1] = ff_mul(w[1], a.epsf[m.y]);
+          w[2] = ff_mul(w[2], a.epsf[m.z]), w[3] = ff_mul(w[3], a.epsf[m.w]);
+          q = ff_quad(v, w);
+        }
+      } else {
+        q = ff_quad(v, w);
       }
+      sum = ff_add(sum, ff_mul(q, wyz));
     }
     acc = ldexp((double)sum.x + (double)sum.y, -(kEnergyVShift * 2 + kEnergyWShift));
   } else {
-    for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-      const long long plane = r % ((long long)a.Z * a.Y);
-      const int k = (int)(plane / a.Y), j = (int)(plane % a.Y);
-      const double wyz = wy[j] * wz[k];
-      const long long row = r * a.X;
-      double racc = 0.0;
-      for (int i = threadIdx.x; i < a.X; i += blockDim.x) {
-        const double v = (double)F[row + i];
-        double term = wx[i] * wyz * v * v;
-        if (cc < 3) term *= a.eps[a.mat[cc][(row % bs) + i]];
-        racc += term;
+    const double* wx = a.w[cc][0];
+    const double* wy = a.w[cc][1];
+    const double* wz = a.w[cc][2];
+    for (; t < quads; advance()) {
+      const double2 f = reinterpret_cast<const double2*>(F)[2 * t], g = reinterpret_cast<const double2*>(F)[2 * t + 1];
+      const int k = (int)(r / a.Y), j = (int)(r - (long long)k * a.Y);
+      double w[4] = {wx[4 * i], wx[4 * i + 1], wx[4 * i + 2], wx[4 * i + 3]};
+      if (M) {
+        const ushort4 m = M[t - base];
+        w[0] *= a.eps[m.x], w[1] *= a.eps[m.y], w[2] *= a.eps[m.z], w[3] *= a.eps[m.w];
       }
-      acc += racc;
+      const double q = w[0] * (f.x * f.x) + w[1] * (f.y * f.y) + (w[2] * (g.x * g.x) + w[3] * (g.y * g.y));
+      acc += wy[j] * wz[k] * q;
     }
   }
 #pragma unroll
@@ -512,12 +542,16 @@ __global__ void __launch_bounds__(256) energy_kernel(const __grid_constant__ Ene
   }
 }
 
-__global__ void energy_final_kernel(const double* partial, int nblocks, double* out) {
-  const int cc = threadIdx.x;
-  if (cc >= 6) return;
+// A warp per component, in a fixed order (one thread per component took 130 us over 1216 partials,
+// each addition behind its load).
+__global__ void __launch_bounds__(192) energy_final_kernel(const double* partial, int nblocks, double* out) {
+  const int cc = threadIdx.x / 32, lane = threadIdx.x % 32;
   double s = 0.0;
-  for (int k = 0; k < nblocks; ++k) s += partial[(long long)cc * nblocks + k];
-  out[cc] = s;
+#pragma unroll 4
+  for (int k = lane; k < nblocks; k += 32) s += partial[(long long)cc * nblocks + k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if (lane == 0) out[cc] = s;
 }
 
 // ----------------------------------------------------------------------------- launchers
@@ -600,10 +634,13 @@ cudaError_t launch_edges(const EdgeArgs<real>& a, int off, cudaStream_t s) {
 template <typename real>
 cudaError_t launch_energy(const EnergyArgs<real>& a, double* partial, int nblocks, double* out,
                           cudaStream_t s) {
+  // at least four quads to a thread, where there are that many: a partial sum costs about as much
+  const long long quads = (long long)a.B * a.Z * a.Y * (a.X / 4);
+  nblocks = (int)std::min<long long>(nblocks, (quads + 4 * 256 - 1) / (4 * 256));
   energy_kernel<real><<<dim3(nblocks, 6), 256, 0, s>>>(a, partial);
   cudaError_t err = cudaGetLastError();
   if (err != cudaSuccess) return err;
-  energy_final_kernel<<<1, 32, 0, s>>>(partial, nblocks, out);
+  energy_final_kernel<<<1, 192, 0, s>>>(partial, nblocks, out);
   return cudaGetLastError();
 }
 
