@@ -64,6 +64,7 @@ __device__ __forceinline__ void ghost_wall(const GhostArgs<real>& g, int wall, i
 
 template <typename real>
 __global__ void __launch_bounds__(256) ghost_kernel(const __grid_constant__ GhostArgs<real> g) {
+  pdl_wait();
   const int wall = blockIdx.y, axis = wall >> 1;
   if (!((g.mask >> wall) & 1)) return;
   const int nu = g.ext[axis == 0 ? 1 : 0], nv = g.ext[axis == 2 ? 1 : 2];
@@ -159,6 +160,7 @@ __device__ __forceinline__ void dft_body(const ProbeArgs<real>& a, int block, in
 template <typename real>
 __global__ void __launch_bounds__(kDftF* kChunk) dft_kernel(const __grid_constant__ ProbeArgs<real> a, int n, int kinds,
                                                             int tail, int bump) {
+  pdl_wait();
   dft_body(a, (int)blockIdx.x, n, kinds, tail != 0, bump);
 }
 
@@ -169,7 +171,9 @@ __global__ void __launch_bounds__(kDftF* kChunk)
   __shared__ __align__(16) unsigned char args[sizeof(ProbeArgs<real>)];
   int e;
   const uint3 bid = G.block(&e);
-  dft_body(stage_args(A + e, args), (int)bid.x, n, 3, tail != 0, n);
+  const ProbeArgs<real>& a = stage_args(A + e, args);
+  pdl_wait();
+  dft_body(a, (int)bid.x, n, 3, tail != 0, n);
 }
 
 template <typename real>
@@ -261,6 +265,7 @@ __device__ __forceinline__ void sibc_body(const SibcArgs<real>& a, int block, in
 
 template <typename real, int BB, int PP>
 __global__ void __launch_bounds__(128) sibc_kernel(const __grid_constant__ SibcArgs<real> a, int lo, int hi) {
+  pdl_wait();
   sibc_body<real, BB, PP>(a, (int)blockIdx.x, lo, hi);
 }
 
@@ -294,6 +299,7 @@ __device__ __forceinline__ void sibc_generic_body(const SibcArgs<real>& a, int b
 
 template <typename real>
 __global__ void __launch_bounds__(128) sibc_generic_kernel(const __grid_constant__ SibcArgs<real> a, int lo, int hi) {
+  pdl_wait();
   sibc_generic_body(a, (int)blockIdx.x, lo, hi);
 }
 
@@ -304,6 +310,7 @@ __global__ void __launch_bounds__(128) sibc_batch_kernel(const SibcArgs<real>* _
   int e;
   const uint3 bid = G.block(&e);
   const SibcArgs<real>& a = stage_args(A + e, args);
+  pdl_wait();
   if constexpr (BB == 0)
     sibc_generic_body(a, (int)bid.x, 0, a.n);
   else
@@ -321,33 +328,26 @@ int sibc_blocks(const SibcArgs<real>& a) {
 }
 
 template <typename real>
-cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int blocks, int variant, cudaStream_t s) {
+cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int blocks, int variant, bool pdl,
+                              cudaStream_t s) {
   if (blocks <= 0) return cudaSuccess;
-  if (variant == 2)
-    sibc_batch_kernel<real, 2, 16><<<blocks, 128, 0, s>>>(A, G);
-  else if (variant == 1)
-    sibc_batch_kernel<real, 1, 16><<<blocks, 128, 0, s>>>(A, G);
-  else if (variant == 4)
-    sibc_batch_kernel<real, 4, 16><<<blocks, 128, 0, s>>>(A, G);
-  else
-    sibc_batch_kernel<real, 0, 16><<<blocks, 128, 0, s>>>(A, G);
-  return cudaGetLastError();
+  auto kernel = variant == 2   ? sibc_batch_kernel<real, 2, 16>
+                : variant == 1 ? sibc_batch_kernel<real, 1, 16>
+                : variant == 4 ? sibc_batch_kernel<real, 4, 16>
+                               : sibc_batch_kernel<real, 0, 16>;
+  return launch_pdl(pdl, kernel, dim3(blocks), dim3(128), 0, s, A, G);
 }
 
 template <typename real>
-cudaError_t launch_sibc(const SibcArgs<real>& a, cudaStream_t s, int lo, int hi) {
+cudaError_t launch_sibc(const SibcArgs<real>& a, cudaStream_t s, int lo, int hi, bool pdl) {
   if (hi < 0) hi = a.n;
   if (hi <= lo) return cudaSuccess;
-  const unsigned blocks = (unsigned)((hi - lo + 127) / 128);
-  if (a.B == 2 && a.P == 16)
-    sibc_kernel<real, 2, 16><<<blocks, 128, 0, s>>>(a, lo, hi);
-  else if (a.B == 1 && a.P == 16)
-    sibc_kernel<real, 1, 16><<<blocks, 128, 0, s>>>(a, lo, hi);
-  else if (a.B == 4 && a.P == 16)
-    sibc_kernel<real, 4, 16><<<blocks, 128, 0, s>>>(a, lo, hi);
-  else
-    sibc_generic_kernel<real><<<blocks, 128, 0, s>>>(a, lo, hi);
-  return cudaGetLastError();
+  const int variant = sibc_variant(a);
+  auto kernel = variant == 2   ? sibc_kernel<real, 2, 16>
+                : variant == 1 ? sibc_kernel<real, 1, 16>
+                : variant == 4 ? sibc_kernel<real, 4, 16>
+                               : sibc_generic_kernel<real>;
+  return launch_pdl(pdl, kernel, dim3((unsigned)((hi - lo + 127) / 128)), dim3(128), 0, s, a, lo, hi);
 }
 
 // ----------------------------------------------------------------------------- injection pass
@@ -559,7 +559,7 @@ static inline unsigned ceil_div(long long a, long long b) { return (unsigned)((a
 
 template <typename real>
 cudaError_t launch_ghosts(real* const H[3], int pmc_mask, int nx, int ny, int nz, int X, int Y, int B,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool pdl) {
   GhostArgs<real> g{{H[0], H[1], H[2]}, pmc_mask, {nx, ny, nz}, {X, Y, nz + 2}, B};
   long long most = 0;
   for (int w = 0; w < 6; ++w)
@@ -568,8 +568,7 @@ cudaError_t launch_ghosts(real* const H[3], int pmc_mask, int nx, int ny, int nz
       most = std::max(most, (long long)g.ext[axis == 0 ? 1 : 0] * g.ext[axis == 2 ? 1 : 2] * B);
     }
   if (most == 0) return cudaSuccess;
-  ghost_kernel<real><<<dim3(std::min(ceil_div(most, 256), 152u * 8u), 6), 256, 0, s>>>(g);
-  return cudaGetLastError();
+  return launch_pdl(pdl, ghost_kernel<real>, dim3(std::min(ceil_div(most, 256), 152u * 8u), 6), dim3(256), 0, s, g);
 }
 
 template <typename real>
@@ -651,25 +650,25 @@ int dft_blocks(const ProbeArgs<real>& a) {
 
 template <typename real>
 cudaError_t launch_dft(const ProbeArgs<real>& a, int n, int kinds, bool tail, int bump, cudaStream_t s) {
-  dft_kernel<real><<<dft_blocks_of(a), kDftF * kChunk, 0, s>>>(a, n, kinds, tail ? 1 : 0, bump);
-  return cudaGetLastError();
+  // tail: the direct sweeps' launches, all of which take part
+  return launch_pdl(tail, dft_kernel<real>, dim3(dft_blocks_of(a)), dim3(kDftF * kChunk), 0, s, a, n, kinds,
+                    tail ? 1 : 0, bump);
 }
 
 template <typename real>
 cudaError_t launch_dft_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int n, bool tail,
                              cudaStream_t s) {
   if (blocks <= 0) return cudaSuccess;
-  dft_batch_kernel<real><<<blocks, kDftF * kChunk, 0, s>>>(A, G, n, tail ? 1 : 0);
-  return cudaGetLastError();
+  return launch_pdl(tail, dft_batch_kernel<real>, dim3(blocks), dim3(kDftF * kChunk), 0, s, A, G, n, tail ? 1 : 0);
 }
 
 #define OAFDTD_INSTANTIATE(real)                                                                   \
   template cudaError_t launch_ghosts<real>(real* const[3], int, int, int, int, int, int, int,      \
-                                           cudaStream_t);                                           \
+                                           cudaStream_t, bool);                                     \
   template cudaError_t launch_pre_e<real>(const ProbeArgs<real>&, int, cudaStream_t);              \
   template cudaError_t launch_probe_e<real>(const ProbeArgs<real>&, int, cudaStream_t);            \
   template cudaError_t launch_edges<real>(const EdgeArgs<real>&, int, cudaStream_t);               \
-  template cudaError_t launch_sibc<real>(const SibcArgs<real>&, cudaStream_t, int, int);            \
+  template cudaError_t launch_sibc<real>(const SibcArgs<real>&, cudaStream_t, int, int, bool);      \
   template int dft_blocks<real>(const ProbeArgs<real>&);                                            \
   template cudaError_t launch_dft<real>(const ProbeArgs<real>&, int, int, bool, int, cudaStream_t); \
   template cudaError_t launch_dft_batch<real>(const ProbeArgs<real>*, const BatchGrid&, int, int, bool, \
@@ -685,7 +684,7 @@ cudaError_t launch_dft_batch(const ProbeArgs<real>* A, const BatchGrid& G, int b
                                                   cudaStream_t);                                    \
   template cudaError_t launch_edges_batch<real>(const EdgeArgs<real>*, const BatchGrid&, int, int,  \
                                                 cudaStream_t);                                      \
-  template cudaError_t launch_sibc_batch<real>(const SibcArgs<real>*, const BatchGrid&, int, int,   \
+  template cudaError_t launch_sibc_batch<real>(const SibcArgs<real>*, const BatchGrid&, int, int, bool,   \
                                                cudaStream_t);                                       \
   template cudaError_t preload_kernels<real>();                                                     \
   template cudaError_t launch_energy<real>(const EnergyArgs<real>&, double*, int, double*,         \

@@ -285,8 +285,10 @@ struct BatchGrid {
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// pdl false: an ordinary launch, which starts when the kernel before it has completed.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+inline cudaError_t launch_pdl(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              A&&... args) {
   cudaLaunchConfig_t c{};
   c.gridDim = grid;
   c.blockDim = block;
@@ -296,7 +298,7 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
-  c.numAttrs = 1;
+  c.numAttrs = pdl ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
@@ -350,7 +352,7 @@ cudaError_t launch_staged_batch(const SweepArgs<real>* A, const SweepMaps* M, co
 template <typename real>
 cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
                               const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
-                              int off, cudaStream_t s);
+                              int off, bool pdl, cudaStream_t s);
 template <typename real>
 cudaError_t launch_pre_e_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int off, cudaStream_t s);
 template <typename real>
@@ -358,7 +360,8 @@ cudaError_t launch_probe_e_batch(const ProbeArgs<real>* A, const BatchGrid& G, i
 template <typename real>
 cudaError_t launch_edges_batch(const EdgeArgs<real>* A, const BatchGrid& G, int blocks, int off, cudaStream_t s);
 template <typename real>
-cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int blocks, int variant, cudaStream_t s);
+cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int blocks, int variant, bool pdl,
+                              cudaStream_t s);
 // The running DFTs of the n steps from the step counter on, for the probe kinds in `kinds` (bit 0
 // E, bit 1 H), which then advances by `bump`. tail: the E samples of the last step are taken here.
 template <typename real>
@@ -383,17 +386,17 @@ int inject_blocks(const EdgeArgs<real>& ed);
 // probes of step off - 1).
 template <typename real>
 cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, const EdgeArgs<real>* ed = nullptr,
-                        const ProbeArgs<real>* pr = nullptr, int off = 0);
+                        const ProbeArgs<real>* pr = nullptr, int off = 0, bool pdl = false);
 template <typename real>
 cudaError_t launch_ghosts(real* const H[3], int pmc_mask, int nx, int ny, int nz, int X, int Y, int B,
-                          cudaStream_t s);
+                          cudaStream_t s, bool pdl = false);
 template <typename real>
 cudaError_t launch_pre_e(const ProbeArgs<real>& a, int off, cudaStream_t s);
 template <typename real>
 cudaError_t launch_edges(const EdgeArgs<real>& a, int off, cudaStream_t s);
 // the surface-impedance edges [lo, hi) (hi < 0: to the last)
 template <typename real>
-cudaError_t launch_sibc(const SibcArgs<real>& a, cudaStream_t s, int lo = 0, int hi = -1);
+cudaError_t launch_sibc(const SibcArgs<real>& a, cudaStream_t s, int lo = 0, int hi = -1, bool pdl = false);
 template <typename real>
 cudaError_t launch_probe_e(const ProbeArgs<real>& a, int off, cudaStream_t s);
 template <typename real>

@@ -459,16 +459,19 @@ template <typename real, bool kMulti>
 __device__ __forceinline__ void slab_e_body(const SweepArgs<real>& a, const SlabLaunch& L, const EdgeArgs<real>& ed,
                                             const ProbeArgs<real>& pr, int off, int block) {
   if (block < L.extra) {
+    pdl_wait();
     probe_sample(pr, 1, block, off);
     return;
   }
   block -= L.extra;
   if (block < L.inject) {
+    pdl_wait();
     const int t = block * kSlabThreads + (int)(threadIdx.x + kSlabCols * threadIdx.y);
     if (t < ed.n * a.B) list_edge<real>(a, ed, off, t);
     return;
   }
   const SlabWork w = slab_work<real>(L, a.nx, block - L.inject);
+  pdl_wait();
   if (!w.live) return;
   const bool inject = L.inject > 0;
   if (threadIdx.y == 0) slab_e_march<real, 0, kMulti>(a, inject, w);
@@ -571,6 +574,7 @@ __device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const Sla
 template <typename real>
 __device__ __forceinline__ void slab_h_body(const SweepArgs<real>& a, const SlabLaunch& L, int block) {
   const SlabWork w = slab_work<real>(L, a.nx, block);
+  pdl_wait();
   if (!w.live) return;
   if (threadIdx.y == 0) slab_h_march<real, 0>(a, w);
   else if (threadIdx.y == 1) slab_h_march<real, 1>(a, w);
@@ -584,6 +588,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4)
     slab_h_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L,
                   const __grid_constant__ ProbeArgs<real> pr, int off) {
   if ((int)blockIdx.x < L.extra) {
+    pdl_wait();
     probe_sample(pr, 0, (int)blockIdx.x, off - 1);
     return;
   }
@@ -602,6 +607,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4)
   const uint3 bid = G.block(&e);
   const SlabLaunch& l = stage_args(L + e, launch);
   if ((int)bid.x < l.extra) {
+    pdl_wait();
     if (off > 0) probe_sample(PR[e], 0, (int)bid.x, off - 1);
     return;
   }
@@ -688,7 +694,7 @@ int inject_blocks(const EdgeArgs<real>& ed) {
 
 template <typename real>
 cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, const EdgeArgs<real>* ed,
-                        const ProbeArgs<real>* pr, int off) {
+                        const ProbeArgs<real>* pr, int off, bool pdl) {
   SlabLaunch L;
   long long blocks = 0;
   if (const cudaError_t e = slab_plan(a, kind, &L, &blocks)) return e;
@@ -700,27 +706,23 @@ cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, cons
   const ProbeArgs<real> no_pr{};
   const EdgeArgs<real>& e = ed ? *ed : no_ed;
   const ProbeArgs<real>& p = pr ? *pr : no_pr;
-  if (kind == 0 && a.ade_P > 1)
-    slab_e_kernel<real, true><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, e, p, off);
-  else if (kind == 0)
-    slab_e_kernel<real, false><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, e, p, off);
-  else
-    slab_h_kernel<real><<<(unsigned)blocks, dim3(kSlabCols, 3), 0, s>>>(a, L, p, off);
-  return cudaGetLastError();
+  const dim3 grid((unsigned)blocks), block(kSlabCols, 3);
+  if (kind == 0)
+    return launch_pdl(pdl, a.ade_P > 1 ? slab_e_kernel<real, true> : slab_e_kernel<real, false>, grid, block, 0, s, a, L,
+                      e, p, off);
+  return launch_pdl(pdl, slab_h_kernel<real>, grid, block, 0, s, a, L, p, off);
 }
 
 template <typename real>
 cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
                               const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
-                              int off, cudaStream_t s) {
+                              int off, bool pdl, cudaStream_t s) {
   if (blocks <= 0) return cudaSuccess;
-  if (kind == 0 && multi_pole)
-    slab_e_batch_kernel<real, true><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, ED, PR, G, off);
-  else if (kind == 0)
-    slab_e_batch_kernel<real, false><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, ED, PR, G, off);
-  else
-    slab_h_batch_kernel<real><<<blocks, dim3(kSlabCols, 3), 0, s>>>(A, L, PR, G, off);
-  return cudaGetLastError();
+  const dim3 grid(blocks), block(kSlabCols, 3);
+  if (kind == 0)
+    return launch_pdl(pdl, multi_pole ? slab_e_batch_kernel<real, true> : slab_e_batch_kernel<real, false>, grid, block,
+                      0, s, A, L, ED, PR, G, off);
+  return launch_pdl(pdl, slab_h_batch_kernel<real>, grid, block, 0, s, A, L, PR, G, off);
 }
 
 template <typename real>
@@ -747,10 +749,10 @@ cudaError_t preload_slab() {
   template cudaError_t slab_plan<real>(const SweepArgs<real>&, int, SlabLaunch*, long long*, int);                    \
   template long long slab_vecs<real>(const SweepArgs<real>&, int);                                                    \
   template cudaError_t launch_slab_batch<real>(const SweepArgs<real>*, const SlabLaunch*, const EdgeArgs<real>*,      \
-                                               const ProbeArgs<real>*, const BatchGrid&, int, int, bool, int,         \
+                                               const ProbeArgs<real>*, const BatchGrid&, int, int, bool, int, bool,   \
                                                cudaStream_t);                                                         \
   template cudaError_t launch_slab<real>(const SweepArgs<real>&, int, cudaStream_t, const EdgeArgs<real>*,            \
-                                         const ProbeArgs<real>*, int);
+                                         const ProbeArgs<real>*, int, bool);
 OAFDTD_SLAB(float)
 OAFDTD_SLAB(double)
 

@@ -437,7 +437,7 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
   }
   const long long tiles = (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + BN - 1) / BN);
   const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch_pdl(umma_gemm_kernel<BN>, dim3(grid), dim3(kUThreads), bytes, s, g, amap, bmap, c32map, c16map, c16tmap);
+  return launch_pdl(true, umma_gemm_kernel<BN>, dim3(grid), dim3(kUThreads), bytes, s, g, amap, bmap, c32map, c16map, c16tmap);
 }
 
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
