@@ -15,8 +15,14 @@
 // one-row halo on every side; the plane itself is still staged from the previous step of the
 // march), H^{n-1/2} of the plane (with a halo on the low sides) and the material index. Each warp
 // waits for the copies itself; one block barrier per plane (after the H update) also agrees on
-// whether every wait succeeded, and the warps release their slots through an mbarrier that the
-// leader waits on before it refills them. It then
+// whether every wait succeeded. Past it no thread reads E^n of the plane in shared memory (each
+// keeps its own cells), nor anything of the plane before: the leader refills those slots at once,
+// a plane and a half before their data are wanted. (Refilled when the last warp had left the plane,
+// one plane ahead, with the leader waiting for it: 2290 of a plane's 7200 cycles went by in waits
+// for data and 500 in the leader's; now 790 of 5820. The Debye currents come by plain loads from the
+// end of the plane before: loaded between the components' updates they held up the coefficient
+// gathers, 2350 to 3050 cycles.) At 400x400x120, two members, the sweep with the H work that runs
+// beside it moves 2.8 GB in 0.43 ms, what the memory gives. It then
 //   1. updates H of its cells (and of the halo column x0 - 1 and row y0 - 1) in shared memory,
 //      with the H sweep's arithmetic (packages/oa-fdtd/src/oa_fdtd/reference.py:152-165);
 //   2. updates E of its cells from the new H (and the carried H of the plane below), with the
@@ -46,7 +52,7 @@ constexpr int kEH = kFY + 2;       // staged E rows: one each side (10)
 constexpr int kHW = kFW + 4;       // staged H width: one quad on the low side (132)
 constexpr int kHH = kFY + 1;       // staged H rows: one on the low side (9)
 constexpr int kSE = 3;             // E slots: the plane, the one above, one in flight
-constexpr int kSH = 2;             // H + index slots: the plane, one in flight
+constexpr int kSH = 3;             // H + index slots: the plane, two in flight (113 KB a block: two on an SM)
 
 template <typename real>
 struct EPlane {
@@ -54,7 +60,9 @@ struct EPlane {
 };
 template <typename real>
 struct HPlane {
-  Box<real, kHH, kHW> h[3];
+  Box<real, kHH, kFW> hx;  // the halo row
+  Box<real, kFY, kHW> hy;  // the halo column
+  Box<real, kHH, kHW> hz;  // both
   Box<uint16_t, kFY, kFW> m[3];
 };
 template <typename real>
@@ -75,12 +83,12 @@ __device__ __forceinline__ void issue_e(const FusedMaps& tm, EPlane<real>& s, un
 template <typename real>
 __device__ __forceinline__ void issue_h(const FusedMaps& tm, HPlane<real>& s, unsigned long long* bar, int x0, int y0,
                                         int k, int b) {
-  mbar_expect_tx(bar, 3u * (kHH * kHW * sizeof(real) + kFY * kFW * sizeof(uint16_t)));
+  mbar_expect_tx(bar, (kHH * kFW + kFY * kHW + kHH * kHW) * sizeof(real) + 3u * kFY * kFW * sizeof(uint16_t));
+  tma_load4(&s.hx, &tm.h_halo[0], bar, x0, y0 - 1, k, b);
+  tma_load4(&s.hy, &tm.h_halo[1], bar, x0 - 4, y0, k, b);
+  tma_load4(&s.hz, &tm.h_halo[2], bar, x0 - 4, y0 - 1, k, b);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    tma_load4(&s.h[c], &tm.h_halo[c], bar, x0 - 4, y0 - 1, k, b);
-    tma_load3(&s.m[c], &tm.mat[c], bar, x0, y0, k);
-  }
+  for (int c = 0; c < 3; ++c) tma_load3(&s.m[c], &tm.mat[c], bar, x0, y0, k);
 }
 
 // A wait gave up: the leader records it and waits (bounded) for every copy it issued that has not
@@ -99,7 +107,6 @@ template <typename real, bool kMulti>
 __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const FusedMaps& tm, const uint3 bid) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ unsigned long long bar_e[kSE], bar_h[kSH];
-  __shared__ unsigned long long bar_done;  // one arrival per warp when it is done with a plane
   FusedSmem<real>& sm = *reinterpret_cast<FusedSmem<real>*>(align_smem(smem_raw));
   const int tx = threadIdx.x, ty = threadIdx.y;
   const bool leader = tx == 0 && ty == 0;
@@ -135,7 +142,6 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
     for (int s = 0; s < kSE; ++s) mbar_init(&bar_e[s], 1);
 #pragma unroll
     for (int s = 0; s < kSH; ++s) mbar_init(&bar_h[s], 1);
-    mbar_init(&bar_done, kFY);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -160,26 +166,24 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
     return;
   }
   Quad<real> hx_m{}, hy_m{};  // H^{n+1/2} of the plane below at the own cells, carried
-  Quad<real> jcur[3], jnext[3];
+  // Debye currents of the next plane to be updated, under way from the end of the plane before
+  Quad<real> j4[3];
+  auto load_j = [&](int c, int k) {
+    if (a.ade_P == 1 && k < kc1 && k >= a.jk0[c] && k < a.jk0[c] + a.jnk[c])
+      j4[c] = ld4(a.J[c] + (((long long)b * a.jnk[c] + (k - a.jk0[c])) * Y + j) * X + i0);
+  };
 #pragma unroll
-  for (int c = 0; c < 3; ++c) jcur[c] = Quad<real>{};
-  if (live && a.ade_P == 1) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      if (kc0 >= a.jk0[c] && kc0 < a.jk0[c] + a.jnk[c])
-        jcur[c] = ld4(a.J[c] + (((long long)b * a.jnk[c] + (kc0 - a.jk0[c])) * Y + j) * X + i0);
+  for (int c = 0; c < 3; ++c) {
+    j4[c] = Quad<real>{};
+    if (live) load_j(c, kc0);
   }
+  real ipz_next = a.ip[2][ks], idz_next = a.idd[2][ks];  // the plane's z metrics, loaded a plane ahead
   for (int t = 0; t < n_planes; ++t) {
     const int k = ks + t;
+    const real ipz = ipz_next, idz = idz_next;
+    ipz_next = a.ip[2][k + 1];  // k + 1 <= nz + 1
+    idz_next = a.idd[2][k + 1];
     const bool inner = k >= kc0;  // a plane of the fused box (else the carry plane below it)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) jnext[c] = Quad<real>{};
-    if (inner && live && a.ade_P == 1 && k + 1 < kc1) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        if (k + 1 >= a.jk0[c] && k + 1 < a.jk0[c] + a.jnk[c])
-          jnext[c] = ld4(a.J[c] + (((long long)b * a.jnk[c] + (k + 1 - a.jk0[c])) * Y + j) * X + i0);
-    }
     // each thread acquires the plane's copies itself; whether every wait succeeded is agreed on
     // at the block's one barrier of the plane, before any global store
     ok = ok && mbar_wait(&bar_e[(t + 1) % kSE], (unsigned)(((t + 1) / kSE) & 1), kWaitNs);
@@ -188,16 +192,16 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
     const EPlane<real>& en = sm.e[(t + 1) % kSE];   // E^n of plane k + 1
     HPlane<real>& hs = sm.h[t % kSH];               // H^{n-1/2} of plane k, updated in place
     const bool kin = k <= nz;
-    const real ipz = a.ip[2][k];
     // ---- 1. H^{n+1/2} of the own quad (the H sweep's arithmetic), kept in shared memory
-    Quad<real> hx_n{}, hy_n{}, hz_n{};
+    Quad<real> hx_n{}, hy_n{}, hz_n{}, ex{}, ey{}, ez{};
     if (live) {
-      const Quad<real> ex = ld4(&ec.e[0].v[ty + 1][cc]), ey = ld4(&ec.e[1].v[ty + 1][cc]);
-      const Quad<real> ez = ld4(&ec.e[2].v[ty + 1][cc]);
+      ex = ld4(&ec.e[0].v[ty + 1][cc]);
+      ey = ld4(&ec.e[1].v[ty + 1][cc]);
+      ez = ld4(&ec.e[2].v[ty + 1][cc]);
       const real ez_r = ec.e[2].v[ty + 1][cc + 4], ey_r = ec.e[1].v[ty + 1][cc + 4];
-      hx_n = ld4(&hs.h[0].v[ty + 1][cc]);
-      hy_n = ld4(&hs.h[1].v[ty + 1][cc]);
-      hz_n = ld4(&hs.h[2].v[ty + 1][cc]);
+      hx_n = ld4(&hs.hx.v[ty + 1][4 * tx]);
+      hy_n = ld4(&hs.hy.v[ty][cc]);
+      hz_n = ld4(&hs.hz.v[ty + 1][cc]);
       if (j <= ny && kin) {  // Hx: node along x (1..nx+1), cell along y and z
         const Quad<real> ezy = ld4(&ec.e[2].v[ty + 2][cc]);
         const Quad<real> ey1 = ld4(&en.e[1].v[ty + 1][cc]);
@@ -232,14 +236,14 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         }
       }
       if (inner) {
-        st4(&hs.h[0].v[ty + 1][cc], hx_n);
-        st4(&hs.h[1].v[ty + 1][cc], hy_n);
-        st4(&hs.h[2].v[ty + 1][cc], hz_n);
+        st4(&hs.hx.v[ty + 1][4 * tx], hx_n);
+        st4(&hs.hy.v[ty][cc], hy_n);
+        st4(&hs.hz.v[ty + 1][cc], hz_n);
       }
     }
     if (inner && halo_live) {  // the halo row y0 - 1: Hx and Hz, one cell per lane, every warp a share
       const int jh = y0 - 1, i = x0 + hc, ch = 4 + hc;
-      real hx = hs.h[0].v[0][ch], hz = hs.h[2].v[0][ch];
+      real hx = hs.hx.v[0][hc], hz = hs.hz.v[0][ch];
       const real ex = ec.e[0].v[0][ch], ey = ec.e[1].v[0][ch], ez = ec.e[2].v[0][ch];
       const real ezy = ec.e[2].v[1][ch], exy = ec.e[0].v[1][ch];
       const real ey1 = en.e[1].v[0][ch], eyr = ec.e[1].v[0][ch + 1];
@@ -253,12 +257,12 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         const real d1 = (exy - ex) * ipy_h;
         if (i >= 1 && i <= nx) hz = hz + dtmu * ((-d0) + d1);
       }
-      hs.h[0].v[0][ch] = hx;
-      hs.h[2].v[0][ch] = hz;
+      hs.hx.v[0][hc] = hx;
+      hs.hz.v[0][ch] = hz;
     }
     if (inner && live && tx == 0) {  // the halo column x0 - 1: Hy and Hz
       const int ih = x0 - 1;
-      real hy = hs.h[1].v[ty + 1][3], hz = hs.h[2].v[ty + 1][3];
+      real hy = hs.hy.v[ty][3], hz = hs.hz.v[ty + 1][3];
       if (kin && ih >= 1 && ih <= nx) {
         const real d0 = (ec.e[2].v[ty + 1][4] - ec.e[2].v[ty + 1][3]) * ipx_h;
         const real d1 = (en.e[0].v[ty + 1][3] - ec.e[0].v[ty + 1][3]) * ipz;
@@ -269,21 +273,32 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         const real d1 = (ec.e[0].v[ty + 2][3] - ec.e[0].v[ty + 1][3]) * ipy;
         hz = hz + dtmu * ((-d0) + d1);
       }
-      hs.h[1].v[ty + 1][3] = hy;
-      hs.h[2].v[ty + 1][3] = hz;
+      hs.hy.v[ty][3] = hy;
+      hs.hz.v[ty + 1][3] = hz;
     }
-    // the new H of the plane (halo included) is complete
+    // The new H of the plane (halo included) is complete; nothing reads E(k) in shared memory any more
+    // (a thread keeps its own cells), nor H(k - 1) and its index.
+    fence_proxy_async();
     if (__syncthreads_or(!ok)) {
       abort_fused(bar_e, bar_h, t + 1, e_issued, t, h_issued, a.status, leader);
       return;
+    }
+    if (leader) {  // those slots are refilled
+      if (e_issued < n_e) {  // E(k + kSE)
+        issue_e(tm, sm.e[e_issued % kSE], &bar_e[e_issued % kSE], x0, y0, ks + e_issued, b);
+        ++e_issued;
+      }
+      if (t > 0 && h_issued < n_planes) {  // H and index of plane k - 1 + kSH
+        issue_h(tm, sm.h[h_issued % kSH], &bar_h[h_issued % kSH], x0, y0, ks + h_issued, b);
+        ++h_issued;
+      }
     }
     // ---- 2. E^{n+1} of the own quad, and the stores
     if (inner && live) {
       const long long p = base + (long long)k * X * Y + (long long)j * X + i0;
       const long long q = (long long)k * X * Y + (long long)j * X + i0;
-      const real idz = a.idd[2][k];
-      const Quad<real> hzy = ld4(&hs.h[2].v[ty][cc]), hxy = ld4(&hs.h[0].v[ty][cc]);
-      const real hz_l = hs.h[2].v[ty + 1][cc - 1], hy_l = hs.h[1].v[ty + 1][cc - 1];
+      const Quad<real> hzy = ld4(&hs.hz.v[ty][cc]), hxy = ld4(&hs.hx.v[ty][4 * tx]);
+      const real hz_l = hs.hz.v[ty + 1][cc - 1], hy_l = hs.hy.v[ty][cc - 1];
       ZTerm<real> none;
       none.on = false;
       real d0[4], d1[4];
@@ -293,8 +308,8 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         d0[e] = (hz_n.v[e] - hzy.v[e]) * idy;
         d1[e] = (hy_n.v[e] - hy_m.v[e]) * idz;
       }
-      e_apply<real, false, kMulti>(a, 0, a.Eo[0] + base, q, ld4(&ec.e[0].v[ty + 1][cc]), &hs.m[0].v[ty][4 * tx], d0,
-                                   d1, true, jcur[0], none, i0, j, k, b, sm.coef);
+      e_apply<real, false, kMulti>(a, 0, a.Eo[0] + base, q, ex, &hs.m[0].v[ty][4 * tx], d0,
+                                   d1, true, j4[0], none, i0, j, k, b, sm.coef);
       // Ey: terms (a = z, +Hx) then (a = x, -Hz)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -302,8 +317,8 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         d0[e] = (hz_n.v[e] - hzl) * idx4.v[e];
         d1[e] = (hx_n.v[e] - hx_m.v[e]) * idz;
       }
-      e_apply<real, false, kMulti>(a, 1, a.Eo[1] + base, q, ld4(&ec.e[1].v[ty + 1][cc]), &hs.m[1].v[ty][4 * tx], d0,
-                                   d1, false, jcur[1], none, i0, j, k, b, sm.coef);
+      e_apply<real, false, kMulti>(a, 1, a.Eo[1] + base, q, ey, &hs.m[1].v[ty][4 * tx], d0,
+                                   d1, false, j4[1], none, i0, j, k, b, sm.coef);
       // Ez: terms (a = x, +Hy) then (a = y, -Hx)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -311,38 +326,18 @@ __device__ __forceinline__ void fused_body(const SweepArgs<real>& a, const Fused
         d0[e] = (hy_n.v[e] - hyl) * idx4.v[e];
         d1[e] = (hx_n.v[e] - hxy.v[e]) * idy;
       }
-      e_apply<real, false, kMulti>(a, 2, a.Eo[2] + base, q, ld4(&ec.e[2].v[ty + 1][cc]), &hs.m[2].v[ty][4 * tx], d0,
-                                   d1, true, jcur[2], none, i0, j, k, b, sm.coef);
+      e_apply<real, false, kMulti>(a, 2, a.Eo[2] + base, q, ez, &hs.m[2].v[ty][4 * tx], d0,
+                                   d1, true, j4[2], none, i0, j, k, b, sm.coef);
       if (j <= ny && kin) st4(a.Ho[0] + p, hx_n);
       if (kin) st4(a.Ho[1] + p, hy_n);
       if (j <= ny) st4(a.Ho[2] + p, hz_n);
     }
+    if (inner && live) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) load_j(c, k + 1);
+    }
     hx_m = hx_n;
     hy_m = hy_n;
-    if (inner) {  // the carry plane keeps the currents of the chunk's first plane
-#pragma unroll
-      for (int c = 0; c < 3; ++c) jcur[c] = jnext[c];
-    }
-    // This warp is done with E(k) and the H / index slot of plane k: its reads and writes of
-    // the slots are ordered before the copies that refill them, and the warp moves on to the
-    // next plane without waiting for the others. The leader refills the slots once every warp
-    // has arrived (phase t of bar_done; phase t + 1 cannot complete before the leader has passed
-    // the next plane's barrier).
-    fence_proxy_async();
-    __syncwarp();
-    if (tx == 0) mbar_arrive(&bar_done);
-    if (leader && ok && (e_issued < n_e || h_issued < n_planes)) {
-      // a wait that gives up is reported at the next plane's barrier; nothing more is issued
-      ok = mbar_wait(&bar_done, (unsigned)(t & 1), kWaitNs);
-      if (ok && e_issued < n_e) {  // E(k + 3) into the slot of E(k)
-        issue_e(tm, sm.e[e_issued % kSE], &bar_e[e_issued % kSE], x0, y0, ks + e_issued, b);
-        ++e_issued;
-      }
-      if (ok && h_issued < n_planes) {  // H and index of plane k + 2 into the slot of plane k
-        issue_h(tm, sm.h[h_issued % kSH], &bar_h[h_issued % kSH], x0, y0, ks + h_issued, b);
-        ++h_issued;
-      }
-    }
   }
 }
 
@@ -409,13 +404,13 @@ bool encode_fused_maps(const SweepArgs<real>& a, FusedMaps* m, std::string* why)
   const cuuint64_t rs = sizeof(real);
   const cuuint64_t strides[3] = {X * rs, X * Y * rs, X * Y * Z * rs};
   const cuuint32_t ebox[4] = {kEW, kEH, 1, 1};
-  const cuuint32_t hbox[4] = {kHW, kHH, 1, 1};
+  const cuuint32_t hbox[3][4] = {{kFW, kHH, 1, 1}, {kHW, kFY, 1, 1}, {kHW, kHH, 1, 1}};
   const cuuint32_t mbox[3] = {kFW, kFY, 1};
   const cuuint64_t mdims[3] = {X, Y, Z};
   const cuuint64_t mstrides[2] = {X * 2, X * Y * 2};
   for (int c = 0; c < 3; ++c) {
     if (!encode_tensor_map(&m->e_halo[c], dt, 4, a.E[c], dims, strides, ebox, "E halo", why) ||
-        !encode_tensor_map(&m->h_halo[c], dt, 4, a.H[c], dims, strides, hbox, "H halo", why) ||
+        !encode_tensor_map(&m->h_halo[c], dt, 4, a.H[c], dims, strides, hbox[c], "H halo", why) ||
         !encode_tensor_map(&m->mat[c], CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, a.mat[c], mdims, mstrides, mbox, "mat",
                            why))
       return false;
