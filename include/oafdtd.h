@@ -447,6 +447,18 @@ int oafdtd_mlp_adam_net(float* w, void* w16, void* w16t, const float* grad, floa
 int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out, const int32_t* idx, int32_t rows,
                      int32_t groups, void* x16, void* x16t, float* t32, int32_t* counter, void* stream);
 
+/* The outputs of a network of n_layers for every member, from inputs x in host memory (rows x fan_in of
+ * the first layer, FP32; read before the call returns): member k's outputs (rows x fan_out of the last
+ * layer, FP32) at y + k * y_stride. p32: FP32 parameters (the biases are read), w16t: transposed BF16
+ * weights, both k * stride elements into their buffer; layers as in oafdtd_mlp_adam_net; act: the hidden
+ * layers' activation as in oafdtd_mlp_gemm_tn (1 or 3). work: device memory of
+ * oafdtd_mlp_predict_bytes(...) bytes, 256-byte aligned, this call's own until the stream has passed it.
+ * status as in oafdtd_mlp_gemm_tn. */
+int64_t oafdtd_mlp_predict_bytes(int32_t rows, int32_t n_layers, const int64_t* layers, int32_t members);
+int oafdtd_mlp_predict(const float* x, int32_t rows, const float* p32, const void* w16t, int32_t n_layers,
+                       const int64_t* layers, int32_t members, int64_t stride, int32_t act, void* work, float* y,
+                       int64_t y_stride, int32_t* status, void* stream);
+
 /* *counter += 1 on the device (the Adam step number inside a captured training step). */
 int oafdtd_mlp_count(int32_t* counter, void* stream);
 

@@ -553,6 +553,12 @@ __global__ void __launch_bounds__(128) batch_kernel(const float* x, int n_in, co
   for (int c = threadIdx.x; c < n_out / 4; c += blockDim.x) d[c] = s[c];
 }
 
+// An FP32 matrix of n elements as BF16, once per blockIdx.y.
+__global__ void __launch_bounds__(256) replicate_kernel(const float* src, long long n, __nv_bfloat16* dst) {
+  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < n) dst[blockIdx.y * n + e] = __float2bfloat16(src[e]);
+}
+
 // Rows idx[0..rows) of an FP32 matrix with `cols` columns, into FP32 and/or BF16 copies.
 __global__ void gather_kernel(const float* src, int cols, const int* idx, int rows, float* d32,
                               __nv_bfloat16* d16) {
@@ -778,6 +784,55 @@ int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out
   oafdtd::batch_kernel<<<(unsigned)(rows * groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       x, n_in, t, n_out, idx, rows, static_cast<__nv_bfloat16*>(x16), static_cast<__nv_bfloat16*>(x16t), t32, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+static size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+// A prediction is a chain of one GEMM per layer, some 8 us each: 62 us for 412 rows of 8 members and seven
+// layers. Layer by layer from Python, with the inputs' conversions and a buffer per layer from the
+// framework, it took 200 us; from here, two activation buffers in turn, 125.
+int64_t oafdtd_mlp_predict_bytes(int32_t rows, int32_t n_layers, const int64_t* layers, int32_t members) {
+  if (rows < 1 || n_layers < 1 || !layers || members < 1) return 0;
+  int64_t widest = 0;
+  for (int l = 0; l + 1 < n_layers; ++l) widest = layers[4 * l + 2] > widest ? layers[4 * l + 2] : widest;
+  const size_t n = (size_t)rows * (size_t)layers[1];
+  return (int64_t)(align256(n * 4) + align256(n * 2 * members) + 2 * align256((size_t)rows * widest * 2 * members));
+}
+
+int oafdtd_mlp_predict(const float* x, int32_t rows, const float* p32, const void* w16t, int32_t n_layers,
+                       const int64_t* layers, int32_t members, int64_t stride, int32_t act, void* work, float* y,
+                       int64_t y_stride, int32_t* status, void* stream) {
+  if (!x || rows < 1 || !p32 || !w16t || n_layers < 1 || !layers || members < 1 || members > 65535 || !work || !y) {
+    oafdtd::set_last_error("oafdtd_mlp_predict: bad arguments");
+    return -1;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  int64_t widest = 0;
+  for (int l = 0; l + 1 < n_layers; ++l) widest = layers[4 * l + 2] > widest ? layers[4 * l + 2] : widest;
+  const long long n = (long long)rows * layers[1];
+  char* at = static_cast<char*>(work);
+  float* x32 = reinterpret_cast<float*>(at);
+  at += align256((size_t)n * 4);
+  void* in = at;
+  at += align256((size_t)n * 2 * members);
+  void* act_buf[2] = {at, at + align256((size_t)rows * widest * 2 * members)};
+  if (cudaMemcpyAsync(x32, x, (size_t)n * 4, cudaMemcpyHostToDevice, s) != cudaSuccess) return -3;
+  oafdtd::replicate_kernel<<<dim3((unsigned)((n + 255) / 256), members), 256, 0, s>>>(
+      x32, n, static_cast<__nv_bfloat16*>(in));
+  if (cudaGetLastError() != cudaSuccess) return -3;
+  for (int l = 0; l < n_layers; ++l) {
+    const int64_t* q = layers + 4 * l;  // weight offset, fan_in, fan_out, bias offset
+    const int a = (int)q[1], b = (int)q[2];
+    const bool last = l == n_layers - 1;
+    void* out = act_buf[l & 1];
+    const int rc = oafdtd_mlp_gemm_tn(in, static_cast<const __nv_bfloat16*>(w16t) + q[0], last ? y : nullptr,
+                                      last ? nullptr : out, nullptr, p32 + q[3], nullptr, rows, b, a, a, a, b, rows,
+                                      last ? 0 : act, 0.f, members, (int64_t)rows * a, stride,
+                                      last ? y_stride : (int64_t)rows * b, (int64_t)b * rows, stride, status, stream);
+    if (rc != 0) return rc;
+    in = out;
+  }
+  return 0;
 }
 
 int oafdtd_mlp_count(int32_t* counter, void* stream) {

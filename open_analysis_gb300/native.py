@@ -223,6 +223,9 @@ SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
     ),
     "oafdtd_mlp_batch": (C.c_int, [C.c_void_p, _i32, C.c_void_p, _i32, C.c_void_p, _i32, _i32] + [C.c_void_p] * 5),
     "oafdtd_mlp_mse_grad_t": (C.c_int, [C.c_void_p, C.c_void_p, _i32, _i32] + [C.c_void_p] * 4 + [_i32, C.c_void_p]),
+    "oafdtd_mlp_predict_bytes": (C.c_int64, [_i32, _i32, C.c_void_p, _i32]),
+    "oafdtd_mlp_predict": (C.c_int, [C.c_void_p, _i32, C.c_void_p, C.c_void_p, _i32, C.c_void_p, _i32, C.c_int64, _i32,
+                                     C.c_void_p, C.c_void_p, C.c_int64, C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_count": (C.c_int, [C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_gather": (C.c_int, [C.c_void_p, _i32, C.c_void_p, _i32, C.c_void_p, C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_gemm_tn": (

@@ -707,17 +707,20 @@ class Mlp:
         torch = self.torch
         x = self.pad(x)
         n, g = x.shape[0], self.members
-        out = torch.empty((g, n, self.sizes[-1]), dtype=torch.float32, device=self.dev)
+        width, layers = self.sizes[-1], len(self.layout)
+        out = torch.empty((g, n, width), dtype=torch.float32, device=self.dev)
+        # inputs of another rank broadcast to members x rows: then member by member
+        xs = [x] if x.ndim == 2 else np.ascontiguousarray(np.broadcast_to(x, (g, n, x.shape[-1])))
+        work = torch.empty(int(self.lib.oafdtd_mlp_predict_bytes(min(n, chunk), layers, self._layers, g)),
+                           dtype=torch.uint8, device=self.dev)
         s = self._stream()
-        for a in range(0, n, chunk):
-            m = min(chunk, n - a)
-            x16 = torch.from_numpy(x[a : a + m]).to(self.dev).to(torch.bfloat16).expand(g, m, -1).contiguous()
-            acts = [torch.empty((g, m, b), dtype=torch.bfloat16, device=self.dev) for b in self.sizes[1:-1]]
-            y = out[:, a : a + m] if g == 1 or n == m else torch.empty((g, m, self.sizes[-1]), dtype=torch.float32,
-                                                                         device=self.dev)
-            self._forward(x16.data_ptr(), acts, y.data_ptr(), m, s)
-            if y.data_ptr() != out[:, a : a + m].data_ptr():
-                out[:, a : a + m].copy_(y)
+        for k, xk in enumerate(xs):
+            for a in range(0, n, chunk):
+                native.check(self.lib.oafdtd_mlp_predict(
+                    xk.ctypes.data + a * xk.strides[0], min(chunk, n - a), self.p32.data_ptr() + 4 * k * self.n_params,
+                    self.p16T.data_ptr() + 2 * k * self.n_params, layers, self._layers, g // len(xs), self.n_params,
+                    self.act, work.data_ptr(), out.data_ptr() + 4 * width * (k * n + a), n * width,
+                    self.status.data_ptr(), s), "predict")
         self.check_status()
         return out
 

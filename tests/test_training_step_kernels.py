@@ -83,3 +83,25 @@ def test_a_batch_is_its_gathered_rows(n_in, n_out, rows, groups):
                                       x16.data_ptr(), x16t.data_ptr(), t32.data_ptr(), step.data_ptr(), s), "batch")
     assert torch.equal(x16, x[idx.long()].bfloat16()) and torch.equal(x16t, x16.transpose(1, 2))
     assert torch.equal(t32, t[idx.long()]) and step.item() == 7
+
+
+@pytest.mark.parametrize("rows,chunk,members,act", [(1, 4096, 1, "tanh"), (37, 4096, 3, "relu"), (200, 64, 2, "tanh")])
+def test_prediction_is_the_layers_one_by_one(rows, chunk, members, act):
+    # one row; rows off every tile; chunks with a remainder, written into their place among the members
+    from open_analysis_gb300.surrogate import Mlp
+
+    net = Mlp([7, 40, 136, 24], 8, seed=5, members=members, act=act)
+    x = torch.randn(rows, 7, generator=torch.Generator().manual_seed(4)).numpy()
+    have = net.predict_device(x, chunk)
+    want = torch.empty_like(have)
+    for a in range(0, rows, chunk):
+        xc = torch.from_numpy(net.pad(x[a : a + chunk])).cuda().bfloat16()
+        m = xc.shape[0]
+        x16 = xc.expand(members, m, -1).contiguous()
+        acts = [torch.empty((members, m, b), dtype=torch.bfloat16, device="cuda") for b in net.sizes[1:-1]]
+        y = torch.empty((members, m, net.sizes[-1]), device="cuda")
+        net._forward(x16.data_ptr(), acts, y.data_ptr(), m, net._stream())
+        want[:, a : a + m] = y
+    assert torch.equal(have, want)
+    one = net.predict_device(x[0], chunk)  # a vector stands for as many equal rows as it is wide, padded
+    assert one.shape[1] == net.sizes[0] and torch.equal(one[:, :1], net.predict_device(x[:1], chunk))
