@@ -29,7 +29,10 @@
 // steps of 16). The training and prediction shapes are bound by latency, not by the tensor pipe (one
 // tile per CTA: launch, descriptors, two rounds of TMA, epilogue): the launches are programmatic
 // dependents, so a kernel sets up in the tail of the one before (8 x 256x512x512: 10.5 to 7.5 us;
-// 32 x 64x512x512, on mma.sync before: 8.5 us).
+// 32 x 64x512x512, on mma.sync before: 8.5 us). Of such a launch the first K step's tiles arrive 1.1 us
+// after its start, the eighth's at 4.6 with four in flight: as many are kept as fit, and the epilogue's
+// bias and mask are loaded before the wait for the accumulator (8 x 256x512x512 with tanh 7.0 to 6.8,
+// with a mask and three results 7.6 to 7.1 us).
 // Every mbarrier wait is bounded (about two seconds, and a poll count); a wait that gives up sets
 // the caller's status word and a flag the other roles poll, every role leaves its loop, copies
 // and MMAs in flight are waited for (bounded again) and TMEM is freed, so no launch hangs.
@@ -46,7 +49,10 @@ namespace oafdtd {
 
 namespace {
 
-constexpr int kUM = 128, kUK = 64, kUStages = 4, kEpiWarps = 8;
+constexpr int kUM = 128, kUK = 64, kEpiWarps = 8;
+// K steps in flight: what the 227 KB hold beside the epilogue's staging.
+template <int BN>
+constexpr int kUStages = BN == 64 ? 6 : 5;
 constexpr int kUThreads = 32 * (2 + kEpiWarps);
 constexpr unsigned long long kUWaitNs = 2000000000ull;
 constexpr unsigned kUPolls = 1u << 28;
@@ -182,20 +188,21 @@ __global__ void __launch_bounds__(kUThreads, 1)
                      const __grid_constant__ CUtensorMap bmap, const __grid_constant__ CUtensorMap c32map,
                      const __grid_constant__ CUtensorMap c16map, const __grid_constant__ CUtensorMap c16tmap) {
   extern __shared__ unsigned char umma_raw[];
-  __shared__ uint64_t full[kUStages], empty[kUStages], tfull[2], tempty[2], done;
+  constexpr int kS = kUStages<BN>;
+  __shared__ uint64_t full[kS], empty[kS], tfull[2], tempty[2], done;
   __shared__ uint32_t tmem_base;
   __shared__ int failed_sh, consumed_sh;
   volatile int* failed = &failed_sh;
   unsigned char* base = umma_raw + ((1024u - (saddr(umma_raw) & 1023u)) & 1023u);
   UStage<BN>* st = reinterpret_cast<UStage<BN>*>(base);
-  EpiStage* ep = reinterpret_cast<EpiStage*>(base + kUStages * sizeof(UStage<BN>));
+  EpiStage* ep = reinterpret_cast<EpiStage*>(base + kS * sizeof(UStage<BN>));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // the last tiles of each extent may reach past it: TMA fills loads there with zeros (a K step of
   // zeros adds nothing) and leaves stores out
   const int MT = (g.M + kUM - 1) / kUM, NT = (g.N + BN - 1) / BN, KT = (g.K + kUK - 1) / kUK;
   const int tiles = g.groups * MT * NT;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kUStages; ++s) {
+    for (int s = 0; s < kS; ++s) {
       ubar_init(&full[s], 1);
       ubar_init(&empty[s], 1);
     }
@@ -230,8 +237,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
         const int nt = tile % NT, mt = (tile / NT) % MT, gi = tile / (NT * MT);
         int kb = 0;
         for (; kb < KT; ++kb, ++issued) {
-          const int s = issued % kUStages;
-          const unsigned r = (unsigned)(issued / kUStages);
+          const int s = issued % kS;
+          const unsigned r = (unsigned)(issued / kS);
           if (!ubar_wait(&empty[s], (r & 1u) ^ 1u, failed)) break;
           ubar_expect(&full[s], kStageBytes);
           utma_load(st[s].a, &amap, &full[s], kb * kUK, mt * kUM, gi);
@@ -256,8 +263,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t d = tmem + (uint32_t)(acc * BN);
         for (int kb = 0; kb < KT; ++kb, ++it) {
-          const int s = it % kUStages;
-          ok = ubar_wait(&full[s], (unsigned)((it / kUStages) & 1), failed);
+          const int s = it % kS;
+          ok = ubar_wait(&full[s], (unsigned)((it / kS) & 1), failed);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const uint32_t a0 = saddr(st[s].a), b0 = saddr(st[s].b);
@@ -282,6 +289,24 @@ __global__ void __launch_bounds__(kUThreads, 1)
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
       const int nt = tile % NT, mt = (tile / NT) % MT, gi = tile / (NT * MT);
       const int acc = t & 1;
+      const int row0 = mt * kUM + 32 * q;  // the chunks' first row within the group
+      const int row = row0 + lane;         // this thread's row
+      // bias and mask of a chunk come before the wait for its accumulator
+      float bl = 0.f;
+      uint4 mk[4];
+      auto fetch = [&](int c) {
+        const int col0 = nt * BN + c;
+        bl = g.bias && col0 + lane < g.N ? g.bias[gi * g.sBias + col0 + lane] : 0.f;
+        if (g.act == 2 || g.act == 4) {
+          const uint4* mp = reinterpret_cast<const uint4*>(g.mask + gi * g.sC + (long long)row * g.ldc + col0);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            mk[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (row < g.M && col0 + 8 * k < g.N) mk[k] = mp[k];
+          }
+        }
+      };
+      fetch(half * (BN / 2));
       // warp-uniform outcome: the TMEM loads below are warp-collective
       const bool ok = __all_sync(0xffffffffu, ubar_wait(&tfull[acc], (unsigned)((t >> 1) & 1), failed));
       if (!ok) {
@@ -289,8 +314,6 @@ __global__ void __launch_bounds__(kUThreads, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const int row0 = mt * kUM + 32 * q;  // the chunk's first row within the group
-      const int row = row0 + lane;         // this thread's row
       for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
         uint32_t r[32];
         tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(acc * BN + c), r);
@@ -301,7 +324,6 @@ __global__ void __launch_bounds__(kUThreads, 1)
         }
         const int col0 = nt * BN + c;  // the chunk's first column
         if (row0 >= g.M || col0 >= g.N) continue;  // nothing of the chunk lies in C
-        const float bl = g.bias && col0 + lane < g.N ? g.bias[gi * g.sBias + col0 + lane] : 0.f;
         float v[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) + __shfl_sync(0xffffffffu, bl, j);
@@ -312,11 +334,9 @@ __global__ void __launch_bounds__(kUThreads, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = tanhf(v[j]);
         } else if (g.act == 2 || g.act == 4) {
-          const uint4* mp = reinterpret_cast<const uint4*>(g.mask + gi * g.sC + (long long)row * g.ldc + col0);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
-            if (row < g.M && col0 + 8 * k < g.N) w = mp[k];
+            const uint4 w = mk[k];
             const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
@@ -333,6 +353,7 @@ __global__ void __launch_bounds__(kUThreads, 1)
             }
           }
         }
+        if (c + 32 < (half + 1) * (BN / 2)) fetch(c + 32);
         // the previous chunk's stores have read the staging buffers
         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
         __syncwarp();
@@ -380,7 +401,7 @@ __global__ void __launch_bounds__(kUThreads, 1)
   if (warp == 0 && lane == 0) {
     // after a failure: copies issued and never consumed land before the CTA exits (bounded)
     const int consumed = *(volatile int*)&consumed_sh;
-    for (int k = consumed; k < issued; ++k) ubar_wait(&full[k % kUStages], (unsigned)((k / kUStages) & 1), nullptr);
+    for (int k = consumed; k < issued; ++k) ubar_wait(&full[k % kS], (unsigned)((k / kS) & 1), nullptr);
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
@@ -425,7 +446,7 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
   g.M = p.M, g.N = p.N, g.K = p.K, g.ldc = p.ldc, g.act = p.act, g.groups = p.groups;
   g.has32 = p.C32 != nullptr, g.has16 = p.C16 != nullptr, g.has16t = p.C16T != nullptr;
   g.status = p.status;
-  const size_t bytes = sizeof(UStage<BN>) * kUStages + sizeof(EpiStage) * kEpiWarps + 1024;
+  const size_t bytes = sizeof(UStage<BN>) * kUStages<BN> + sizeof(EpiStage) * kEpiWarps + 1024;
   cudaError_t err = cudaFuncSetAttribute(umma_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   static int sms = 0;
@@ -475,7 +496,8 @@ static_assert(sizeof(UStage<128>) == (kUM + 128) * kUK * 2, "stage tiles are con
 static_assert(sizeof(UStage<64>) == (kUM + 64) * kUK * 2, "stage tiles are contiguous and 1024-byte multiples");
 static_assert(sizeof(EpiStage) == 8192, "epilogue staging: three 1024-byte aligned chunks");
 static_assert(kUK * sizeof(__nv_bfloat16) == 128, "one K step is one 128-byte swizzle row");
-static_assert(sizeof(UStage<128>) * kUStages + sizeof(EpiStage) * kEpiWarps + 1024 <= 232448,
+static_assert(sizeof(UStage<128>) * kUStages<128> + sizeof(EpiStage) * kEpiWarps + 1024 + 256 <= 232448 &&
+                  sizeof(UStage<64>) * kUStages<64> + sizeof(EpiStage) * kEpiWarps + 1024 + 256 <= 232448,
               "shared memory within the 227 KB a CTA may use");
 
 }  // namespace oafdtd
