@@ -426,6 +426,17 @@ int oafdtd_mlp_gemm_tn(const void* A, const void* B, float* C32, void* C16, void
                        int32_t ldct, int32_t act, float beta, int32_t groups, int64_t strideA, int64_t strideB,
                        int64_t strideC, int64_t strideCT, int64_t strideBias, int32_t* status, void* stream);
 
+/* n independent products C32 = A . B^T in FP32, arguments as in oafdtd_mlp_gemm_tn: in as few launches as
+ * the tcgen05 kernel allows, each with the bits of its own call. */
+typedef struct {
+  const void* A;
+  const void* B;
+  float* C32;
+  int32_t M, N, K, lda, ldb, ldc, groups;
+  int64_t strideA, strideB, strideC;
+} oafdtd_gemm;
+int oafdtd_mlp_gemm_list(const oafdtd_gemm* list, int32_t n, int32_t* status, void* stream);
+
 /* dst_g (cols x rows, leading dimension ldd) = src_g^T (rows x cols, leading dimension lds), BF16,
  * for g < groups, src_g and dst_g src_stride and dst_stride elements after group g - 1's. */
 int oafdtd_mlp_transpose(const void* src, int32_t rows, int32_t cols, int32_t lds, void* dst, int32_t ldd,

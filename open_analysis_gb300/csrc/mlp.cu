@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "../../include/oafdtd.h"
 #include "oafdtd_internal.cuh"
 
 namespace oafdtd {
@@ -784,6 +785,44 @@ int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out
   oafdtd::batch_kernel<<<(unsigned)(rows * groups), 128, 0, static_cast<cudaStream_t>(stream)>>>(
       x, n_in, t, n_out, idx, rows, static_cast<__nv_bfloat16*>(x16), static_cast<__nv_bfloat16*>(x16t), t32, counter);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+int oafdtd_mlp_gemm_list(const oafdtd_gemm* list, int32_t n, int32_t* status, void* stream) {
+  if (!list || n < 1) {
+    oafdtd::set_last_error("oafdtd_mlp_gemm_list: bad arguments");
+    return -1;
+  }
+  for (int32_t at = 0; at < n;) {
+    // as many as one launch takes, where every one suits it; else one by one
+    oafdtd::UmmaProblem p[oafdtd::kUmmaList];
+    int k = 0;
+    for (; k < oafdtd::kUmmaList && at + k < n; ++k) {
+      const oafdtd_gemm& q = list[at + k];
+      p[k] = oafdtd::UmmaProblem{q.A, q.B, q.C32, nullptr, nullptr, nullptr, nullptr, q.M, q.N, q.K, q.lda, q.ldb,
+                                 q.ldc, q.M, 0, q.groups, q.strideA, q.strideB, q.strideC, 0, 0, 0.f, status};
+      if (!q.A || !q.B || !q.C32 || q.groups > 65535 || !oafdtd::umma_shape_ok(p[k])) break;
+    }
+    if (k > 1) {
+      std::string why;
+      const cudaError_t err = oafdtd::launch_umma_list(p, k, static_cast<cudaStream_t>(stream), &why);
+      if (err == cudaSuccess) {
+        at += k;
+        continue;
+      }
+      if (err != cudaErrorNotSupported) {
+        oafdtd::set_last_error(std::string("oafdtd_mlp_gemm_list: ") + (why.empty() ? cudaGetErrorString(err) : why));
+        return -3;
+      }
+    }
+    for (int end = at + (k > 1 ? k : 1); at < end; ++at) {
+      const oafdtd_gemm& q = list[at];
+      if (const int rc = oafdtd_mlp_gemm_tn(q.A, q.B, q.C32, nullptr, nullptr, nullptr, nullptr, q.M, q.N, q.K, q.lda,
+                                            q.ldb, q.ldc, q.M, 0, 0.f, q.groups, q.strideA, q.strideB, q.strideC, 0, 0,
+                                            status, stream))
+        return rc;
+    }
+  }
+  return 0;
 }
 
 static size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }

@@ -182,11 +182,33 @@ __device__ __forceinline__ void raise_failure(volatile int* failed, int* status)
   if (status) atomicOr(status, 1);
 }
 
-template <int BN>
-__global__ void __launch_bounds__(kUThreads, 1)
-    umma_gemm_kernel(const __grid_constant__ UmmaArgs g, const __grid_constant__ CUtensorMap amap,
-                     const __grid_constant__ CUtensorMap bmap, const __grid_constant__ CUtensorMap c32map,
-                     const __grid_constant__ CUtensorMap c16map, const __grid_constant__ CUtensorMap c16tmap) {
+// The problems of one launch, with the first tile of each (first[n]: all of them).
+template <int kMax>
+struct UmmaList {
+  CUtensorMap a[kMax], b[kMax], c32[kMax], c16[kMax], c16t[kMax];
+  UmmaArgs g[kMax];
+  int first[kMax + 1];
+  int n;
+};
+
+// Where a tile lies: its problem, row and column of tiles, group, and the problem's K steps. The last
+// tiles of each extent may reach past it: TMA fills loads there with zeros (a K step of zeros adds
+// nothing) and leaves stores out.
+struct UmmaTile {
+  int p, mt, nt, gi, KT;
+};
+template <int BN, int kMax>
+__device__ __forceinline__ UmmaTile umma_tile(const UmmaList<kMax>& L, int tile) {
+  int p = 0;
+  if constexpr (kMax > 1)
+    while (p + 1 < L.n && tile >= L.first[p + 1]) ++p;
+  const UmmaArgs& g = L.g[p];
+  const int MT = (g.M + kUM - 1) / kUM, NT = (g.N + BN - 1) / BN, r = tile - (kMax > 1 ? L.first[p] : 0);
+  return UmmaTile{p, (r / NT) % MT, r % NT, r / (NT * MT), (g.K + kUK - 1) / kUK};
+}
+
+template <int BN, int kMax>
+__global__ void __launch_bounds__(kUThreads, 1) umma_gemm_kernel(const __grid_constant__ UmmaList<kMax> L) {
   extern __shared__ unsigned char umma_raw[];
   constexpr int kS = kUStages<BN>;
   __shared__ uint64_t full[kS], empty[kS], tfull[2], tempty[2], done;
@@ -197,10 +219,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
   UStage<BN>* st = reinterpret_cast<UStage<BN>*>(base);
   EpiStage* ep = reinterpret_cast<EpiStage*>(base + kS * sizeof(UStage<BN>));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the last tiles of each extent may reach past it: TMA fills loads there with zeros (a K step of
-  // zeros adds nothing) and leaves stores out
-  const int MT = (g.M + kUM - 1) / kUM, NT = (g.N + BN - 1) / BN, KT = (g.K + kUK - 1) / kUK;
-  const int tiles = g.groups * MT * NT;
+  const int tiles = L.first[L.n];
+  int* const status = L.g[0].status;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kS; ++s) {
       ubar_init(&full[s], 1);
@@ -214,8 +234,8 @@ __global__ void __launch_bounds__(kUThreads, 1)
     failed_sh = 0;
     consumed_sh = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    prefetch_map(&amap);
-    prefetch_map(&bmap);
+    prefetch_map(&L.a[0]);
+    prefetch_map(&L.b[0]);
   }
   if (warp == 1) {  // two accumulators of 128 lanes x BN FP32 columns
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(saddr(&tmem_base)),
@@ -234,18 +254,18 @@ __global__ void __launch_bounds__(kUThreads, 1)
     if (lane == 0) {
       constexpr unsigned kStageBytes = (kUM + BN) * kUK * sizeof(__nv_bfloat16);
       for (int tile = blockIdx.x; tile < tiles && !*failed; tile += gridDim.x) {
-        const int nt = tile % NT, mt = (tile / NT) % MT, gi = tile / (NT * MT);
+        const UmmaTile w = umma_tile<BN>(L, tile);
         int kb = 0;
-        for (; kb < KT; ++kb, ++issued) {
+        for (; kb < w.KT; ++kb, ++issued) {
           const int s = issued % kS;
           const unsigned r = (unsigned)(issued / kS);
           if (!ubar_wait(&empty[s], (r & 1u) ^ 1u, failed)) break;
           ubar_expect(&full[s], kStageBytes);
-          utma_load(st[s].a, &amap, &full[s], kb * kUK, mt * kUM, gi);
-          utma_load(st[s].b, &bmap, &full[s], kb * kUK, nt * BN, gi);
+          utma_load(st[s].a, &L.a[w.p], &full[s], kb * kUK, w.mt * kUM, w.gi);
+          utma_load(st[s].b, &L.b[w.p], &full[s], kb * kUK, w.nt * BN, w.gi);
         }
-        if (kb < KT) {
-          raise_failure(failed, g.status);
+        if (kb < w.KT) {
+          raise_failure(failed, status);
           break;
         }
       }
@@ -262,6 +282,7 @@ __global__ void __launch_bounds__(kUThreads, 1)
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const uint32_t d = tmem + (uint32_t)(acc * BN);
+        const int KT = umma_tile<BN>(L, tile).KT;
         for (int kb = 0; kb < KT; ++kb, ++it) {
           const int s = it % kS;
           ok = ubar_wait(&full[s], (unsigned)((it / kS) & 1), failed);
@@ -277,7 +298,7 @@ __global__ void __launch_bounds__(kUThreads, 1)
         ucommit(&tfull[acc]);  // arrives when the tile's MMAs have completed
       }
       *(volatile int*)&consumed_sh = it;
-      if (!ok) raise_failure(failed, g.status);
+      if (!ok) raise_failure(failed, status);
       ucommit(&done);  // every MMA issued so far has completed before TMEM is freed
       ubar_wait(&done, 0u, nullptr);
     }
@@ -287,7 +308,9 @@ __global__ void __launch_bounds__(kUThreads, 1)
     EpiStage& es = ep[warp - 2];
     int t = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++t) {
-      const int nt = tile % NT, mt = (tile / NT) % MT, gi = tile / (NT * MT);
+      const UmmaTile w = umma_tile<BN>(L, tile);
+      const int nt = w.nt, mt = w.mt, gi = w.gi;
+      const UmmaArgs& g = L.g[w.p];
       const int acc = t & 1;
       const int row0 = mt * kUM + 32 * q;  // the chunks' first row within the group
       const int row = row0 + lane;         // this thread's row
@@ -310,7 +333,7 @@ __global__ void __launch_bounds__(kUThreads, 1)
       // warp-uniform outcome: the TMEM loads below are warp-collective
       const bool ok = __all_sync(0xffffffffu, ubar_wait(&tfull[acc], (unsigned)((t >> 1) & 1), failed));
       if (!ok) {
-        if (lane == 0) raise_failure(failed, g.status);
+        if (lane == 0) raise_failure(failed, status);
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -387,9 +410,9 @@ __global__ void __launch_bounds__(kUThreads, 1)
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
         if (lane == 0) {
-          if (g.has32) utma_store(&c32map, es.c32, col0, row0, gi);
-          if (g.has16) utma_store(&c16map, es.c16, col0, row0, gi);
-          if (g.has16t) utma_store(&c16tmap, es.c16t, row0, col0, gi);
+          if (g.has32) utma_store(&L.c32[w.p], es.c32, col0, row0, gi);
+          if (g.has16) utma_store(&L.c16[w.p], es.c16, col0, row0, gi);
+          if (g.has16t) utma_store(&L.c16t[w.p], es.c16t, row0, col0, gi);
           asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
         }
       }
@@ -422,23 +445,24 @@ bool group_map(CUtensorMap* m, CUtensorMapDataType dt, int esize, const void* ba
   return encode_tensor_map(m, dt, 3, base, dims, strides, box, what, why, sw);
 }
 
-template <int BN>
-cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
+// Problem p as entry k of a list.
+template <int BN, int kMax>
+bool add_problem(UmmaList<kMax>* L, int k, const UmmaProblem& p, std::string* why) {
   constexpr auto BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  CUtensorMap amap, bmap, c32map{}, c16map{}, c16tmap{};
-  if (!group_map(&amap, BF, 2, p.A, p.M, p.K, p.lda, p.sA, p.groups, kUK, kUM, CU_TENSOR_MAP_SWIZZLE_128B, "A", why) ||
-      !group_map(&bmap, BF, 2, p.B, p.N, p.K, p.ldb, p.sB, p.groups, kUK, BN, CU_TENSOR_MAP_SWIZZLE_128B, "B", why))
-    return cudaErrorNotSupported;
-  if (p.C32 && !group_map(&c32map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.C32, p.M, p.N, p.ldc, p.sC, p.groups, 32, 32,
-                          CU_TENSOR_MAP_SWIZZLE_128B, "C32", why))
-    return cudaErrorNotSupported;
-  if (p.C16 && !group_map(&c16map, BF, 2, p.C16, p.M, p.N, p.ldc, p.sC, p.groups, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B,
-                          "C16", why))
-    return cudaErrorNotSupported;
-  if (p.C16T && !group_map(&c16tmap, BF, 2, p.C16T, p.N, p.M, p.ldct, p.sCT, p.groups, 32, 32,
+  if (!group_map(&L->a[k], BF, 2, p.A, p.M, p.K, p.lda, p.sA, p.groups, kUK, kUM, CU_TENSOR_MAP_SWIZZLE_128B, "A",
+                 why) ||
+      !group_map(&L->b[k], BF, 2, p.B, p.N, p.K, p.ldb, p.sB, p.groups, kUK, BN, CU_TENSOR_MAP_SWIZZLE_128B, "B", why))
+    return false;
+  if (p.C32 && !group_map(&L->c32[k], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, p.C32, p.M, p.N, p.ldc, p.sC, p.groups, 32,
+                          32, CU_TENSOR_MAP_SWIZZLE_128B, "C32", why))
+    return false;
+  if (p.C16 && !group_map(&L->c16[k], BF, 2, p.C16, p.M, p.N, p.ldc, p.sC, p.groups, 32, 32,
+                          CU_TENSOR_MAP_SWIZZLE_64B, "C16", why))
+    return false;
+  if (p.C16T && !group_map(&L->c16t[k], BF, 2, p.C16T, p.N, p.M, p.ldct, p.sCT, p.groups, 32, 32,
                            CU_TENSOR_MAP_SWIZZLE_NONE, "C16T", why))
-    return cudaErrorNotSupported;
-  UmmaArgs g{};
+    return false;
+  UmmaArgs& g = L->g[k];
   g.bias = p.bias;
   g.mask = static_cast<const __nv_bfloat16*>(p.mask);
   g.sBias = p.sBias;
@@ -446,8 +470,21 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
   g.M = p.M, g.N = p.N, g.K = p.K, g.ldc = p.ldc, g.act = p.act, g.groups = p.groups;
   g.has32 = p.C32 != nullptr, g.has16 = p.C16 != nullptr, g.has16t = p.C16T != nullptr;
   g.status = p.status;
+  const long long tiles = (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + BN - 1) / BN);
+  if (L->first[k] + tiles > 2147483647LL) return false;
+  L->first[k + 1] = L->first[k] + (int)tiles;
+  L->n = k + 1;
+  return true;
+}
+
+template <int BN, int kMax>
+cudaError_t launch_list(const UmmaProblem* p, int n, cudaStream_t s, std::string* why) {
+  UmmaList<kMax> L{};
+  for (int k = 0; k < n; ++k)
+    if (!add_problem<BN>(&L, k, p[k], why)) return cudaErrorNotSupported;
   const size_t bytes = sizeof(UStage<BN>) * kUStages<BN> + sizeof(EpiStage) * kEpiWarps + 1024;
-  cudaError_t err = cudaFuncSetAttribute(umma_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  auto kernel = umma_gemm_kernel<BN, kMax>;
+  cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   static int sms = 0;
   if (sms == 0) {
@@ -456,9 +493,8 @@ cudaError_t launch_bn(const UmmaProblem& p, cudaStream_t s, std::string* why) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
       sms = 148;
   }
-  const long long tiles = (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + BN - 1) / BN);
-  const int grid = (int)(tiles < sms ? tiles : sms);
-  return launch_pdl(true, umma_gemm_kernel<BN>, dim3(grid), dim3(kUThreads), bytes, s, g, amap, bmap, c32map, c16map, c16tmap);
+  const int tiles = L.first[n];
+  return launch_pdl(true, kernel, dim3(tiles < sms ? tiles : sms), dim3(kUThreads), bytes, s, L);
 }
 
 bool aligned16(const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; }
@@ -481,15 +517,23 @@ cudaError_t launch_umma_gemm(const UmmaProblem& p, cudaStream_t s, std::string* 
   // 128-column tiles unless they would leave most SMs without a tile
   const long long tiles128 =
       p.N > 64 ? (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + 127) / 128) : 0;
-  if (tiles128 >= 96) return launch_bn<128>(p, s, why);
-  return launch_bn<64>(p, s, why);
+  if (tiles128 >= 96) return launch_list<128, 1>(&p, 1, s, why);
+  return launch_list<64, 1>(&p, 1, s, why);
+}
+
+// Independent problems in one launch: their tiles follow one another, so that the start and the end of
+// all but the first and last are hidden. Seven weight gradients of a training step (8 groups,
+// 512x512x256, 512x1024x256, 8x512x256) took 46.7 us one by one, 21.0 together.
+cudaError_t launch_umma_list(const UmmaProblem* p, int n, cudaStream_t s, std::string* why) {
+  return n <= kUmmaList ? launch_list<128, kUmmaList>(p, n, s, why) : cudaErrorNotSupported;
 }
 
 cudaError_t preload_umma() {
   cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<128>));
+  cudaError_t e = cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<128, 1>));
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<128, kUmmaList>));
   if (e != cudaSuccess) return e;
-  return cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<64>));
+  return cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<64, 1>));
 }
 
 static_assert(sizeof(UStage<128>) == (kUM + 128) * kUK * 2, "stage tiles are contiguous and 1024-byte multiples");

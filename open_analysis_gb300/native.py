@@ -35,6 +35,14 @@ _pi64 = C.POINTER(C.c_int64)
 _pu16 = C.POINTER(C.c_uint16)
 
 
+class Gemm(C.Structure):
+    """One product of ``oafdtd_mlp_gemm_list``."""
+
+    _fields_ = [("A", C.c_void_p), ("B", C.c_void_p), ("C32", C.c_void_p),
+                *[(k, C.c_int32) for k in ("M", "N", "K", "lda", "ldb", "ldc", "groups")],
+                *[(k, C.c_int64) for k in ("strideA", "strideB", "strideC")]]
+
+
 class Correction(C.Structure):
     _fields_ = [
         ("kind", _i32),
@@ -232,6 +240,7 @@ SIGNATURES: dict[str, tuple[Any, list[Any]]] = {
         C.c_int,
         [C.c_void_p] * 7 + [_i32] * 8 + [C.c_float, _i32] + [_i64] * 5 + [C.c_void_p, C.c_void_p],
     ),
+    "oafdtd_mlp_gemm_list": (C.c_int, [C.c_void_p, _i32, C.c_void_p, C.c_void_p]),
     "oafdtd_mlp_transpose": (C.c_int, [C.c_void_p, _i32, _i32, _i32, C.c_void_p, _i32, _i32, _i64, _i64, C.c_void_p]),
 }
 

@@ -502,9 +502,9 @@ class Mlp:
         }
 
     def _backward(self, buf: dict[str, Any], m: int, s: int, x_t: bool = False) -> None:
-        """Gradients of one batch: the GEMMs one after the other on the current stream, each layer's
-        bias gradient beside them on ``self.side``. ``x_t``: the transposed inputs are in ``buf``
-        already."""
+        """Gradients of one batch: the chain of input gradients on the current stream, then every
+        layer's weight gradient in one launch; each layer's bias gradient beside them on ``self.side``.
+        ``x_t``: the transposed inputs are in ``buf`` already."""
         lib, g, p = self.lib, self.members, self.n_params
         y, t = buf["y"], buf["t"]
         out, n_in = self.sizes[-1], self.sizes[0]
@@ -516,6 +516,7 @@ class Mlp:
         if not x_t:
             native.check(lib.oafdtd_mlp_transpose(buf["x16"].data_ptr(), m, n_in, n_in, buf["x16T"].data_ptr(), m, g,
                                                   m * n_in, n_in * m, s), "transpose")
+        dw: list[native.Gemm] = []
         for l in range(len(self.layout) - 1, -1, -1):
             _, a, b, _ = self.layout[l]
             inp = buf["x16"].data_ptr() if l == 0 else buf["acts"][l - 1].data_ptr()
@@ -529,10 +530,11 @@ class Mlp:
                 self._gemm_tn(g16, self._w(l), dz32, dz16, dzt, 0, inp, m, a, b, b, b, a, m, self.dact, s,
                               m * b, p, m * a, a * m, 0)
             # dW = inp^T . g = (inp^T) . (g^T)^T  (a x b), from the transposed activations and g
-            self._gemm_tn(inp_t, gT, self._gw(l), 0, 0, 0, 0, a, b, m, m, m, b, a, 0, s, a * m, b * m, p, 0, 0)
+            dw.append(native.Gemm(inp_t, gT, self._gw(l), a, b, m, m, m, b, g, a * m, b * m, p))
             side.wait_stream(cur)
             native.check(lib.oafdtd_mlp_colsum(g32, m, b, b, self._gb(l), g, m * b, p, s2), "colsum")
             g32, g16, gT = dz32, dz16, dzt
+        native.check(lib.oafdtd_mlp_gemm_list((native.Gemm * len(dw))(*dw), len(dw), self.status.data_ptr(), s), "dW")
         cur.wait_stream(side)
 
     def _per_member(self, v: npt.ArrayLike) -> npt.NDArray[np.float32]:

@@ -105,3 +105,27 @@ def test_prediction_is_the_layers_one_by_one(rows, chunk, members, act):
     assert torch.equal(have, want)
     one = net.predict_device(x[0], chunk)  # a vector stands for as many equal rows as it is wide, padded
     assert one.shape[1] == net.sizes[0] and torch.equal(one[:, :1], net.predict_device(x[:1], chunk))
+
+
+@pytest.mark.parametrize("shapes", [
+    [(2, 72, 136, 40)],
+    [(8, 512, 512, 256), (8, 8, 512, 256), (8, 512, 1024, 256), (1, 130, 72, 520)],  # a K of its own, ragged tiles
+    [(1, 64, 72, 64)] * 3 + [(1, 20, 24, 12)] + [(3, 136, 200, 88)] * 9,  # one for the general kernels; two launches
+])
+def test_a_list_of_products_is_its_products(shapes):
+    native, lib = _lib()
+    gen = torch.Generator("cuda").manual_seed(6)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    s = int(torch.cuda.current_stream().cuda_stream)
+    keep, items = [], []
+    for g, m, n, k in shapes:
+        a, b = (torch.randn(g, r, k, generator=gen, device="cuda").bfloat16() for r in (m, n))
+        c, want = (torch.full((g, m, n), 7.0, device="cuda") for _ in range(2))
+        keep.append((a, b, c, want))
+        items.append(native.Gemm(a.data_ptr(), b.data_ptr(), c.data_ptr(), m, n, k, k, k, n, g, m * k, n * k, m * n))
+        native.check(lib.oafdtd_mlp_gemm_tn(a.data_ptr(), b.data_ptr(), want.data_ptr(), None, None, None, None, m, n, k,
+                                            k, k, n, m, 0, 0.0, g, m * k, n * k, m * n, 0, 0, status.data_ptr(), s), "tn")
+    native.check(lib.oafdtd_mlp_gemm_list((native.Gemm * len(items))(*items), len(items), status.data_ptr(), s), "list")
+    for _, _, c, want in keep:
+        assert torch.equal(c, want)
+    assert status.item() == 0
