@@ -253,8 +253,8 @@ struct SlabLaunch {
   int n;
   int first[7];  // first block of each box; first[n] = total blocks
   int planes;       // planes marched per thread
+  FastDiv nb;       // members
   FastDiv cblk[6];  // column blocks per (box, chunk, member)
-  FastDiv nch[6];   // z chunks per box
   FastDiv nv[6];    // vector columns per row
   Span3 core;    // holds no correction cell (quads, rows, planes)
   int extra;     // leading blocks that sample probes (variant 0)

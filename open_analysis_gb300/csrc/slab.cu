@@ -108,10 +108,17 @@ __device__ __forceinline__ SlabWork slab_work(const SlabLaunch& L, int nx, int b
   while (s + 1 < L.n && blk >= L.first[s + 1]) ++s;
   const Span3 bx = L.box[s];
   const int r = blk - L.first[s];
-  const int t = fast_div(L.cblk[s], r), cb = r - t * L.cblk[s].d;
+  // Member fastest: the members of a column block run side by side and read its indices, metrics and
+  // CPML coefficients from memory once (120x60x40, two members: 21.5 to 20.0 us a step; the slabs' E of
+  // 397x323x160, eight members: 503 to 476 us).
   SlabWork w;
-  w.b = fast_div(L.nch[s], t);
-  const int ch = t - w.b * L.nch[s].d;
+  int t = r;
+  w.b = 0;
+  if (L.nb.d != 1) {
+    t = fast_div(L.nb, r);
+    w.b = r - t * L.nb.d;
+  }
+  const int ch = fast_div(L.cblk[s], t), cb = t - ch * L.cblk[s].d;
   const int c = cb * kSlabCols + (int)threadIdx.x;
   const int row = fast_div(L.nv[s], c);
   w.j = bx.j0 + row;
@@ -675,14 +682,14 @@ cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long lo
     const long long cblk = (cols + kSlabCols - 1) / kSlabCols;
     const int nch = (bx.k1 - bx.k0 + L->planes - 1) / L->planes;
     const long long blocks_here = cblk * nch * a.B;
-    L->cblk[L->n] = fast_divisor(cblk, blocks_here);
-    L->nch[L->n] = fast_divisor(nch, (long long)nch * a.B);
+    L->cblk[L->n] = fast_divisor(cblk, cblk * nch);
     L->nv[L->n] = fast_divisor((bx.q1 - bx.q0) * kPerQuad, cblk * kSlabCols);
     total += blocks_here;
     ++L->n;
   }
   if (total > 2147483647LL) return cudaErrorInvalidConfiguration;
   L->first[L->n] = (int)total;
+  L->nb = fast_divisor(a.B, total);
   *blocks = total;
   return cudaSuccess;
 }
