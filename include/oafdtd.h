@@ -244,7 +244,8 @@ int oafdtd_peak_bytes(const oafdtd_engine* engine, int64_t* out);
  * and replay it (the reference's use_graph flag, engine.py:80,425-429). */
 int oafdtd_set_graph(oafdtd_engine* engine, int32_t use_graph);
 
-/* Launch shape of the sweeps: z planes marched per block (tile_z, 0 keeps the current value) and
+/* Launch shape of the sweeps: z planes marched per block (tile_z, 0 keeps the current value; at first
+ * 16, in the fused variant 32 or all where the blocks are enough) and
  * the sweep variant (3: the fused sweep, which updates H and E of the interior in one z-march and
  * runs the rest as variant 2; it keeps two buffers per field, reading the current ones and writing
  * the others, and is the default of float32 grids above 16 million cells times members where the

@@ -40,9 +40,9 @@ int fail(int code, const std::string& msg) {
   } while (0)
 
 // Cells times members up to which the direct sweeps are the default in float32. us per step, direct
-// against the best fused shape (via transition, batch 2): 4.8 million 164 / 227, 9.6 million 268 /
-// 351, 10.8 million 320 / 378, 19.2 million 474 / 463, 27.2 million 638 / 622, 51.2 million 1139 /
-// 1055. Small fields stay in the 129 MB L2, where the fused sweep saves little, and its march over
+// against the best fused shape (via transition, batch 2): 4.8 million 146 / 191, 9.6 million 267 /
+// 341, 10.8 million 293 / 326, 19.2 million 470 / 449, 27.3 million 650 / 661, 38.4 million 889 /
+// 820. Small fields stay in the 129 MB L2, where the fused sweep saves little, and its march over
 // the planes of a tile is a long serial chain on few blocks; large ones are bound by the memory
 // traffic it saves. In float64 the two float64 operations a clock and SM bound every variant, and the
 // fused sweep computes its tiles' halos twice: 853 against 1406 us at 161 x 143 x 88.
@@ -1271,8 +1271,20 @@ int Engine<real>::build(const oafdtd_problem& p) {
   } else if (fused_ok && staged == 2) {
     size_t free_b = 0, total_b = 0;
     OA_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if ((double)free_b > 1.05 * 6.0 * (double)bs * B * sizeof(real))
+    if ((double)free_b > 1.05 * 6.0 * (double)bs * B * sizeof(real)) {
       if (int rc = set_variant(3)) return rc;
+      // Planes per block of the fused sweep, two blocks to an SM. Tiles that nearly fill the chip
+      // once march all planes; several rounds of blocks take 32, fewer tiles 16. us per step with
+      // 16 / 32 / all: 288 tiles (400x400x120, two members) 844 / 833 / 820; 912 tiles (397x323x160,
+      // eight) 3058 / 3040 / 3111; 560 tiles 897 / 887 / 881; 240 tiles 662 / 670 / 661; 174 tiles
+      // 500 / 505 / 518.
+      int sms = 0;
+      OA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+      const oafdtd::Span3& F = fused_box;
+      const long long tiles = (long long)((F.q1 - F.q0 + 31) / 32) * ((F.j1 - F.j0 + 7) / 8) * B, slots = 2LL * sms;
+      if (tiles > slots) tile_z = 32;
+      else if (10 * tiles >= 9 * slots) tile_z = F.k1 - F.k0;
+    }
   }
   OA_CUDA(cudaStreamSynchronize(stream));
   timer.mark("device_sync");
