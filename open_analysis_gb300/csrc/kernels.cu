@@ -220,21 +220,33 @@ __global__ void __launch_bounds__(256) probe_e_batch_kernel(const ProbeArgs<real
 
 // ----------------------------------------------------------------------------- surface impedance
 // E_face = r0 J + sum_p v_p, v_p = alpha_p (J - J_prev) + g_p v_p, J = sum of the signed outside
-// H samples (reference.py:129-150). One thread per edge handles every batch member; BB and PP
+// H samples (reference.py:129-150). A thread handles the batch members of an edge (kSibcMembers); BB and PP
 // unroll the batch and pole loops so all loads of an edge are issued together.
+// Members of one edge that a thread takes, of BB in all: all of them in float32 (one per thread 146 us
+// against 123 for 1.9 million edges, two members); one in float64, where two take 190 registers and
+// four 254 with spills (84 against 92 us for 0.27 million edges, two members).
+template <typename real, int BB>
+constexpr int kSibcMembers = sizeof(real) == 4 ? BB : (BB < 1 ? BB : 1);
+
 template <typename real, int BB, int PP>
 __device__ __forceinline__ void sibc_body(const SibcArgs<real>& a, int block, int lo, int hi) {
+  constexpr int N = kSibcMembers<real, BB>;
+  int b0 = 0;
+  if constexpr (N < BB) {  // the members of an edge in blocks side by side
+    b0 = block % BB;
+    block /= BB;
+  }
   const int s = lo + block * (int)blockDim.x + (int)threadIdx.x;
   if (s >= hi) return;
   const SibcEdge<real> ed = a.edge[s];
   const real* __restrict__ alpha = a.alpha + (long long)ed.mat * PP;
   const long long n = a.n;
   // every load of this edge first (the stores below would otherwise order them one by one)
-  real vv[BB][PP], hs[BB][2], jp[BB];
+  real vv[N][PP], hs[N][2], jp[N];
 #pragma unroll
-  for (int b = 0; b < BB; ++b) {
-    const long long off = (long long)b * a.bs;
-    const long long be = (long long)b * n + s;
+  for (int b = 0; b < N; ++b) {
+    const long long off = (long long)(b0 + b) * a.bs;
+    const long long be = (long long)(b0 + b) * n + s;
     hs[b][0] = ed.sign[0] != (real)0 ? a.H[ed.hcomp0][off + ed.hflat[0]] : (real)0;
     hs[b][1] = ed.sign[1] != (real)0 ? a.H[ed.hcomp1][off + ed.hflat[1]] : (real)0;
     jp[b] = a.jprev[be];
@@ -243,7 +255,7 @@ __device__ __forceinline__ void sibc_body(const SibcArgs<real>& a, int block, in
   }
   const real r0 = a.r0[ed.mat];
 #pragma unroll
-  for (int b = 0; b < BB; ++b) {
+  for (int b = 0; b < N; ++b) {
     real jj = (real)0;
     if (ed.sign[0] != (real)0) jj = jj + ed.sign[0] * hs[b][0];
     if (ed.sign[1] != (real)0) jj = jj + ed.sign[1] * hs[b][1];
@@ -255,11 +267,11 @@ __device__ __forceinline__ void sibc_body(const SibcArgs<real>& a, int block, in
       vv[b][p] = nv;
       vsum = p == 0 ? nv : vsum + nv;
     }
-    const long long be = (long long)b * n + s;
+    const long long be = (long long)(b0 + b) * n + s;
 #pragma unroll
     for (int p = 0; p < PP; ++p) a.v[((long long)p * BB) * n + be] = vv[b][p];
     a.jprev[be] = jj;
-    a.E[ed.comp][(long long)b * a.bs + ed.flat] = r0 * jj + vsum;
+    a.E[ed.comp][(long long)(b0 + b) * a.bs + ed.flat] = r0 * jj + vsum;
   }
 }
 
@@ -322,9 +334,16 @@ int sibc_variant(const SibcArgs<real>& a) {
   return a.P == 16 && (a.B == 1 || a.B == 2 || a.B == 4) ? a.B : 0;
 }
 
+// Blocks of 128 threads for n edges.
+template <typename real>
+int sibc_blocks_of(const SibcArgs<real>& a, int n) {
+  const int split = sizeof(real) == 8 ? std::max(sibc_variant(a), 1) : 1;  // BB / kSibcMembers
+  return (n + 127) / 128 * split;
+}
+
 template <typename real>
 int sibc_blocks(const SibcArgs<real>& a) {
-  return (int)((a.n + 127) / 128);
+  return sibc_blocks_of(a, a.n);
 }
 
 template <typename real>
@@ -347,7 +366,7 @@ cudaError_t launch_sibc(const SibcArgs<real>& a, cudaStream_t s, int lo, int hi,
                 : variant == 1 ? sibc_kernel<real, 1, 16>
                 : variant == 4 ? sibc_kernel<real, 4, 16>
                                : sibc_generic_kernel<real>;
-  return launch_pdl(pdl, kernel, dim3((unsigned)((hi - lo + 127) / 128)), dim3(128), 0, s, a, lo, hi);
+  return launch_pdl(pdl, kernel, dim3((unsigned)sibc_blocks_of(a, hi - lo)), dim3(128), 0, s, a, lo, hi);
 }
 
 // ----------------------------------------------------------------------------- injection pass
