@@ -86,9 +86,14 @@ __global__ void __launch_bounds__(256) ghost_kernel(const __grid_constant__ Ghos
 // (probe, member, frequency) for the sums.
 constexpr int kDftF = 4;
 
+// Blocks per kind: one also without frequencies, for the tail samples.
+template <typename real>
+__host__ __device__ __forceinline__ int dft_blocks_per_kind(const ProbeArgs<real>& a) {
+  return a.n_freq > kDftF ? (a.n_freq + kDftF - 1) / kDftF : 1;
+}
 template <typename real>
 __host__ __device__ __forceinline__ int dft_blocks_of(const ProbeArgs<real>& a) {
-  return a.n_probe > 0 && a.n_freq > 0 ? 2 * ((a.n_freq + kDftF - 1) / kDftF) : 1;
+  return a.n_probe > 0 ? 2 * dft_blocks_per_kind(a) : 1;
 }
 
 // Steps base .. base + n - 1 of the probes of the kinds in `kinds` (bit 0 E, bit 1 H). tail: the last
@@ -98,10 +103,10 @@ __device__ __forceinline__ void dft_body(const ProbeArgs<real>& a, int block, in
   __shared__ double2 ph[kDftF][kChunk];
   __shared__ double tails[kChunk];
   const long long base = *a.step_base;
-  const int nfb = (a.n_freq + kDftF - 1) / kDftF;
-  const int kind = nfb > 0 ? block / nfb : 0, f0 = nfb > 0 ? (block % nfb) * kDftF : 0;
-  const int pairs = kind < 2 && ((kinds >> kind) & 1) ? a.n_kind[kind] * a.B : 0;
-  if (pairs > 0 && a.n_freq > 0) {
+  const int nfb = dft_blocks_per_kind(a);
+  const int kind = block / nfb, f0 = (block % nfb) * kDftF;
+  const int pairs = (kinds >> kind) & 1 ? a.n_kind[kind] * a.B : 0;
+  if (pairs > 0) {
     const int fi = threadIdx.x / kChunk, o = threadIdx.x % kChunk;
     if (o < n && f0 + fi < a.n_freq) {
       const double t = ((double)(base + o) + (kind == 0 ? 1.0 : 0.5)) * a.dt;
