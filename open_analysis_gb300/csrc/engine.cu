@@ -2022,7 +2022,7 @@ struct Batch final : BatchBase {
     const std::vector<oafdtd::SweepArgs<real>>& a = h_sw[0];
     std::vector<dim3> g_fused(n), g_hi(n), g_hz(n), g_ei(n), g_ez(n), g_sh(n), g_se(n), g_pre(n), g_probe(n),
         g_edge(n), g_sibc(n), g_dft(n);
-    std::vector<int> k_pole(n), k_zero(n, 0), k_sibc(n);
+    std::vector<int> k_pole(n), k_zero(n, 0), k_sibc(n), k_slab[2] = {std::vector<int>(n), std::vector<int>(n)};
     std::vector<oafdtd::SlabLaunch> slabs[2];
     slabs[0].resize(n);
     slabs[1].resize(n);
@@ -2066,14 +2066,16 @@ struct Batch final : BatchBase {
       g_sibc[i] = dim3((unsigned)oafdtd::sibc_blocks(e.sb), 1, 1);
       g_dft[i] = dim3((unsigned)oafdtd::dft_blocks(e.pr), 1, 1);
       k_pole[i] = a[i].ade_P > 1 ? 1 : 0;
+      k_slab[0][i] = k_pole[i] + 2 * oafdtd::slab_thin(a[i], 0);  // bit 0 several poles, bit 1 thin
+      k_slab[1][i] = 2 * oafdtd::slab_thin(a[i], 1);
       k_sibc[i] = oafdtd::sibc_variant(e.sb);
     }
     for (int kind = 0; kind < 2; ++kind)
       if (int rc = upload(&d_slab[kind], slabs[kind].data(), n)) return rc;
     const std::pair<std::vector<dim3>*, std::pair<std::vector<int>*, std::vector<Launch>*>> plans[] = {
         {&g_fused, {&k_pole, &fused}},  {&g_hi, {&k_zero, &h_inner}}, {&g_hz, {&k_zero, &h_z}},
-        {&g_ei, {&k_pole, &e_inner}},   {&g_ez, {&k_pole, &e_z}},     {&g_sh, {&k_zero, &slab_h}},
-        {&g_se, {&k_pole, &slab_e}},    {&g_pre, {&k_zero, &pre_e}},  {&g_probe, {&k_zero, &probe_e}},
+        {&g_ei, {&k_pole, &e_inner}},   {&g_ez, {&k_pole, &e_z}},     {&g_sh, {&k_slab[1], &slab_h}},
+        {&g_se, {&k_slab[0], &slab_e}},    {&g_pre, {&k_zero, &pre_e}},  {&g_probe, {&k_zero, &probe_e}},
         {&g_edge, {&k_zero, &edges}},   {&g_sibc, {&k_sibc, &sibc}},
         {&g_dft, {&k_zero, &dft}},
     };
@@ -2093,7 +2095,8 @@ struct Batch final : BatchBase {
   int slab_launches(int kind, int p, int off, cudaStream_t s) {
     for (const Launch& L : kind == 0 ? slab_e : slab_h) {
       const cudaError_t err = oafdtd::launch_slab_batch<real>(d_sw[p], d_slab[kind], d_ed[p], d_pr[p], L.g, L.blocks,
-                                                              kind, L.key != 0, off, variant == 0, s);
+                                                              kind, (L.key & 1) != 0, (L.key & 2) != 0, off,
+                                                              variant == 0, s);
       if (err != cudaSuccess) return fail(OAFDTD_E_CUDA, std::string("batched slab: ") + cudaGetErrorString(err));
     }
     return OAFDTD_OK;

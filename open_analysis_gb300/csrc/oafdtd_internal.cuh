@@ -332,6 +332,9 @@ cudaError_t slab_plan(const SweepArgs<real>& a, int kind, SlabLaunch* L, long lo
 template <typename real>
 long long slab_vecs(const SweepArgs<real>& a, int kind);
 int slab_planes(long long vecs);
+// Whether one kind's sweep needs the kernels for x slabs that share a vector of cells.
+template <typename real>
+bool slab_thin(const SweepArgs<real>& a, int kind);
 template <typename real>
 int pre_e_blocks(const ProbeArgs<real>& a);
 template <typename real>
@@ -352,7 +355,7 @@ cudaError_t launch_staged_batch(const SweepArgs<real>* A, const SweepMaps* M, co
 template <typename real>
 cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
                               const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
-                              int off, bool pdl, cudaStream_t s);
+                              bool thin, int off, bool pdl, cudaStream_t s);
 template <typename real>
 cudaError_t launch_pre_e_batch(const ProbeArgs<real>* A, const BatchGrid& G, int blocks, int off, cudaStream_t s);
 template <typename real>

@@ -146,9 +146,11 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // One correction term of a component (AX: its derivative axis) on a thread's column, worked out once
 // for the march: psi of the march's first plane is at p, of the next a stride further on; `mask` holds
 // the vector's cells inside the box (low bits) and, from bit 8, the march's planes inside it (0: no
-// slab of this term holds the column). A march meets at most one side of an axis (slab_plan sees to
-// it in z). y and z slabs keep psi rows at the field pitch, so their vectors are whole 16 bytes
-// (elements outside the box are written back unchanged); x slabs are read per element.
+// slab of this term holds the column). A march meets at most one side of an axis in y, and in z
+// (slab_plan sees to it); in x, where the two slabs of a very thin grid can share a vector, the kernels
+// of such grids (kThin) keep a second column. y and z slabs keep psi rows at the field pitch, so their
+// vectors are whole 16 bytes (elements outside the box are written back unchanged); x slabs are read
+// per element.
 template <typename real>
 struct PsiCol {
   real* p;
@@ -156,16 +158,17 @@ struct PsiCol {
   unsigned mask;
 };
 
+// The first side from `from` on that holds the column; returns the one after it.
 template <typename real, int AX>
-__device__ __forceinline__ void psi_column(const CpmlTerm<real>& T, PsiCol<real>& c, const SlabWork& w, int X, int Y,
-                                           int Z) {
+__device__ __forceinline__ int psi_column(const CpmlTerm<real>& T, PsiCol<real>& c, const SlabWork& w, int X, int Y,
+                                          int Z, int from = 0) {
   constexpr int V = kVec<real>;
   c.mask = 0;
   c.p = nullptr;
   c.stride = 0;
-  if (w.core) return;
+  if (w.core) return 2;
 #pragma unroll 1
-  for (int sd = 0; sd < 2; ++sd) {
+  for (int sd = from; sd < 2; ++sd) {
     const CpmlSide<real>& s = T.side[sd];
     if (s.psi == nullptr || w.i0 + V <= s.lo[0] || w.i0 >= s.hi[0] || w.j < s.lo[1] || w.j >= s.hi[1] ||
         w.k1 <= s.lo[2] || w.k0 >= s.hi[2])
@@ -178,8 +181,9 @@ __device__ __forceinline__ void psi_column(const CpmlTerm<real>& T, PsiCol<real>
     const int lo = max(s.lo[0] - w.i0, 0), hi = min(s.hi[0] - w.i0, V);
     const int klo = max(s.lo[2] - w.k0, 0), khi = min(s.hi[2], w.k1) - w.k0;
     c.mask = (((1u << hi) - 1u) & ~((1u << lo) - 1u)) | ((((1u << khi) - 1u) & ~((1u << klo) - 1u)) << 8);
-    return;
+    return sd + 1;
   }
+  return 2;
 }
 
 // psi of plane t of the march (false: the plane has none of this term); the march moves p on by the
@@ -304,8 +308,8 @@ __device__ __forceinline__ void st_unlisted(real* p, const Vec<real>& v, const M
 // One E component on one vector column. Per plane every load first (H, E, indices, Debye current,
 // psi), then the arithmetic, then every store. C: 0 Ex (terms y +Hz, z -Hy), 1 Ey (z +Hx, x -Hz),
 // 2 Ez (x +Hy, y -Hx). kMulti: more than one Debye pole; the currents of each pole are then read
-// twice (the second time from the L1 cache).
-template <typename real, int C, bool kMulti>
+// twice (the second time from the L1 cache). kThin: a vector may lie in both x slabs (slab_thin).
+template <typename real, int C, bool kMulti, bool kThin>
 __device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inject, const SlabWork& w) {
   constexpr int V = kVec<real>;
   constexpr int A0 = C == 0 ? 1 : 0, A1 = C == 2 ? 1 : 2;  // the derivative axes, ascending
@@ -327,14 +331,15 @@ __device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inje
   if (C != 0) wx = ldv(a.idd[0] + i0);
   const real wy = a.idd[1][w.j];
   const unsigned vm = valid_cells<real>(i0, a.nx + 1);
-  PsiCol<real> c0, c1;
-  psi_column<real, A0>(a.ecorr[C][0], c0, w, X, Y, a.nz + 2);
+  PsiCol<real> c0, c1, c2{};  // c2: the other x slab
+  const int other = psi_column<real, A0>(a.ecorr[C][0], c0, w, X, Y, a.nz + 2);
+  if (kThin && A0 == 0) psi_column<real, A0>(a.ecorr[C][0], c2, w, X, Y, a.nz + 2, other);
   psi_column<real, A1>(a.ecorr[C][1], c1, w, X, Y, a.nz + 2);
   int q = (w.k0 * Y + w.j) * X + i0;  // offset within one member (below 2^31)
   Vec<real> below;                    // the z-derivative's source on the plane below, carried
   if (C != 2) below = ldv(s1 + (q - sz));
 #pragma unroll 1
-  for (int k = w.k0; k < w.k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride) {
+  for (int k = w.k0; k < w.k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride, c2.p += c2.stride) {
     // ---- loads
     Mats<real> m;
     ld_mat(mat + q, m);
@@ -346,10 +351,11 @@ __device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inje
     else if (i0 > 0) x0 = s0[q - 1];
     if (C == 2) n1 = ldv(s1 + (q - X));
     else n1 = below;
-    Vec<real> j4, p0, p1;
+    Vec<real> j4, p0, p1, p2;
     const bool debye = k >= jlo && k < jhi;
     if (!kMulti && debye) j4 = ldv(J + q);
     const bool on0 = psi_load<real, A0>(c0, p0, k - w.k0), on1 = psi_load<real, A1>(c1, p1, k - w.k0);
+    const bool on2 = kThin && A0 == 0 && psi_load<real, A0>(c2, p2, k - w.k0);
     const real w1 = C == 2 ? wy : a.idd[2][k];
     if (k + 1 < w.k1) {
       prefetch_l2(mat + (q + sz));
@@ -409,6 +415,7 @@ __device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inje
     // ---- corrections
     auto kf = [&](int e) { return coef(e).cb; };
     if (on0) psi_apply<real, A0>(c0, p0, a.pe[A0], a.ecorr[C][0].sign, f, d0, kf, w, k);
+    if (on2) psi_apply<real, A0>(c2, p2, a.pe[A0], a.ecorr[C][0].sign, f, d0, kf, w, k);
     if (on1) psi_apply<real, A1>(c1, p1, a.pe[A1], a.ecorr[C][1].sign, f, d1, kf, w, k);
     // ---- Debye
     if (dis) {
@@ -462,7 +469,7 @@ __device__ __forceinline__ void slab_e_march(const SweepArgs<real>& a, bool inje
 
 // The E boxes; the first L.extra blocks sample the H probes of the step instead (H is complete), the
 // next L.inject blocks take the edge list's edges.
-template <typename real, bool kMulti>
+template <typename real, bool kMulti, bool kThin>
 __device__ __forceinline__ void slab_e_body(const SweepArgs<real>& a, const SlabLaunch& L, const EdgeArgs<real>& ed,
                                             const ProbeArgs<real>& pr, int off, int block) {
   if (block < L.extra) {
@@ -481,20 +488,20 @@ __device__ __forceinline__ void slab_e_body(const SweepArgs<real>& a, const Slab
   pdl_wait();
   if (!w.live) return;
   const bool inject = L.inject > 0;
-  if (threadIdx.y == 0) slab_e_march<real, 0, kMulti>(a, inject, w);
-  else if (threadIdx.y == 1) slab_e_march<real, 1, kMulti>(a, inject, w);
-  else slab_e_march<real, 2, kMulti>(a, inject, w);
+  if (threadIdx.y == 0) slab_e_march<real, 0, kMulti, kThin>(a, inject, w);
+  else if (threadIdx.y == 1) slab_e_march<real, 1, kMulti, kThin>(a, inject, w);
+  else slab_e_march<real, 2, kMulti, kThin>(a, inject, w);
 }
 
-template <typename real, bool kMulti>
+template <typename real, bool kMulti, bool kThin>
 __global__ void __launch_bounds__(kSlabThreads, 4)
     slab_e_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L,
                   const __grid_constant__ EdgeArgs<real> ed, const __grid_constant__ ProbeArgs<real> pr, int off) {
-  slab_e_body<real, kMulti>(a, L, ed, pr, off, (int)blockIdx.x);
+  slab_e_body<real, kMulti, kThin>(a, L, ed, pr, off, (int)blockIdx.x);
 }
 
 // Several engines' E updates in one launch: engine e's arguments at A[e], L[e], ED[e] and PR[e].
-template <typename real, bool kMulti>
+template <typename real, bool kMulti, bool kThin>
 __global__ void __launch_bounds__(kSlabThreads, 4)
     slab_e_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L,
                         const EdgeArgs<real>* __restrict__ ED, const ProbeArgs<real>* __restrict__ PR, const BatchGrid G,
@@ -504,14 +511,14 @@ __global__ void __launch_bounds__(kSlabThreads, 4)
   int e;
   const uint3 bid = G.block(&e);
   const SlabLaunch& l = stage_args(L + e, launch);
-  slab_e_body<real, kMulti>(stage_args(A + e, args), l, ED[e], PR[e], off, (int)bid.x);
+  slab_e_body<real, kMulti, kThin>(stage_args(A + e, args), l, ED[e], PR[e], off, (int)bid.x);
 }
 
 // ------------------------------------------------------------------------------------- H
 // One H component on one vector column. C: 0 Hx (terms y -Ez, z +Ey), 1 Hy (z -Ex, x +Ez), 2 Hz
 // (x -Ey, y +Ex). The cells each updates: Hx i in 1..nx+1, j <= ny, k <= nz; Hy i <= nx, k <= nz; Hz
-// i <= nx, j <= ny.
-template <typename real, int C>
+// i <= nx, j <= ny. kThin as in slab_e_march.
+template <typename real, int C, bool kThin>
 __device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const SlabWork& w) {
   constexpr int V = kVec<real>;
   constexpr int A0 = C == 0 ? 1 : 0, A1 = C == 2 ? 1 : 2;  // the derivative axes, ascending
@@ -529,14 +536,15 @@ __device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const Sla
   const bool right = i0 + V < X;  // the x + 1 neighbour of the last element is in the row
   const unsigned vm = valid_cells<real>(i0, C == 0 ? a.nx + 1 : a.nx);
   const real dtmu = a.dtmu;
-  PsiCol<real> c0, c1;
-  psi_column<real, A0>(a.hcorr[C][0], c0, w, X, Y, a.nz + 2);
+  PsiCol<real> c0, c1, c2{};  // c2: the other x slab
+  const int other = psi_column<real, A0>(a.hcorr[C][0], c0, w, X, Y, a.nz + 2);
+  if (kThin && A0 == 0) psi_column<real, A0>(a.hcorr[C][0], c2, w, X, Y, a.nz + 2, other);
   psi_column<real, A1>(a.hcorr[C][1], c1, w, X, Y, a.nz + 2);
   int q = (w.k0 * Y + w.j) * X + i0;
   Vec<real> here;  // the z-derivative's source on this plane, carried from the last one's plane above
   if (C != 2) here = ldv(s1 + q);
 #pragma unroll 1
-  for (int k = w.k0; k < k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride) {
+  for (int k = w.k0; k < k1; ++k, q += sz, c0.p += c0.stride, c1.p += c1.stride, c2.p += c2.stride) {
     // ---- loads
     Vec<real> h = ldv(H + q);
     const Vec<real> u0 = ldv(s0 + q);
@@ -552,8 +560,9 @@ __device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const Sla
       n1 = ldv(s1 + (q + sz));
       here = n1;
     }
-    Vec<real> p0, p1;
+    Vec<real> p0, p1, p2;
     const bool on0 = psi_load<real, A0>(c0, p0, k - w.k0), on1 = psi_load<real, A1>(c1, p1, k - w.k0);
+    const bool on2 = kThin && A0 == 0 && psi_load<real, A0>(c2, p2, k - w.k0);
     const real w1 = C == 2 ? wy : a.ip[2][k];
     if (k + 1 < k1) {
       prefetch_l2(H + (q + sz));
@@ -573,24 +582,25 @@ __device__ __forceinline__ void slab_h_march(const SweepArgs<real>& a, const Sla
     }
     auto kf = [&](int) { return dtmu; };
     if (on0) psi_apply<real, A0>(c0, p0, a.ph[A0], a.hcorr[C][0].sign, h, d0, kf, w, k);
+    if (on2) psi_apply<real, A0>(c2, p2, a.ph[A0], a.hcorr[C][0].sign, h, d0, kf, w, k);
     if (on1) psi_apply<real, A1>(c1, p1, a.ph[A1], a.hcorr[C][1].sign, h, d1, kf, w, k);
     stv(Ho + q, h);
   }
 }
 
-template <typename real>
+template <typename real, bool kThin>
 __device__ __forceinline__ void slab_h_body(const SweepArgs<real>& a, const SlabLaunch& L, int block) {
   const SlabWork w = slab_work<real>(L, a.nx, block);
   pdl_wait();
   if (!w.live) return;
-  if (threadIdx.y == 0) slab_h_march<real, 0>(a, w);
-  else if (threadIdx.y == 1) slab_h_march<real, 1>(a, w);
-  else slab_h_march<real, 2>(a, w);
+  if (threadIdx.y == 0) slab_h_march<real, 0, kThin>(a, w);
+  else if (threadIdx.y == 1) slab_h_march<real, 1, kThin>(a, w);
+  else slab_h_march<real, 2, kThin>(a, w);
 }
 
 // The H boxes; the first L.extra blocks sample the E probes of the previous step instead (the H
 // update leaves E alone; off - 1 is that step).
-template <typename real>
+template <typename real, bool kThin>
 __global__ void __launch_bounds__(kSlabThreads, 4)
     slab_h_kernel(const __grid_constant__ SweepArgs<real> a, const __grid_constant__ SlabLaunch L,
                   const __grid_constant__ ProbeArgs<real> pr, int off) {
@@ -599,12 +609,12 @@ __global__ void __launch_bounds__(kSlabThreads, 4)
     probe_sample(pr, 0, (int)blockIdx.x, off - 1);
     return;
   }
-  slab_h_body<real>(a, L, (int)blockIdx.x - L.extra);
+  slab_h_body<real, kThin>(a, L, (int)blockIdx.x - L.extra);
 }
 
 // Several engines' H updates in one launch. The E probes of a step before the first of a group
 // (off 0) are already in: those blocks return.
-template <typename real>
+template <typename real, bool kThin>
 __global__ void __launch_bounds__(kSlabThreads, 4)
     slab_h_batch_kernel(const SweepArgs<real>* __restrict__ A, const SlabLaunch* __restrict__ L,
                         const ProbeArgs<real>* __restrict__ PR, const BatchGrid G, int off) {
@@ -618,7 +628,7 @@ __global__ void __launch_bounds__(kSlabThreads, 4)
     if (off > 0) probe_sample(PR[e], 0, (int)bid.x, off - 1);
     return;
   }
-  slab_h_body<real>(stage_args(A + e, args), l, (int)bid.x - l.extra);
+  slab_h_body<real, kThin>(stage_args(A + e, args), l, (int)bid.x - l.extra);
 }
 
 // ------------------------------------------------------------------------------------- launch
@@ -630,6 +640,21 @@ static FastDiv fast_divisor(long long d, long long limit) {
   const unsigned long long excess = m * (unsigned long long)d - (1ull << 32);
   if (d > 1 && (unsigned long long)limit * std::max(excess, 1ull) < (1ull << 32)) f.m = (unsigned)m;
   return f;
+}
+
+// Whether a vector of cells can lie in both x slabs of a term (grids of twice the slab and a cell or
+// two): the kernels then keep a second x column, which takes registers that the others need.
+template <typename real>
+bool slab_thin(const SweepArgs<real>& a, int kind) {
+  constexpr int V = kVec<real>;
+  for (int c = 1; c < 3; ++c) {
+    const CpmlTerm<real>& T = kind == 0 ? a.ecorr[c][0] : a.hcorr[c][0];
+    const CpmlSide<real>* s = T.side;
+    if (s[0].psi == nullptr || s[1].psi == nullptr) continue;
+    const int lo = s[0].lo[0] < s[1].lo[0] ? 0 : 1;
+    if ((s[lo].hi[0] - 1) / V >= s[1 - lo].lo[0] / V) return true;
+  }
+  return false;
 }
 
 // Vectors of the boxes of one kind, all members.
@@ -714,34 +739,45 @@ cudaError_t launch_slab(const SweepArgs<real>& a, int kind, cudaStream_t s, cons
   const EdgeArgs<real>& e = ed ? *ed : no_ed;
   const ProbeArgs<real>& p = pr ? *pr : no_pr;
   const dim3 grid((unsigned)blocks), block(kSlabCols, 3);
-  if (kind == 0)
-    return launch_pdl(pdl, a.ade_P > 1 ? slab_e_kernel<real, true> : slab_e_kernel<real, false>, grid, block, 0, s, a, L,
-                      e, p, off);
-  return launch_pdl(pdl, slab_h_kernel<real>, grid, block, 0, s, a, L, p, off);
+  const bool thin = slab_thin(a, kind);
+  if (kind == 1)
+    return launch_pdl(pdl, thin ? slab_h_kernel<real, true> : slab_h_kernel<real, false>, grid, block, 0, s, a, L, p,
+                      off);
+  auto kernel = a.ade_P > 1 ? (thin ? slab_e_kernel<real, true, true> : slab_e_kernel<real, true, false>)
+                            : (thin ? slab_e_kernel<real, false, true> : slab_e_kernel<real, false, false>);
+  return launch_pdl(pdl, kernel, grid, block, 0, s, a, L, e, p, off);
 }
 
 template <typename real>
 cudaError_t launch_slab_batch(const SweepArgs<real>* A, const SlabLaunch* L, const EdgeArgs<real>* ED,
                               const ProbeArgs<real>* PR, const BatchGrid& G, int blocks, int kind, bool multi_pole,
-                              int off, bool pdl, cudaStream_t s) {
+                              bool thin, int off, bool pdl, cudaStream_t s) {
   if (blocks <= 0) return cudaSuccess;
   const dim3 grid(blocks), block(kSlabCols, 3);
-  if (kind == 0)
-    return launch_pdl(pdl, multi_pole ? slab_e_batch_kernel<real, true> : slab_e_batch_kernel<real, false>, grid, block,
-                      0, s, A, L, ED, PR, G, off);
-  return launch_pdl(pdl, slab_h_batch_kernel<real>, grid, block, 0, s, A, L, PR, G, off);
+  if (kind == 1)
+    return launch_pdl(pdl, thin ? slab_h_batch_kernel<real, true> : slab_h_batch_kernel<real, false>, grid, block, 0, s,
+                      A, L, PR, G, off);
+  auto kernel = multi_pole ? (thin ? slab_e_batch_kernel<real, true, true> : slab_e_batch_kernel<real, true, false>)
+                           : (thin ? slab_e_batch_kernel<real, false, true> : slab_e_batch_kernel<real, false, false>);
+  return launch_pdl(pdl, kernel, grid, block, 0, s, A, L, ED, PR, G, off);
 }
 
 template <typename real>
 cudaError_t preload_slab() {
   cudaFuncAttributes fa;
   const void* fns[] = {
-      reinterpret_cast<const void*>(slab_e_kernel<real, false>),
-      reinterpret_cast<const void*>(slab_e_kernel<real, true>),
-      reinterpret_cast<const void*>(slab_h_kernel<real>),
-      reinterpret_cast<const void*>(slab_e_batch_kernel<real, false>),
-      reinterpret_cast<const void*>(slab_e_batch_kernel<real, true>),
-      reinterpret_cast<const void*>(slab_h_batch_kernel<real>),
+      reinterpret_cast<const void*>(slab_e_kernel<real, false, false>),
+      reinterpret_cast<const void*>(slab_e_kernel<real, false, true>),
+      reinterpret_cast<const void*>(slab_e_kernel<real, true, false>),
+      reinterpret_cast<const void*>(slab_e_kernel<real, true, true>),
+      reinterpret_cast<const void*>(slab_h_kernel<real, false>),
+      reinterpret_cast<const void*>(slab_h_kernel<real, true>),
+      reinterpret_cast<const void*>(slab_e_batch_kernel<real, false, false>),
+      reinterpret_cast<const void*>(slab_e_batch_kernel<real, false, true>),
+      reinterpret_cast<const void*>(slab_e_batch_kernel<real, true, false>),
+      reinterpret_cast<const void*>(slab_e_batch_kernel<real, true, true>),
+      reinterpret_cast<const void*>(slab_h_batch_kernel<real, false>),
+      reinterpret_cast<const void*>(slab_h_batch_kernel<real, true>),
   };
   for (const void* f : fns) {
     const cudaError_t err = cudaFuncGetAttributes(&fa, f);
@@ -755,9 +791,10 @@ cudaError_t preload_slab() {
   template cudaError_t preload_slab<real>();                                                                          \
   template cudaError_t slab_plan<real>(const SweepArgs<real>&, int, SlabLaunch*, long long*, int);                    \
   template long long slab_vecs<real>(const SweepArgs<real>&, int);                                                    \
+  template bool slab_thin<real>(const SweepArgs<real>&, int);                                                         \
   template cudaError_t launch_slab_batch<real>(const SweepArgs<real>*, const SlabLaunch*, const EdgeArgs<real>*,      \
-                                               const ProbeArgs<real>*, const BatchGrid&, int, int, bool, int, bool,   \
-                                               cudaStream_t);                                                         \
+                                               const ProbeArgs<real>*, const BatchGrid&, int, int, bool, bool, int,   \
+                                               bool, cudaStream_t);                                                   \
   template cudaError_t launch_slab<real>(const SweepArgs<real>&, int, cudaStream_t, const EdgeArgs<real>*,            \
                                          const ProbeArgs<real>*, int, bool);
 OAFDTD_SLAB(float)
