@@ -460,7 +460,8 @@ int oafdtd_mlp_batch(const float* x, int32_t n_in, const float* t, int32_t n_out
                      int32_t groups, void* x16, void* x16t, float* t32, int32_t* counter, void* stream);
 
 /* The outputs of a network of n_layers for every member, from inputs x in host memory (rows x fan_in of
- * the first layer, FP32; read before the call returns): member k's outputs (rows x fan_out of the last
+ * the first layer, FP32; read before the call returns, above 4096 values by waiting for the work queued
+ * before it; in a stream capture, x stays as it is for the replays): member k's outputs (rows x fan_out of the last
  * layer, FP32) at y + k * y_stride. p32: FP32 parameters (the biases are read), w16t: transposed BF16
  * weights, both k * stride elements into their buffer; layers as in oafdtd_mlp_adam_net; act: the hidden
  * layers' activation as in oafdtd_mlp_gemm_tn (1 or 3). work: device memory of
