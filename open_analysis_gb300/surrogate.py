@@ -635,6 +635,10 @@ class Mlp:
             "rows": [None if rows is None else torch.from_numpy(r.astype(np.int64)).to(self.dev) for r in subsets],
             # batch j of member k: perm[j, k, :]
             "perm": torch.zeros((nb, self.members, self.batch), dtype=torch.int32, device=self.dev),
+            # two shuffles drawn ahead, row by member, each with the event of its last use
+            "drawn": [(torch.zeros((self.members, nb * self.batch), dtype=torch.int64, device=self.dev),
+                       torch.cuda.Event()) for _ in range(2)],
+            "epoch": 0,
             "buf": self._buffers(self.batch),
         }
         self._train = tr
@@ -662,18 +666,22 @@ class Mlp:
         tr = self._train
         assert tr is not None
         nb, m = tr["nb"], self.batch
-        # the shuffles are drawn on a stream of their own, beside the epoch before
+        # the shuffles are drawn on a stream of their own, beside the epoch before, into the buffer of the
+        # epoch before that: however many epochs are queued, two shuffles are held
+        drawn, used = tr["drawn"][tr["epoch"] % 2]
+        tr["epoch"] += 1
         with torch.cuda.stream(self.draw):
             picks = []
             for r in tr["rows"]:
                 pick = torch.randperm(tr["n"] if r is None else r.numel(), generator=self.gen, device=self.dev)[: nb * m]
                 picks.append(pick if r is None else r[pick])
-            perm = torch.stack(picks).view(self.members, nb, m).transpose(0, 1)
+            self.draw.wait_event(used)
+            torch.stack(picks, out=drawn)
         with torch.cuda.stream(self.stream):
             self.lr.fill_(lr)
             self.stream.wait_stream(self.draw)
-            tr["perm"].copy_(perm)
-            perm.record_stream(self.stream)
+            tr["perm"].copy_(drawn.view(self.members, nb, m).transpose(0, 1))
+            used.record(self.stream)
             if self.graph is not None:
                 self.graph.replay()
             else:

@@ -39,3 +39,41 @@ def test_inputs_may_be_reused_when_predict_returns(rows: int) -> None:
     pinned.fill_(0.0)
     torch.cuda.synchronize()
     assert torch.equal(out, want)
+
+
+def test_queued_epochs_hold_a_bounded_number_of_shuffles() -> None:
+    """Many epochs queued behind a busy stream (some 250 ms): the shuffles drawn ahead of the training
+    stream do not pile up (each is 2 members x 65536 rows of 8 bytes here, 1 MB)."""
+    net = _net(2, batch=65536)
+    rng = np.random.default_rng(2)
+    x, t = rng.standard_normal((66000, 8)), rng.standard_normal((66000, 16))
+    net.prepare(x, t)
+    net.run_epoch(1e-3)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_stats()["active_bytes.all.current"]
+    with torch.cuda.stream(net.stream):
+        torch.cuda._sleep(500_000_000)
+    for _ in range(40):
+        net.run_epoch(1e-3)
+    held = torch.cuda.memory_stats()["active_bytes.all.current"] - before
+    torch.cuda.synchronize()
+    assert held <= 4 * 2 * 65536 * 8, held
+
+
+def test_epochs_draw_the_shuffles_of_one_seed() -> None:
+    """Networks of one seed and data train alike, queued or waited for epoch by epoch, with all rows and
+    with row subsets: an epoch's shuffle is not overwritten before its steps have read it."""
+    rng = np.random.default_rng(3)
+    x, t = rng.standard_normal((300, 8)), rng.standard_normal((300, 16))
+    for rows in (None, [np.arange(0, 300, 2), np.arange(100, 290)]):
+        got = []
+        for wait in (False, True):
+            net = _net(2)
+            net.prepare(x, t, rows=rows)
+            for _ in range(12):
+                net.run_epoch(1e-3)
+                if wait:
+                    torch.cuda.synchronize()
+            torch.cuda.synchronize()
+            got.append(net.p32.clone())
+        assert torch.equal(got[0], got[1])
