@@ -245,16 +245,16 @@ int oafdtd_peak_bytes(const oafdtd_engine* engine, int64_t* out);
 int oafdtd_set_graph(oafdtd_engine* engine, int32_t use_graph);
 
 /* Launch shape of the sweeps: z planes marched per block (tile_z, 0 keeps the current value; at first
- * 16, in the fused variant 32 or all where the blocks are enough) and
- * the sweep variant (3: the fused sweep, which updates H and E of the interior in one z-march and
- * runs the rest as variant 2; it keeps two buffers per field, reading the current ones and writing
+ * 16, and where the fused variant is the default that sweep's own 32 or all planes where the blocks are
+ * enough) and the sweep variant (3: the fused sweep, which updates H and E of the interior in one z-march
+ * and runs the rest as variant 2; it keeps two buffers per field, reading the current ones and writing
  * the others, and is the default of float32 grids above 16 million cells times members where the
  * interior is not empty and the device has room for them; 2 stages the planes through shared memory
  * with TMA tensor copies, the default of the other large ones where the driver encodes the
  * descriptors; 1 stages them with cp.async; 0 sweeps the whole domain with the direct kernels, the
- * default of smaller grids and of float64; -1 keeps it). Variants 2 and 3 without descriptors, and 3 without an interior, are
- * OAFDTD_E_INVALID. The autotuner sets these. A staged sweep whose copies do not arrive within its
- * bounded wait makes the step return OAFDTD_E_TIMEOUT. */
+ * default of smaller grids and of float64; -1 keeps it). Variants 2 and 3 without descriptors, and 3
+ * without an interior, are OAFDTD_E_INVALID. The autotuner sets these. A staged sweep whose copies do
+ * not arrive within its bounded wait makes the step return OAFDTD_E_TIMEOUT. */
 int oafdtd_set_tuning(oafdtd_engine* engine, int32_t tile_z, int32_t variant);
 /* The current launch shape: planes per block and sweep variant (as oafdtd_set_tuning takes them). */
 int oafdtd_get_tuning(const oafdtd_engine* engine, int32_t* tile_z, int32_t* variant);

@@ -79,7 +79,10 @@ struct EngineBase {
   int64_t bytes = 0;
   int use_graph = 1;
   int profiling = 0;
-  int tile_z = 16;
+  int tile_z = 16;  // planes per block of the staged sweeps, and of the fused one where fused_tile is 0
+  // The fused sweep's own height, chosen in build() where it is the default variant; 0 where that is
+  // tile_z, and once the caller has set one.
+  int fused_tile = 0;
   // 3: fused H + E sweep of the interior (two buffers per field), the rest as 2; 2: sweeps
   // staged by TMA; 1: staged by cp.async; 0: the direct sweeps over the whole domain
   int staged = 2;
@@ -216,6 +219,7 @@ struct Engine final : EngineBase {
   // the staged interior with its z-slab and slab boxes (1, 2), or the slab kernel alone (0).
   void use_regions(int rv) {
     sw.staged = rv == 3 ? 2 : rv;
+    sw.tile_z = rv == 3 && fused_tile ? fused_tile : tile_z;
     sw.fused = rv == 3 ? fused_box : oafdtd::Span3{0, 0, 0, 0, 0, 0};
     for (int kind = 0; kind < 2; ++kind) {
       for (int zr = 0; zr < 2; ++zr)
@@ -769,7 +773,6 @@ int Engine<real>::build(const oafdtd_problem& p) {
   sw.Y = Y;
   sw.bs = bs;
   sw.B = B;
-  sw.tile_z = tile_z;
   if (int rc = alloc(&status, 1)) return rc;
   sw.status = status;
   sw.staged = staged;
@@ -1277,13 +1280,15 @@ int Engine<real>::build(const oafdtd_problem& p) {
       // once march all planes; several rounds of blocks take 32, fewer tiles 16. us per step with
       // 16 / 32 / all: 288 tiles (400x400x120, two members) 844 / 833 / 820; 912 tiles (397x323x160,
       // eight) 3058 / 3040 / 3111; 560 tiles 897 / 887 / 881; 240 tiles 662 / 670 / 661; 174 tiles
-      // 500 / 505 / 518.
+      // 500 / 505 / 518. A batch keeps each engine's own (two engines of 288 tiles 834 with all planes,
+      // 840 with the 32 of their 576 together). The staged sweeps, the halves' among them, keep 16:
+      // with these heights the halves of 400x400x120 took 1005 instead of 990.
       int sms = 0;
       OA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
       const oafdtd::Span3& F = fused_box;
       const long long tiles = (long long)((F.q1 - F.q0 + 31) / 32) * ((F.j1 - F.j0 + 7) / 8) * B, slots = 2LL * sms;
-      if (tiles > slots) tile_z = 32;
-      else if (10 * tiles >= 9 * slots) tile_z = F.k1 - F.k0;
+      if (tiles > slots) fused_tile = 32;
+      else if (10 * tiles >= 9 * slots) fused_tile = F.k1 - F.k0;
     }
   }
   OA_CUDA(cudaStreamSynchronize(stream));
@@ -1546,7 +1551,6 @@ int Engine<real>::enqueue(int64_t n) {
     for (auto& e : events) OA_CUDA(cudaEventCreate(&e));
     graph_ready = false;
   }
-  sw.tile_z = tile_z;
   if (profiling) {
     for (double& v : prof_ms) v = 0.0;
     prof_steps = 0;
@@ -1687,7 +1691,6 @@ int Engine<real>::step_half(int which) {
   if (which == 0) {
     if (half_pending) return fail(OAFDTD_E_INVALID, "an H half is already pending");
     if (steps + 1 > max_steps) return fail(OAFDTD_E_RANGE, "step count exceeds max_steps (wave table length)");
-    sw.tile_z = tile_z;
     if (int rc = launch_step(0, nullptr, false, 1)) return rc;
     OA_CUDA(oafdtd::launch_dft<real>(pr, 1, 2, false, 0, stream));
     half_pending = true;
@@ -2000,7 +2003,6 @@ struct Batch final : BatchBase {
       h_sw[p].resize(n);
       for (int i = 0; i < n; ++i) {
         Engine<real>& e = *eng[i];
-        e.sw.tile_z = e.tile_z;
         e.use_regions(rv);
         e.bind(p, p);
         h_sw[p][i] = e.sw;
@@ -2457,14 +2459,18 @@ int oafdtd_set_tuning(oafdtd_engine* engine, int32_t tile_z, int32_t variant) {
   if (variant < -1 || variant > 3) return fail(OAFDTD_E_INVALID, "variant must be -1, 0, 1, 2 or 3");
   if (variant >= 0 && variant != engine->impl->staged)
     if (int rc = engine->impl->set_variant(variant)) return rc;
-  if (tile_z) engine->impl->tile_z = tile_z;
+  if (tile_z) {
+    engine->impl->tile_z = tile_z;
+    engine->impl->fused_tile = 0;
+  }
   engine->impl->graph_dirty = true;  // a new launch shape needs a new graph
   return OAFDTD_OK;
 }
 
 int oafdtd_get_tuning(const oafdtd_engine* engine, int32_t* tile_z, int32_t* variant) {
   if (!engine || !tile_z || !variant) return fail(OAFDTD_E_INVALID, "null argument");
-  *tile_z = engine->impl->tile_z;
+  const EngineBase& e = *engine->impl;
+  *tile_z = e.staged == 3 && e.fused_tile ? e.fused_tile : e.tile_z;
   *variant = engine->impl->staged;
   return OAFDTD_OK;
 }
