@@ -1899,6 +1899,7 @@ struct Batch final : BatchBase {
   };
   std::vector<Engine<real>*> eng;
   int device = 0, variant = 0;
+  int home = -1;  // the buffer that an in-place variant steps (-1: variant 3 steps both in turn)
   cudaStream_t stream = nullptr, side = nullptr;
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr, done_ev = nullptr;
   std::vector<cudaEvent_t> in_ev;
@@ -1992,14 +1993,15 @@ struct Batch final : BatchBase {
     for (cudaEvent_t& ev : in_ev) OA_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     tma = variant >= 2;
     const int rv = variant;
-    // the engines' arguments of a step starting in buffer p (in place: p = 0 only)
-    const int parities = variant == 3 ? 2 : 1;
+    // the engines' arguments of a step starting in buffer p (in place: the one the fields are in)
+    home = variant == 3 ? -1 : e0.cur[0];
     std::vector<oafdtd::SweepMaps> mp(n);
     std::vector<oafdtd::FusedMaps> fm(n);
     std::vector<oafdtd::ProbeArgs<real>> pr(n);
     std::vector<oafdtd::SibcArgs<real>> sb(n);
     std::vector<oafdtd::EdgeArgs<real>> ed(n);
-    for (int p = 0; p < parities; ++p) {
+    for (int p = 0; p < 2; ++p) {
+      if (home >= 0 && p != home) continue;
       h_sw[p].resize(n);
       for (int i = 0; i < n; ++i) {
         Engine<real>& e = *eng[i];
@@ -2020,8 +2022,8 @@ struct Batch final : BatchBase {
       if (int rc = upload(&d_ed[p], ed.data(), n)) return rc;
     }
     for (Engine<real>* e : eng) e->bind(e->cur[0], e->cur[1]);
-    // launch geometry, from the parity-0 arguments (the boxes do not depend on the buffers)
-    const std::vector<oafdtd::SweepArgs<real>>& a = h_sw[0];
+    // launch geometry (the boxes do not depend on the buffers)
+    const std::vector<oafdtd::SweepArgs<real>>& a = h_sw[std::max(home, 0)];
     std::vector<dim3> g_fused(n), g_hi(n), g_hz(n), g_ei(n), g_ez(n), g_sh(n), g_se(n), g_pre(n), g_probe(n),
         g_edge(n), g_sibc(n), g_dft(n);
     std::vector<int> k_pole(n), k_zero(n, 0), k_sibc(n), k_slab[2] = {std::vector<int>(n), std::vector<int>(n)};
@@ -2207,7 +2209,7 @@ struct Batch final : BatchBase {
     if (n < 0) return fail(OAFDTD_E_INVALID, "negative step count");
     Engine<real>& e0 = *eng[0];
     for (Engine<real>* e : eng) {
-      if (e->steps != e0.steps || e->cur[0] != e0.cur[0] || e->half_pending)
+      if (e->steps != e0.steps || e->cur[0] != e0.cur[0] || e->half_pending || (home >= 0 && e->cur[0] != home))
         return fail(OAFDTD_E_INVALID, "an engine of the batch was stepped on its own");
       if (e->steps + n > e->max_steps) return fail(OAFDTD_E_RANGE, "step count exceeds max_steps (wave table length)");
     }
@@ -2220,7 +2222,7 @@ struct Batch final : BatchBase {
     while (done < n) {
       const int64_t start = e0.steps;
       const int take = (int)std::min<int64_t>(n - done, oafdtd::kChunk - start % oafdtd::kChunk);
-      const int p = variant == 3 ? e0.cur[0] : 0;
+      const int p = home >= 0 ? home : e0.cur[0];
       if (e0.use_graph && take == oafdtd::kChunk) {
         if (!graph[p])
           if (int rc = capture(p)) return rc;
