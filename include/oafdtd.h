@@ -194,8 +194,9 @@ int oafdtd_step_async(oafdtd_engine* engine, int64_t n);
 int oafdtd_wait(oafdtd_engine* engine);
 
 /* A batched sweep: n engines of one precision, device and sweep variant, at the same step, stepped
- * together. Every kernel class of a time step is then one launch over the blocks of all n engines
- * (the same kernel bodies on each engine's own arguments, so each engine's fields, DFTs and
+ * together. (Engines at their default variant count as of one, though a small grid's direct sweeps and a
+ * large one's fused sweep then run in launches and graphs of their own.) Every kernel class of a time
+ * step is then one launch over the blocks of all n engines (the same kernel bodies on each engine's own arguments, so each engine's fields, DFTs and
  * S-parameters are bit for bit those of stepping it alone); whole 64-step chunks replay one
  * captured graph for the whole batch. The engines stay owned by the caller and must outlive the
  * batch; while it exists they are stepped through it only (OAFDTD_E_INVALID otherwise), and

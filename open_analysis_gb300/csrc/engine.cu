@@ -86,6 +86,9 @@ struct EngineBase {
   // 3: fused H + E sweep of the interior (two buffers per field), the rest as 2; 2: sweeps
   // staged by TMA; 1: staged by cp.async; 0: the direct sweeps over the whole domain
   int staged = 2;
+  // The variant that a batch holds this engine to: the one the caller set, else the default it would have
+  // whatever its size, since the size alone must not keep default engines from one batch.
+  int batch_as = 2;
   bool tma_ok = false;  // the TMA descriptors were encoded (variant 2 available)
   bool fused_ok = false;  // the fused box is not empty and its descriptors were encoded
   bool graph_dirty = false;  // launch shape or profiling changed: the graph is re-captured
@@ -1269,6 +1272,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
   // The default variant. The direct sweeps (0) up to kDirectCells cells times members and for every
   // float64 grid, the fused sweep above where it applies and the device has room for the second
   // field buffers, else the staged sweeps in place.
+  batch_as = fused_ok && staged == 2 ? 3 : staged;
   if (sizeof(real) == 8 || (double)nx * ny * nz * B <= kDirectCells) {
     if (int rc = set_variant(0)) return rc;
   } else if (fused_ok && staged == 2) {
@@ -1290,6 +1294,7 @@ int Engine<real>::build(const oafdtd_problem& p) {
       if (tiles > slots) fused_tile = 32;
       else if (10 * tiles >= 9 * slots) fused_tile = F.k1 - F.k0;
     }
+    batch_as = staged;
   }
   OA_CUDA(cudaStreamSynchronize(stream));
   timer.mark("device_sync");
@@ -1885,6 +1890,8 @@ int Engine<real>::set_variant(int v) {
 // engine at once; nothing waits on the device. Whole 64-step chunks replay one captured graph.
 struct BatchBase {
   virtual ~BatchBase() = default;
+  virtual int check(int64_t n) = 0;  // whether n more steps may be queued
+  virtual int64_t steps() const = 0;
   virtual int enqueue(int64_t n) = 0;
   virtual int wait() = 0;
   int64_t graph_kernels = 0;
@@ -2205,7 +2212,9 @@ struct Batch final : BatchBase {
     return OAFDTD_OK;
   }
 
-  int enqueue(int64_t n) override {
+  int64_t steps() const override { return eng[0]->steps; }
+
+  int check(int64_t n) override {
     if (n < 0) return fail(OAFDTD_E_INVALID, "negative step count");
     Engine<real>& e0 = *eng[0];
     for (Engine<real>* e : eng) {
@@ -2213,6 +2222,12 @@ struct Batch final : BatchBase {
         return fail(OAFDTD_E_INVALID, "an engine of the batch was stepped on its own");
       if (e->steps + n > e->max_steps) return fail(OAFDTD_E_RANGE, "step count exceeds max_steps (wave table length)");
     }
+    return OAFDTD_OK;
+  }
+
+  int enqueue(int64_t n) override {
+    if (int rc = check(n)) return rc;
+    Engine<real>& e0 = *eng[0];
     OA_CUDA(cudaSetDevice(device));
     for (size_t i = 0; i < eng.size(); ++i) {
       OA_CUDA(cudaEventRecord(in_ev[i], eng[i]->stream));
@@ -2271,8 +2286,33 @@ struct oafdtd_engine {
 };
 
 struct oafdtd_batch {
-  std::unique_ptr<BatchBase> impl;
+  std::vector<std::unique_ptr<BatchBase>> parts;  // one per sweep variant
 };
+
+namespace {
+// The engines of a batch as one native batch per sweep variant. Variants that the callers set are one and
+// the same; beside them only defaults differ (the direct sweeps of a small grid, the fused of a large one).
+template <typename real>
+int make_batch(const std::vector<Engine<real>*>& engines, oafdtd_batch* b) {
+  bool one = true, one_default = true;
+  for (const Engine<real>* e : engines) {
+    one = one && e->staged == engines[0]->staged;
+    one_default = one_default && e->batch_as == engines[0]->batch_as;
+    if (e->device != engines[0]->device) return fail(OAFDTD_E_INVALID, "the engines of a batch share one device");
+    if (e->steps != engines[0]->steps)
+      return fail(OAFDTD_E_INVALID, "the engines of a batch start at the same step and buffers");
+  }
+  if (!one && !one_default) return fail(OAFDTD_E_INVALID, "the engines of a batch run one sweep variant");
+  std::map<int, std::vector<Engine<real>*>> by_variant;
+  for (Engine<real>* e : engines) by_variant[e->staged].push_back(e);
+  for (const auto& group : by_variant) {
+    auto part = std::make_unique<Batch<real>>();
+    if (int rc = part->build(group.second)) return rc;
+    b->parts.push_back(std::move(part));
+  }
+  return OAFDTD_OK;
+}
+}  // namespace
 
 extern "C" {
 
@@ -2461,6 +2501,7 @@ int oafdtd_set_tuning(oafdtd_engine* engine, int32_t tile_z, int32_t variant) {
   if (variant < -1 || variant > 3) return fail(OAFDTD_E_INVALID, "variant must be -1, 0, 1, 2 or 3");
   if (variant >= 0 && variant != engine->impl->staged)
     if (int rc = engine->impl->set_variant(variant)) return rc;
+  if (variant >= 0) engine->impl->batch_as = variant;
   if (tile_z) {
     engine->impl->tile_z = tile_z;
     engine->impl->fused_tile = 0;
@@ -2491,32 +2532,35 @@ int oafdtd_batch_create(oafdtd_engine* const* engines, int32_t n, oafdtd_batch**
   if (!f32.empty() && !f64.empty()) return fail(OAFDTD_E_INVALID, "the engines of a batch share one precision");
   std::unique_ptr<oafdtd_batch> b(new (std::nothrow) oafdtd_batch);
   if (!b) return fail(OAFDTD_E_OOM, "host allocation");
-  if (!f32.empty()) {
-    auto* impl = new Batch<float>();
-    b->impl.reset(impl);
-    if (int rc = impl->build(f32)) return rc;
-  } else {
-    auto* impl = new Batch<double>();
-    b->impl.reset(impl);
-    if (int rc = impl->build(f64)) return rc;
-  }
+  if (int rc = f32.empty() ? make_batch(f64, b.get()) : make_batch(f32, b.get())) return rc;
   *out = b.release();
   return OAFDTD_OK;
 }
 
 int oafdtd_batch_step_async(oafdtd_batch* batch, int64_t n) {
   if (!batch) return fail(OAFDTD_E_INVALID, "null batch");
-  return batch->impl->enqueue(n);
+  for (const auto& part : batch->parts) {  // all may, or none moves
+    if (int rc = part->check(n)) return rc;
+    if (part->steps() != batch->parts[0]->steps())
+      return fail(OAFDTD_E_INVALID, "an engine of the batch was stepped on its own");
+  }
+  for (const auto& part : batch->parts)
+    if (int rc = part->enqueue(n)) return rc;
+  return OAFDTD_OK;
 }
 
 int oafdtd_batch_wait(oafdtd_batch* batch) {
   if (!batch) return fail(OAFDTD_E_INVALID, "null batch");
-  return batch->impl->wait();
+  int first = OAFDTD_OK;
+  for (const auto& part : batch->parts)
+    if (int rc = part->wait()) first = first ? first : rc;
+  return first;
 }
 
 int oafdtd_batch_graph_kernels(const oafdtd_batch* batch, int64_t* out) {
   if (!batch || !out) return fail(OAFDTD_E_INVALID, "null argument");
-  *out = batch->impl->graph_kernels;
+  *out = 0;
+  for (const auto& part : batch->parts) *out += part->graph_kernels;
   return OAFDTD_OK;
 }
 
