@@ -46,7 +46,7 @@ int fail(int code, const std::string& msg) {
 // the planes of a tile is a long serial chain on few blocks; large ones are bound by the memory
 // traffic it saves. In float64 the two float64 operations a clock and SM bound every variant, and the
 // fused sweep computes its tiles' halos twice: 853 against 1406 us at 161 x 143 x 88.
-constexpr double kDirectCells = 16e6;
+constexpr double kDirectCells = 16e6;  // engine.py: DIRECT_CELLS
 
 constexpr double kEps0 = 1.0 / (4e-7 * 3.14159265358979323846 * 299792458.0 * 299792458.0);
 constexpr double kMu0 = 4e-7 * 3.14159265358979323846;

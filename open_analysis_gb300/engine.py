@@ -20,16 +20,18 @@ from open_analysis_gb300.grid import MU0
 
 FloatArray = npt.NDArray[np.float64]
 CHUNK = 64
+DIRECT_CELLS = 16_000_000  # cells times members up to which float32 grids run the direct sweeps by default
 
 
 def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_series: bool = False) -> int:
-    """Device bytes ``Gb300Engine`` allocates for a compiled problem: the role of the reference's
+    """Device bytes ``Gb300Engine`` allocates for a compiled problem at its default sweeps: the role of the reference's
     ``estimate_bytes`` (``engine.py:29-40``), which the run driver checks against free device
     memory before it builds the engine, counted from this engine's own buffers.
 
-    * six field arrays ``(B, Z, Y, X)`` twice (the fused sweep, the default of large float32 grids
-      and open to every grid with an interior free of CPML cells, reads one set and writes the
-      other) and the three uint16 index arrays ``(Z, Y, X)``;
+    * six field arrays ``(B, Z, Y, X)``, twice for the float32 grids above ``DIRECT_CELLS`` cells times
+      members whose default is the fused sweep (it reads one set and writes the other; on another grid
+      ``set_tuning(..., 3)`` allocates the second set then), and the three uint16 index arrays
+      ``(Z, Y, X)``;
     * dense Debye currents ``(P, B, nk, Y, X)`` per component over the z range ``nk`` of its
       dispersive edges;
     * one CPML psi array per correction: the slab width on its derivative axis, the full storage
@@ -38,7 +40,8 @@ def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_serie
       ``J_prev (B, n)`` and ``v (P, B, n)``;
     * the edge list of injection targets and deferred Debye edges with their saved ``E^n``, the
       sampled wave table ``(channels, max_steps)``, the probe lists, the DFT accumulators
-      ``(probes, B, F)`` complex128 and, when recording, the series ``(probes, B, max_steps)``;
+      ``(probes, B, F)`` complex128, the samples of a chunk ``(probes, B, 64)`` and, when recording, the
+      series ``(probes, B, max_steps)``;
     * the energy sum's float-float weights for float32 fields (per component, the x row and the
       y-z plane of pairs of float32);
     * the one-dimensional metrics, CPML coefficients, energy weights and partial sums, which are
@@ -49,7 +52,9 @@ def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_serie
     B = int(c.batch)
     bs = Z * Y * X
     rb = int(itemsize)
-    total = 2 * 6 * bs * B * rb + 3 * bs * 2
+    nx, ny, nz = g.n
+    sets = 2 if rb == 4 and nx * ny * nz * B > DIRECT_CELLS else 1
+    total = sets * 6 * bs * B * rb + 3 * bs * 2
     ade_flat: list[np.ndarray] = [np.zeros(0, np.int64)] * 3
     if c.ade is not None:
         P = int(c.ade.tau.size)
@@ -90,7 +95,7 @@ def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_serie
     total += n_chan * max_steps * 8 + B * n_chan * 8
     n_probe = len(c.probes)
     total += sum(np.asarray(q["flat"]).size for q in c.probes) * 16 + n_probe * 16
-    total += n_probe * B * int(c.frequencies.size) * 16
+    total += n_probe * B * (int(c.frequencies.size) * 16 + CHUNK * 8)
     if record_series:
         total += n_probe * B * max_steps * 8
     if rb == 4:  # the float-float weights of the float32 energy sum: x row and y-z plane per component
