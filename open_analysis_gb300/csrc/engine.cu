@@ -978,6 +978,9 @@ int Engine<real>::build(const oafdtd_problem& p) {
     pr.max_steps = p.max_steps;
     if ((rc = alloc(&dd, (size_t)std::max(p.n_probe, 1) * B * oafdtd::kChunk))) return rc;
     pr.vals = dd;
+    double2* tail_phase = nullptr;
+    if ((rc = alloc(&tail_phase, (size_t)std::max(p.n_freq, 1)))) return rc;
+    pr.tail_phase = tail_phase;
     if ((rc = alloc(&di, 1))) return rc;
     pr.dft_done = di;
     pr.series = nullptr;
@@ -2075,7 +2078,7 @@ struct Batch final : BatchBase {
       if (variant == 0) g_probe[i] = dim3(0, 0, 0);
       if (variant == 0 && e.inject_direct) g_pre[i] = g_edge[i] = dim3(0, 0, 0);
       g_sibc[i] = dim3((unsigned)oafdtd::sibc_blocks(e.sb), 1, 1);
-      g_dft[i] = dim3((unsigned)oafdtd::dft_blocks(e.pr), 1, 1);
+      g_dft[i] = dim3((unsigned)oafdtd::dft_blocks(e.pr, variant == 0), 1, 1);
       k_pole[i] = a[i].ade_P > 1 ? 1 : 0;
       k_slab[0][i] = k_pole[i] + 2 * oafdtd::slab_thin(a[i], 0);  // bit 0 several poles, bit 1 thin
       k_slab[1][i] = 2 * oafdtd::slab_thin(a[i], 1);

@@ -79,86 +79,98 @@ __global__ void __launch_bounds__(256) ghost_kernel(const __grid_constant__ Ghos
 // ----------------------------------------------------------------------------- probes
 // Every step's probe samples (probe_sample) are kept for the chunk; one launch at its end adds
 // them to the running DFTs, acc[f] += exp(-j w t) dt V with t = (n + offset) dt, step after step as
-// the reference does, and advances the step counter. A DFT per step put 256 float64 sincos of one
+// the reference does, and advances the step counter. In variant 0 the sweeps take every sample but the last
+// step's E probes, which this launch takes. A DFT per step put 256 float64 sincos of one
 // block on the path of every step (8 us a step for the E probes at 64 to 256 frequencies: GB300
 // issues two float64 operations a clock and SM); here a block takes four frequencies, one thread
 // per (frequency, step) for the phases, which all probes of a kind share, then one thread per
 // (probe, member, frequency) for the sums.
 constexpr int kDftF = 4;
 
-// Blocks per kind: one also without frequencies, for the tail samples.
+// Blocks of a DFT launch; tail: it takes the last step's E samples first, a block each.
 template <typename real>
-__host__ __device__ __forceinline__ int dft_blocks_per_kind(const ProbeArgs<real>& a) {
-  return a.n_freq > kDftF ? (a.n_freq + kDftF - 1) / kDftF : 1;
-}
-template <typename real>
-__host__ __device__ __forceinline__ int dft_blocks_of(const ProbeArgs<real>& a) {
-  return a.n_probe > 0 ? 2 * dft_blocks_per_kind(a) : 1;
+__host__ __device__ __forceinline__ int dft_blocks_of(const ProbeArgs<real>& a, bool tail) {
+  return (a.n_probe > 0 && a.n_freq > 0 ? 2 * ((a.n_freq + kDftF - 1) / kDftF) : 1) + (tail ? a.n_kind[0] * a.B : 0);
 }
 
 // Steps base .. base + n - 1 of the probes of the kinds in `kinds` (bit 0 E, bit 1 H). tail: the last
-// step's E samples are not in yet and taken here (by every block: a few points each).
+// step's E samples are not in yet. The first blocks take one each, the others leave them out of their
+// sums, and the block that ends last adds them. (Every block taking them all, one after the other: a single
+// step with 30 probes of 11932 points 4150 us at 200x160x80, 209 now, 156 with port probes alone.)
 template <typename real>
 __device__ __forceinline__ void dft_body(const ProbeArgs<real>& a, int block, int n, int kinds, bool tail, int bump) {
   __shared__ double2 ph[kDftF][kChunk];
-  __shared__ double tails[kChunk];
+  __shared__ int last;
   const long long base = *a.step_base;
-  const int nfb = dft_blocks_per_kind(a);
-  const int kind = block / nfb, f0 = (block % nfb) * kDftF;
-  const int pairs = (kinds >> kind) & 1 ? a.n_kind[kind] * a.B : 0;
-  if (pairs > 0) {
-    const int fi = threadIdx.x / kChunk, o = threadIdx.x % kChunk;
-    if (o < n && f0 + fi < a.n_freq) {
-      const double t = ((double)(base + o) + (kind == 0 ? 1.0 : 0.5)) * a.dt;
-      double sn, cs;
-      sincos(a.omega[f0 + fi] * t, &sn, &cs);
-      ph[fi][o] = make_double2(cs * a.dt, -(sn * a.dt));
-    }
-    const bool last = tail && kind == 0;
-    for (int p0 = 0; p0 < pairs; p0 += kChunk) {
-      if (last) {
-        for (int q = p0; q < min(pairs, p0 + kChunk); ++q) {
-          const int pid = a.list[0][q / a.B], b = q % a.B;
-          const double s = probe_sum(a, 0, pid, b);
-          if (threadIdx.x == 0) {
-            tails[q - p0] = s;
-            if (f0 == 0 && a.series != nullptr)
-              a.series[((long long)pid * a.B + b) * a.max_steps + base + n - 1] = s;
-          }
-        }
+  const int tails = tail ? a.n_kind[0] * a.B : 0, tid = (int)threadIdx.x;
+  if (block < tails) {
+    probe_sample(a, 0, block, n - 1);
+  } else {
+    const int nfb = (a.n_freq + kDftF - 1) / kDftF, d = block - tails;
+    const int kind = nfb > 0 ? d / nfb : 0, f0 = nfb > 0 ? (d % nfb) * kDftF : 0;
+    const int pairs = (kinds >> kind) & 1 ? a.n_kind[kind] * a.B : 0;
+    if (pairs > 0 && a.n_freq > 0) {
+      const int fi = tid / kChunk, o = tid % kChunk, m = tail && kind == 0 ? n - 1 : n;
+      if (o < n && f0 + fi < a.n_freq) {
+        const double t = ((double)(base + o) + (kind == 0 ? 1.0 : 0.5)) * a.dt;
+        double sn, cs;
+        sincos(a.omega[f0 + fi] * t, &sn, &cs);
+        ph[fi][o] = make_double2(cs * a.dt, -(sn * a.dt));
+        if (o >= m) a.tail_phase[f0 + fi] = ph[fi][o];
       }
       __syncthreads();
-      const int q = p0 + (int)threadIdx.x / kDftF, f = (int)threadIdx.x % kDftF;
-      if (q < pairs && f0 + f < a.n_freq) {
+      const int f = tid % kDftF;
+      for (int q = tid / kDftF; q < pairs && f0 + f < a.n_freq && m > 0; q += kChunk) {
         const long long pb = (long long)a.list[kind][q / a.B] * a.B + q % a.B;
         const double* v = a.vals + pb * kChunk;
         double2* out = a.acc + pb * a.n_freq + f0 + f;
         double2 cur = *out;
-        const int m = last ? n - 1 : n;
 #pragma unroll 8
         for (int s = 0; s < m; ++s) {
           const double x = v[s];
           cur.x += ph[f][s].x * x;
           cur.y += ph[f][s].y * x;
         }
-        if (last) {
-          cur.x += ph[f][n - 1].x * tails[q - p0];
-          cur.y += ph[f][n - 1].y * tails[q - p0];
-        }
         *out = cur;
       }
-      __syncthreads();
     }
   }
   if (bump == 0) return;
-  // the last block to get here advances the counter: every block has read it
+  // the last block to get here advances the counter: every block has read it, and its work is done
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (tid == 0) {
     __threadfence();
-    if (atomicAdd(a.dft_done, 1) == dft_blocks_of(a) - 1) {
-      *a.dft_done = 0;
-      *a.counter += bump;
+    last = atomicAdd(a.dft_done, 1) == dft_blocks_of(a, tail) - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int terms = tails * a.n_freq;  // the accumulators of one kind: below 2^31 elements in memory
+  constexpr int kAhead = 8, kStep = kDftF * kChunk;
+  for (int e0 = tid; e0 < terms; e0 += kAhead * kStep) {
+    double2* out[kAhead];
+    double2 cur[kAhead], p[kAhead];
+    double x[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int e = min(e0 + u * kStep, terms - 1), q = e / a.n_freq, f = e - q * a.n_freq;
+      const long long pb = (long long)a.list[0][q / a.B] * a.B + q % a.B;
+      x[u] = __ldcg(a.vals + pb * kChunk + n - 1);
+      p[u] = __ldcg(a.tail_phase + f);
+      out[u] = a.acc + pb * a.n_freq + f;
+      cur[u] = __ldcg(out[u]);
     }
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (e0 + u * kStep >= terms) continue;
+      cur[u].x += p[u].x * x[u];
+      cur[u].y += p[u].y * x[u];
+      *out[u] = cur[u];
+    }
+  }
+  if (tid == 0) {
+    *a.dft_done = 0;
+    *a.counter += bump;
   }
 }
 
@@ -668,14 +680,14 @@ cudaError_t launch_energy(const EnergyArgs<real>& a, double* partial, int nblock
 }
 
 template <typename real>
-int dft_blocks(const ProbeArgs<real>& a) {
-  return dft_blocks_of(a);
+int dft_blocks(const ProbeArgs<real>& a, bool tail) {
+  return dft_blocks_of(a, tail);
 }
 
 template <typename real>
 cudaError_t launch_dft(const ProbeArgs<real>& a, int n, int kinds, bool tail, int bump, cudaStream_t s) {
   // tail: the direct sweeps' launches, all of which take part
-  return launch_pdl(tail, dft_kernel<real>, dim3(dft_blocks_of(a)), dim3(kDftF * kChunk), 0, s, a, n, kinds,
+  return launch_pdl(tail, dft_kernel<real>, dim3(dft_blocks_of(a, tail)), dim3(kDftF * kChunk), 0, s, a, n, kinds,
                     tail ? 1 : 0, bump);
 }
 
@@ -693,7 +705,7 @@ cudaError_t launch_dft_batch(const ProbeArgs<real>* A, const BatchGrid& G, int b
   template cudaError_t launch_probe_e<real>(const ProbeArgs<real>&, int, cudaStream_t);            \
   template cudaError_t launch_edges<real>(const EdgeArgs<real>&, int, cudaStream_t);               \
   template cudaError_t launch_sibc<real>(const SibcArgs<real>&, cudaStream_t, int, int, bool);      \
-  template int dft_blocks<real>(const ProbeArgs<real>&);                                            \
+  template int dft_blocks<real>(const ProbeArgs<real>&, bool);                                      \
   template cudaError_t launch_dft<real>(const ProbeArgs<real>&, int, int, bool, int, cudaStream_t); \
   template cudaError_t launch_dft_batch<real>(const ProbeArgs<real>*, const BatchGrid&, int, int, bool, \
                                               cudaStream_t);                                        \

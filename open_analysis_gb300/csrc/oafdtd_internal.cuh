@@ -210,7 +210,8 @@ struct ProbeArgs {
   double2* acc;              // (n_probe, B, F)
   double* series;            // (n_probe, B, max_steps) or nullptr
   double* vals;              // (n_probe, B, kChunk): the samples of the steps of a chunk
-  int* dft_done;             // blocks of the DFT launch that have read the step counter
+  double2* tail_phase;       // (F): exp(-j w t) dt of the last step's E samples, while a DFT launch adds them
+  int* dft_done;             // blocks of the DFT launch whose work is done
   long long* counter;        // the step counter the DFT launch advances (step_base)
   int max_steps;
   long long bs;
@@ -368,7 +369,7 @@ cudaError_t launch_sibc_batch(const SibcArgs<real>* A, const BatchGrid& G, int b
 // The running DFTs of the n steps from the step counter on, for the probe kinds in `kinds` (bit 0
 // E, bit 1 H), which then advances by `bump`. tail: the E samples of the last step are taken here.
 template <typename real>
-int dft_blocks(const ProbeArgs<real>& a);
+int dft_blocks(const ProbeArgs<real>& a, bool tail);
 template <typename real>
 cudaError_t launch_dft(const ProbeArgs<real>& a, int n, int kinds, bool tail, int bump, cudaStream_t s);
 // Several engines' n steps, both kinds; every counter advances by n.
