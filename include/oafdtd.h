@@ -249,8 +249,9 @@ int oafdtd_set_graph(oafdtd_engine* engine, int32_t use_graph);
  * 16, and where the fused variant is the default that sweep's own 32 or all planes where the blocks are
  * enough) and the sweep variant (3: the fused sweep, which updates H and E of the interior in one z-march
  * and runs the rest as variant 2; it keeps two buffers per field, reading the current ones and writing
- * the others, and is the default of float32 grids above 16 million cells times members where the
- * interior is not empty and the device has room for them; 2 stages the planes through shared memory
+ * the others, and is the default of float32 grids above 16 million cells times members, 10 million
+ * where few edges are dispersive and the interior is most of the grid, if it is not empty and the
+ * device has room for them; 2 stages the planes through shared memory
  * with TMA tensor copies, the default of the other large ones where the driver encodes the
  * descriptors; 1 stages them with cp.async; 0 sweeps the whole domain with the direct kernels, the
  * default of smaller grids and of float64; -1 keeps it). Variants 2 and 3 without descriptors, and 3

@@ -45,8 +45,13 @@ int fail(int code, const std::string& msg) {
 // 820. Small fields stay in the 129 MB L2, where the fused sweep saves little, and its march over
 // the planes of a tile is a long serial chain on few blocks; large ones are bound by the memory
 // traffic it saves. In float64 the two float64 operations a clock and SM bound every variant, and the
-// fused sweep computes its tiles' halos twice: 853 against 1406 us at 161 x 143 x 88.
-constexpr double kDirectCells = 16e6;  // engine.py: DIRECT_CELLS
+// fused sweep computes its tiles' halos twice: 783 against 1406 us at 161 x 143 x 88.
+// The via's stack is dispersive in two thirds of its edges. Where few are, and the fused sweep's box holds
+// most of the grid, the lines cross earlier: microstrips 8.6 million 175 / 169, 12.0 million 235 / 202, 12.3
+// million 248 / 239, 14.4 million 276 / 230, 15 million (240x240x130) 307 / 274; substrates of one Debye
+// pole in a tenth of the planes 8.6 million 183 / 198, 10.2 million 211 / 193, 12.4 million 248 / 238, of
+// five 8.6 million 222 / 245, 10.2 million 258 / 247.
+constexpr double kDirectCells = 16e6, kDirectCellsPlain = 10e6;  // the lower one: engine.py, DIRECT_CELLS
 
 constexpr double kEps0 = 1.0 / (4e-7 * 3.14159265358979323846 * 299792458.0 * 299792458.0);
 constexpr double kMu0 = 4e-7 * 3.14159265358979323846;
@@ -1276,7 +1281,12 @@ int Engine<real>::build(const oafdtd_problem& p) {
   // float64 grid, the fused sweep above where it applies and the device has room for the second
   // field buffers, else the staged sweeps in place.
   batch_as = fused_ok && staged == 2 ? 3 : staged;
-  if (sizeof(real) == 8 || (double)nx * ny * nz * B <= kDirectCells) {
+  const double all_cells = (double)nx * ny * nz;
+  const double box_cells = 4.0 * (fused_box.q1 - fused_box.q0) * (fused_box.j1 - fused_box.j0) *
+                           (fused_box.k1 - fused_box.k0);
+  const double dispersive = (double)(ade_edges[0].size() + ade_edges[1].size() + ade_edges[2].size());
+  const bool mostly_plain = box_cells >= 0.7 * all_cells && dispersive <= 0.25 * 3.0 * all_cells;
+  if (sizeof(real) == 8 || all_cells * B <= (mostly_plain ? kDirectCellsPlain : kDirectCells)) {
     if (int rc = set_variant(0)) return rc;
   } else if (fused_ok && staged == 2) {
     size_t free_b = 0, total_b = 0;

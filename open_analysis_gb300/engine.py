@@ -20,7 +20,7 @@ from open_analysis_gb300.grid import MU0
 
 FloatArray = npt.NDArray[np.float64]
 CHUNK = 64
-DIRECT_CELLS = 16_000_000  # cells times members up to which float32 grids run the direct sweeps by default
+DIRECT_CELLS = 10_000_000  # cells times members up to which every float32 grid runs the direct sweeps by default
 
 
 def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_series: bool = False) -> int:
@@ -29,8 +29,8 @@ def estimate_bytes(c: Any, itemsize: int, max_steps: int = 200_000, record_serie
     memory before it builds the engine, counted from this engine's own buffers.
 
     * six field arrays ``(B, Z, Y, X)``, twice for the float32 grids above ``DIRECT_CELLS`` cells times
-      members whose default is the fused sweep (it reads one set and writes the other; on another grid
-      ``set_tuning(..., 3)`` allocates the second set then), and the three uint16 index arrays
+      members, whose default is or may be the fused sweep (it reads one set and writes the other; on
+      another grid ``set_tuning(..., 3)`` allocates the second set then), and the three uint16 index arrays
       ``(Z, Y, X)``;
     * dense Debye currents ``(P, B, nk, Y, X)`` per component over the z range ``nk`` of its
       dispersive edges;

@@ -11,15 +11,15 @@ from open_analysis_gb300.pml import CpmlSpec
 H = 0.2e-3
 
 
-def compiled_box(n):  # type: ignore[no-untyped-def]
+def compiled_box(n, poles=(), batch=2):  # type: ignore[no-untyped-def]
     nx, ny, nz = n
     m = Model(Grid(*(uniform_lines(k, H) for k in n)), Waveform("gauss_mod", 10e9, 18e9), np.linspace(1e9, 19e9, 3),
               walls=("cpml",) * 6, cpml=CpmlSpec(cells=6))
-    m.regions.append(Region((-1, -1, 2 * H), (1, 1, (nz // 2) * H), 3.7, 0.01))
+    m.regions.append(Region((-1, -1, 2 * H), (1, 1, (nz // 2) * H), 3.7, 0.01, False, poles))
     at = (nx // 3 * H, ny // 2 * H, (nz // 2 + 2) * H)
     m.sources.append(SoftSource("s", 2, at, at))
     m.probes.append(Probe("e", "E", 2, at, at))
-    m.drive = np.array([[1.0], [-2.0]])
+    m.drive = np.linspace(1.0, -2.0, batch)[:, None]
     return compile_model(m, "float32")
 
 
