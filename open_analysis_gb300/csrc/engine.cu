@@ -248,9 +248,9 @@ struct Engine final : EngineBase {
         sw.inner[kind] = oafdtd::Span3{0, 0, 0, 0, 0, 0};
         sw.zin[kind][0] = sw.zin[kind][1] = oafdtd::Span3{0, 0, 0, 0, 0, 0};
         // float32: one box. float64: the interior with its z slabs and the slab boxes around it, so
-        // that warps that pay for x and y corrections in float64 operations hold little else (853
-        // against 783 us per step at 161 x 143 x 88; in float32 more, smaller boxes cost more than
-        // that saves: microstrip 21.6 against 24.8 us).
+        // that warps that pay for x and y corrections in float64 operations hold little else (783
+        // us per step at 161 x 143 x 88, 853 as one box; in float32 more, smaller boxes cost more than
+        // that saves: microstrip 24.8 us, 21.6 as one box).
         int n = 0;
         const oafdtd::Span3& in = inner_staged[kind];
         const oafdtd::Span3 col{in.q0, in.q1, in.j0, in.j1, 1, nz + 2};
@@ -1753,8 +1753,8 @@ int Engine<real>::plane(int comp, int k, double* out, const double* in) {
 }
 
 // The same plane in the engine's own precision, device to device (dst or src is device memory
-// of (B, Y, X) elements, on this GPU or a peer): one copy per batch member on the engine's
-// stream, finished before the call returns.
+// of (B, Y, X) elements, on this GPU or a peer): a strided copy on the engine's stream, finished
+// before the call returns.
 template <typename real>
 int Engine<real>::plane_device(int comp, int k, void* dst, const void* src) {
   if (comp < 0 || comp > 5) return fail(OAFDTD_E_INVALID, "component must be 0..5");

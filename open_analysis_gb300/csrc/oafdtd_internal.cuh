@@ -442,7 +442,6 @@ bool umma_shape_ok(const UmmaProblem& p);
 cudaError_t launch_umma_gemm(const UmmaProblem& p, cudaStream_t s, std::string* why);
 constexpr int kUmmaList = 8;  // problems of one launch
 cudaError_t launch_umma_list(const UmmaProblem* p, int n, cudaStream_t s, std::string* why);
-cudaError_t preload_umma();
 // Encodes the TMA descriptors of the staged sweeps for the fields and indices in a; false (with
 // a message) when the driver entry point is missing or rejects a descriptor.
 template <typename real>

@@ -2,8 +2,9 @@
 //
 // The update domain of each sweep is split into an interior box, which holds no CPML correction
 // cell and is swept by the staged or fused kernels (staged.cu, fused.cu), and up to six disjoint
-// boxes around it: these kernels march those boxes. In variant 0 their one box is the whole
-// domain; it is the default where the fields of a grid stay in the L2 cache or are float64.
+// boxes around it: these kernels march those boxes. In variant 0 they have the whole domain, as one box
+// in float32; it is the default of float64 grids and of float32 grids whose fields mostly stay in the
+// L2 cache.
 //
 // Each thread owns one component of one 16-byte vector of x cells (four float32 or two float64) of one
 // storage row and marches a few z planes, carrying the plane its z derivative needs again; the three
@@ -11,7 +12,9 @@
 // Per plane every load is issued first (sources, field, index, Debye current, psi), then the
 // arithmetic, then the stores, so no load waits behind a store it cannot be proven not to alias; and
 // the next plane's lines are prefetched into L2, which needs no registers. What bounds these kernels
-// is the latency of those loads at 24 warps per SM (80 registers): at 400x400x120, batch 2, over the
+// is the latency of those loads at 24 warps per SM, which leaves a thread 80 registers (spilled bytes:
+// H none; E in float32 40 with one pole, 136 with several, in float64 232 and 112; the batched kernels,
+// whose arguments are in shared memory, H 8 and 32, E 236, 320, 292 and 308): at 400x400x120, batch 2, over the
 // whole grid H takes 0.31 ms and E 0.49 ms (4.5 and 4.1 TB/s of the measured 6.8; 0.32 and 0.52
 // without the prefetch at 16 planes). Three shapes measured and left: every component in one thread
 // (168 registers, 0.62 and 1.53 ms), one plane per thread (set-up dominates: 0.59 and 0.88 ms), one

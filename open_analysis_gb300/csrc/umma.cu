@@ -10,7 +10,7 @@
 // of every group with a stride of the grid size. Ten warps with fixed roles:
 //   warp 0, one lane: the producer. Each K step (64 elements, 128 bytes) of a tile's A and B
 //     arrives by one TMA tensor copy each (cp.async.bulk.tensor, 3-D maps over rows, K and the
-//     group, 128-byte swizzle) into a 4-stage shared-memory ring, completing on the stage's
+//     group, 128-byte swizzle) into a ring of stages in shared memory (kUStages), completing on the stage's
 //     "full" mbarrier; the producer refills a stage once its "empty" mbarrier says the MMAs have
 //     read it. It runs ahead across tile boundaries.
 //   warp 1: allocates 2 x BN columns of TMEM (two accumulators); one lane issues the MMAs
@@ -526,14 +526,6 @@ cudaError_t launch_umma_gemm(const UmmaProblem& p, cudaStream_t s, std::string* 
 // 512x512x256, 512x1024x256, 8x512x256) took 46.7 us one by one, 21.0 together.
 cudaError_t launch_umma_list(const UmmaProblem* p, int n, cudaStream_t s, std::string* why) {
   return n <= kUmmaList ? launch_list<128, kUmmaList>(p, n, s, why) : cudaErrorNotSupported;
-}
-
-cudaError_t preload_umma() {
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<128, 1>));
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<128, kUmmaList>));
-  if (e != cudaSuccess) return e;
-  return cudaFuncGetAttributes(&fa, reinterpret_cast<const void*>(umma_gemm_kernel<64, 1>));
 }
 
 static_assert(sizeof(UStage<128>) == (kUM + 128) * kUK * 2, "stage tiles are contiguous and 1024-byte multiples");
