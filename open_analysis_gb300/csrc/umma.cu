@@ -25,7 +25,7 @@
 //     it with cp.async.bulk.tensor (FP32: 128-byte swizzle; BF16: 64-byte; transposed BF16:
 //     plain rows of 64 bytes), so the epilogue of one tile overlaps the MMAs of the next.
 // Ragged extents: TMA fills a box's part past the matrix with zeros on loads and leaves it out on
-// stores, so any M, N and K run here; the results are bit for bit the mma.sync kernel's (the same K
+// stores (but for the rest of a row's last 16 bytes, see the epilogue), so any M, N and K run here; the results are bit for bit the mma.sync kernel's (the same K
 // steps of 16). The training and prediction shapes are bound by latency, not by the tensor pipe (one
 // tile per CTA: launch, descriptors, two rounds of TMA, epilogue): the launches are programmatic
 // dependents, so a kernel sets up in the tail of the one before (8 x 256x512x512: 10.5 to 7.5 us;
@@ -60,8 +60,10 @@ constexpr unsigned kUPolls = 1u << 28;
 struct UmmaArgs {
   const float* bias;          // per column and group (nullable)
   const __nv_bfloat16* mask;  // epilogues 2 and 4: layout of C (ldc, group stride sC)
-  long long sBias, sC;
-  int M, N, K, ldc, act, groups;
+  float* C32;
+  __nv_bfloat16 *C16, *C16T;
+  long long sBias, sC, sCT;
+  int M, N, K, ldc, ldct, act, groups;
   int has32, has16, has16t;
   int* status;
 };
@@ -207,7 +209,8 @@ __device__ __forceinline__ UmmaTile umma_tile(const UmmaList<kMax>& L, int tile)
   return UmmaTile{p, (r / NT) % MT, r % NT, r / (NT * MT), (g.K + kUK - 1) / kUK};
 }
 
-template <int BN, int kMax>
+// kEnds: some result's rows end within 16 bytes (see the epilogue; its code costs the others 1 to 10 %).
+template <int BN, int kMax, bool kEnds>
 __global__ void __launch_bounds__(kUThreads, 1) umma_gemm_kernel(const __grid_constant__ UmmaList<kMax> L) {
   extern __shared__ unsigned char umma_raw[];
   constexpr int kS = kUStages<BN>;
@@ -409,11 +412,31 @@ __global__ void __launch_bounds__(kUThreads, 1) umma_gemm_kernel(const __grid_co
         }
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         __syncwarp();
+        // A TMA store writes whole 16 bytes of a row, past the end of one that ends within them: such ends
+        // go out by plain stores.
+        const int rows = min(32, g.M - row0), cols = min(32, g.N - col0);
+        const bool whole32 = !kEnds || (cols & 3) == 0, whole16 = !kEnds || (cols & 7) == 0;
+        const bool whole_t = !kEnds || (rows & 7) == 0;
         if (lane == 0) {
-          if (g.has32) utma_store(&L.c32[w.p], es.c32, col0, row0, gi);
-          if (g.has16) utma_store(&L.c16[w.p], es.c16, col0, row0, gi);
-          if (g.has16t) utma_store(&L.c16t[w.p], es.c16t, row0, col0, gi);
+          if (g.has32 && whole32) utma_store(&L.c32[w.p], es.c32, col0, row0, gi);
+          if (g.has16 && whole16) utma_store(&L.c16[w.p], es.c16, col0, row0, gi);
+          if (g.has16t && whole_t) utma_store(&L.c16t[w.p], es.c16t, row0, col0, gi);
           asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+        }
+        if (!(whole32 && whole16) && lane < cols) {
+          const long long at = gi * g.sC + (long long)row0 * g.ldc + col0 + lane;
+#pragma unroll 1
+          for (int i = 0; i < rows; ++i) {
+            if (g.has32 && !whole32)
+              g.C32[at + (long long)i * g.ldc] = es.c32[32 * i + ((((lane >> 2) ^ (i & 7)) << 2) | (lane & 3))];
+            if (g.has16 && !whole16)
+              g.C16[at + (long long)i * g.ldc] = es.c16[32 * i + ((((lane >> 3) ^ ((i >> 1) & 3)) << 3) | (lane & 7))];
+          }
+        }
+        if (g.has16t && !whole_t && lane < rows) {
+          const long long at = gi * g.sCT + (long long)col0 * g.ldct + row0 + lane;
+#pragma unroll 1
+          for (int j = 0; j < cols; ++j) g.C16T[at + (long long)j * g.ldct] = es.c16t[32 * j + lane];
         }
       }
     }
@@ -468,6 +491,8 @@ bool add_problem(UmmaList<kMax>* L, int k, const UmmaProblem& p, std::string* wh
   g.sBias = p.sBias;
   g.sC = p.sC;
   g.M = p.M, g.N = p.N, g.K = p.K, g.ldc = p.ldc, g.act = p.act, g.groups = p.groups;
+  g.C32 = p.C32, g.C16 = static_cast<__nv_bfloat16*>(p.C16), g.C16T = static_cast<__nv_bfloat16*>(p.C16T);
+  g.sCT = p.sCT, g.ldct = p.ldct;
   g.has32 = p.C32 != nullptr, g.has16 = p.C16 != nullptr, g.has16t = p.C16T != nullptr;
   g.status = p.status;
   const long long tiles = (long long)p.groups * ((p.M + kUM - 1) / kUM) * ((p.N + BN - 1) / BN);
@@ -483,7 +508,10 @@ cudaError_t launch_list(const UmmaProblem* p, int n, cudaStream_t s, std::string
   for (int k = 0; k < n; ++k)
     if (!add_problem<BN>(&L, k, p[k], why)) return cudaErrorNotSupported;
   const size_t bytes = sizeof(UStage<BN>) * kUStages<BN> + sizeof(EpiStage) * kEpiWarps + 1024;
-  auto kernel = umma_gemm_kernel<BN, kMax>;
+  bool ends = false;
+  for (int k = 0; k < n; ++k)
+    ends = ends || (p[k].C32 && p[k].N % 4) || (p[k].C16 && p[k].N % 8) || (p[k].C16T && p[k].M % 8);
+  auto kernel = ends ? umma_gemm_kernel<BN, kMax, true> : umma_gemm_kernel<BN, kMax, false>;
   cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   if (err != cudaSuccess) return err;
   static int sms = 0;
