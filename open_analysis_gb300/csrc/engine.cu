@@ -1277,38 +1277,42 @@ int Engine<real>::build(const oafdtd_problem& p) {
     });
   }
   timer.mark("traffic_model");
-  // The default variant. The direct sweeps (0) up to kDirectCells cells times members and for every
-  // float64 grid, the fused sweep above where it applies and the device has room for the second
-  // field buffers, else the staged sweeps in place.
+  // The default variant. The direct sweeps (0) up to kDirectCells cells times members (kDirectCellsPlain
+  // of mostly plain grids) and for every float64 grid, the fused sweep above where it applies and the
+  // device has room for the second field buffers, else the direct sweeps up to kDirectCells and the
+  // staged ones in place.
   batch_as = fused_ok && staged == 2 ? 3 : staged;
   const double all_cells = (double)nx * ny * nz;
   const double box_cells = 4.0 * (fused_box.q1 - fused_box.q0) * (fused_box.j1 - fused_box.j0) *
                            (fused_box.k1 - fused_box.k0);
   const double dispersive = (double)(ade_edges[0].size() + ade_edges[1].size() + ade_edges[2].size());
   const bool mostly_plain = box_cells >= 0.7 * all_cells && dispersive <= 0.25 * 3.0 * all_cells;
-  if (sizeof(real) == 8 || all_cells * B <= (mostly_plain ? kDirectCellsPlain : kDirectCells)) {
-    if (int rc = set_variant(0)) return rc;
-  } else if (fused_ok && staged == 2) {
+  bool fused_default = sizeof(real) == 4 && fused_ok && staged == 2 &&
+                       all_cells * B > (mostly_plain ? kDirectCellsPlain : kDirectCells);
+  if (fused_default) {
     size_t free_b = 0, total_b = 0;
     OA_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    if ((double)free_b > 1.05 * 6.0 * (double)bs * B * sizeof(real)) {
-      if (int rc = set_variant(3)) return rc;
-      // Planes per block of the fused sweep, two blocks to an SM. Tiles that nearly fill the chip
-      // once march all planes; several rounds of blocks take 32, fewer tiles 16. us per step with
-      // 16 / 32 / all: 288 tiles (400x400x120, two members) 844 / 833 / 820; 912 tiles (397x323x160,
-      // eight) 3058 / 3040 / 3111; 560 tiles 897 / 887 / 881; 240 tiles 662 / 670 / 661; 174 tiles
-      // 500 / 505 / 518. A batch keeps each engine's own (two engines of 288 tiles 834 with all planes,
-      // 840 with the 32 of their 576 together). The staged sweeps, the halves' among them, keep 16:
-      // with these heights the halves of 400x400x120 took 1005 instead of 990.
-      int sms = 0;
-      OA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-      const oafdtd::Span3& F = fused_box;
-      const long long tiles = (long long)((F.q1 - F.q0 + 31) / 32) * ((F.j1 - F.j0 + 7) / 8) * B, slots = 2LL * sms;
-      if (tiles > slots) fused_tile = 32;
-      else if (10 * tiles >= 9 * slots) fused_tile = F.k1 - F.k0;
-    }
-    batch_as = staged;
+    fused_default = (double)free_b > 1.05 * 6.0 * (double)bs * B * sizeof(real);
   }
+  if (fused_default) {
+    if (int rc = set_variant(3)) return rc;
+    // Planes per block of the fused sweep, two blocks to an SM. Tiles that nearly fill the chip
+    // once march all planes; several rounds of blocks take 32, fewer tiles 16. us per step with
+    // 16 / 32 / all: 288 tiles (400x400x120, two members) 844 / 833 / 820; 912 tiles (397x323x160,
+    // eight) 3058 / 3040 / 3111; 560 tiles 897 / 887 / 881; 240 tiles 662 / 670 / 661; 174 tiles
+    // 500 / 505 / 518. A batch keeps each engine's own (two engines of 288 tiles 834 with all planes,
+    // 840 with the 32 of their 576 together). The staged sweeps, the halves' among them, keep 16:
+    // with these heights the halves of 400x400x120 took 1005 instead of 990.
+    int sms = 0;
+    OA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const oafdtd::Span3& F = fused_box;
+    const long long tiles = (long long)((F.q1 - F.q0 + 31) / 32) * ((F.j1 - F.j0 + 7) / 8) * B, slots = 2LL * sms;
+    if (tiles > slots) fused_tile = 32;
+    else if (10 * tiles >= 9 * slots) fused_tile = F.k1 - F.k0;
+  } else if (sizeof(real) == 8 || all_cells * B <= kDirectCells) {
+    if (int rc = set_variant(0)) return rc;
+  }
+  if (staged != 0) batch_as = staged;
   OA_CUDA(cudaStreamSynchronize(stream));
   timer.mark("device_sync");
   return OAFDTD_OK;

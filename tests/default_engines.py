@@ -11,11 +11,14 @@ from open_analysis_gb300.pml import CpmlSpec
 H = 0.2e-3
 
 
-def compiled_box(n, poles=(), batch=2):  # type: ignore[no-untyped-def]
+def compiled_box(n, poles=(), batch=2, materials=0):  # type: ignore[no-untyped-def]
     nx, ny, nz = n
     m = Model(Grid(*(uniform_lines(k, H) for k in n)), Waveform("gauss_mod", 10e9, 18e9), np.linspace(1e9, 19e9, 3),
               walls=("cpml",) * 6, cpml=CpmlSpec(cells=6))
     m.regions.append(Region((-1, -1, 2 * H), (1, 1, (nz // 2) * H), 3.7, 0.01, False, poles))
+    for k in range(materials):  # a row of little blocks, each of its own permittivity
+        x, y = (8 + 3 * (k % 100)) * H, (8 + 3 * (k // 100)) * H
+        m.regions.append(Region((x, y, (nz // 2) * H), (x + 2 * H, y + 2 * H, (nz // 2 + 2) * H), 1.5 + 0.01 * k))
     at = (nx // 3 * H, ny // 2 * H, (nz // 2 + 2) * H)
     m.sources.append(SoftSource("s", 2, at, at))
     m.probes.append(Probe("e", "E", 2, at, at))

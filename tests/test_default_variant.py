@@ -21,3 +21,10 @@ def test_default_variant(n, dispersive, want) -> None:  # type: ignore[no-untype
     eng = engine(c)
     assert c.batch == batch and eng.get_tuning()[1] == want
     eng.close()
+
+
+def test_default_of_a_plain_grid_that_the_fused_sweep_cannot_take() -> None:
+    """10.8 million cells with more materials than the fused sweep's table holds: the direct sweeps."""
+    eng = engine(compiled_box((400, 300, 90), batch=1, materials=300))
+    assert eng.get_tuning()[1] == 0
+    eng.close()
